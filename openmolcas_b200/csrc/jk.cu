@@ -32,6 +32,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "coulomb.cuh"
 #include "kern_common.cuh"
 #include "mg_internal.h"
 #include "oz_gemm.cuh"
@@ -248,10 +249,6 @@ __device__ __forceinline__ int oz_exponent(double m) {
 
 __device__ __forceinline__ double warp_max(double v) {
   for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-__device__ __forceinline__ double warp_sum(double v) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
@@ -476,39 +473,6 @@ __global__ void k_jacc64(const double* __restrict__ L, int64_t nrs, int nb, cons
   double s = 0.0;
   for (int J = 0; J < nb; ++J) s = fma(L[t + nrs * J], V[J], s);
   jrs[t] += s;
-}
-
-// Coulomb contractions of a batch's further densities (the first one's are
-// formed by the L unpacking): V[d nb + J] = sum_t L[t, J] dw_d[t] for
-// d = 1 .. kd, dw_d = dws + (d - 1) nrs the packed weighted density
-// (k_pack_density).  One CTA per vector J, each vector element read once.
-constexpr int kJkMaxDens = 8;
-
-__global__ void __launch_bounds__(256) k_vmulti(const double* __restrict__ L, int64_t nrs, int nb, int kd,
-                                                const double* __restrict__ dws, double* __restrict__ V) {
-  __shared__ double red[kJkMaxDens][8];
-  const int J = blockIdx.x;
-  const double* LJ = L + nrs * J;
-  double acc[kJkMaxDens - 1];
-#pragma unroll
-  for (int d = 0; d < kJkMaxDens - 1; ++d) acc[d] = 0.0;
-  for (int64_t t = threadIdx.x; t < nrs; t += blockDim.x) {
-    const double x = __ldg(LJ + t);
-#pragma unroll
-    for (int d = 0; d < kJkMaxDens - 1; ++d)
-      if (d < kd) acc[d] = fma(x, __ldg(dws + (size_t)d * nrs + t), acc[d]);
-  }
-#pragma unroll
-  for (int d = 0; d < kJkMaxDens - 1; ++d) {
-    const double v = warp_sum(acc[d]);
-    if ((threadIdx.x & 31) == 0) red[d][threadIdx.x >> 5] = v;
-  }
-  __syncthreads();
-  if ((int)threadIdx.x < kd) {
-    double v = 0.0;
-    for (int w = 0; w < 8; ++w) v += red[threadIdx.x][w];
-    V[(size_t)(threadIdx.x + 1) * nb + J] = v;
-  }
 }
 
 // jrs_d[t] += sum_J L[t, J] V[d nb + J] for the k densities of a batch,
@@ -832,7 +796,7 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
       const int nv = std::min(nb, M - J0);
       const double* Lb = cho_vec_ptr(c, J0, nv, st, h);
       if (!Lb) { h->err = "vector block straddles storage blocks"; return MG_ERR_ARG; }
-      cudaMemsetAsync(V, 0, 8 * (size_t)nb, st);
+      cudaMemsetAsync(V, 0, 8 * (size_t)nb * k, st);
       oz_with_slices(s, [&](auto S) {
         k_oz_slice_l_blocks<decltype(S)::value>
             <<<dim3((ld + kOzChunk - 1) / kOzChunk, ld / kOzRows, nv), kOzChunk, 0, st>>>(
@@ -844,7 +808,7 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
         k_jacc64<<<nb256(nrs), 256, 0, st>>>(Lb, nrs, nv, V, dd[0].jrs);
         if (!launched("k_jacc64")) return MG_ERR_CUDA;
       } else {
-        k_vmulti<<<nv, 256, 0, st>>>(Lb, nrs, nb, k - 1, dws, V);
+        launch_vmulti(Lb, nrs, nv, nb, k - 1, dws, V + nb, st);
         if (!launched("k_vmulti")) return MG_ERR_CUDA;
         k_jacc_multi<<<nb256(nrs), 256, 0, st>>>(Lb, nrs, nv, nb, k, V, jrs_all);
         if (!launched("k_jacc_multi")) return MG_ERR_CUDA;
