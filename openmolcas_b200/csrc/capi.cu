@@ -542,7 +542,7 @@ int mg_cho_jk(mg_handle* H, const double* d_C, int r, double* d_J, double* d_K, 
   Handle* h = &H->h;
   if (!h->cho) { h->err = "mg_cho_jk: no Cholesky vectors (call mg_cho_drv)"; return MG_ERR_ARG; }
   cudaSetDevice(h->device);
-  if (precision == MG_PREC_FP64) return jk_fp64(h, d_C, r, d_J, d_K, (cudaStream_t)stream, 32);
+  if (precision == MG_PREC_FP64) return jk_fp64(h, d_C, r, d_J, d_K, (cudaStream_t)stream);
   if (precision == MG_PREC_MIXED)
     return jk_mixed(h, d_C, r, d_J, d_K, (cudaStream_t)stream, 64, MG_JK_SLICES, MG_JK_SLICES_K);
   if (precision > 100 && precision <= 108)
@@ -558,7 +558,7 @@ int mg_cho_jk_batch(mg_handle* H, int ndens, const double* const* d_C, const int
   if (!h->cho) { h->err = "mg_cho_jk_batch: no Cholesky vectors (call mg_cho_drv)"; return MG_ERR_ARG; }
   cudaSetDevice(h->device);
   cudaStream_t st = (cudaStream_t)stream;
-  if (precision == MG_PREC_FP64) return jk_fp64_batch(h, ndens, d_C, r, d_J, d_K, st, 32);
+  if (precision == MG_PREC_FP64) return jk_fp64_batch(h, ndens, d_C, r, d_J, d_K, st);
   if (precision == MG_PREC_MIXED) return jk_mixed_batch(h, ndens, d_C, r, d_J, d_K, st, 64, MG_JK_SLICES, MG_JK_SLICES_K);
   if (precision > 100 && precision <= 108)
     return jk_mixed_batch(h, ndens, d_C, r, d_J, d_K, st, 64, precision - 100, precision - 100);

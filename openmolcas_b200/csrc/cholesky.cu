@@ -217,6 +217,7 @@ struct ChoState {
   cublasHandle_t cublas = nullptr;
   short* d_lexp = nullptr;      // row exponents of the square L_J (mixed J/K), M x lexp_ld
   int lexp_ld = 0;
+  int* d_inv = nullptr;         // rs index of every AO pair (n x n, -1: no row), J/K
 };
 
 static const int kVecBlock = 1024;
@@ -224,7 +225,7 @@ static const int kVecBlock = 1024;
 void cho_free(ChoState* c) {
   if (!c) return;
   cudaFree(c->d_rs); cudaFree(c->d_sp_first); cudaFree(c->d_sp_count); cudaFree(c->d_rs_a); cudaFree(c->d_rs_b);
-  cudaFree(c->d_diag); cudaFree(c->d_diag0); cudaFree(c->d_inred); cudaFree(c->d_lexp);
+  cudaFree(c->d_diag); cudaFree(c->d_diag0); cudaFree(c->d_inred); cudaFree(c->d_lexp); cudaFree(c->d_inv);
   for (auto p : c->Lblk) cudaFree(p);
   if (c->cublas) cublasDestroy(c->cublas);
   delete c;
@@ -624,6 +625,33 @@ void cho_set_lexp(ChoState* c, short* p, int ld) {
   cudaFree(c->d_lexp);
   c->d_lexp = p;
   c->lexp_ld = ld;
+}
+
+// inv[a*n + b] = inv[b*n + a] = t for every rs pair t (filled with -1 first:
+// AO pairs of shell pairs without rows keep it)
+__global__ void k_rs_inverse(const int* __restrict__ rs_a, const int* __restrict__ rs_b, int64_t nrs, int n,
+                             int* __restrict__ inv) {
+  int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (t >= nrs) return;
+  const int a = rs_a[t], b = rs_b[t];
+  inv[(size_t)a * n + b] = (int)t;
+  inv[(size_t)b * n + a] = (int)t;
+}
+
+const int* cho_inv_dev(ChoState* c, int n, cudaStream_t st) {
+  if (c->d_inv) return c->d_inv;
+  int* p = nullptr;
+  const size_t bytes = sizeof(int) * (size_t)n * n;
+  if (dev_malloc(&p, bytes) != cudaSuccess) return nullptr;
+  cudaMemsetAsync(p, 0xFF, bytes, st);
+  k_rs_inverse<<<nblk(std::max<int64_t>(c->nrs, 1)), 256, 0, st>>>(c->d_rs_a, c->d_rs_b, c->nrs, n, p);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  // later calls may come on other streams: the table is complete before it is kept
+  if (cudaStreamSynchronize(st) != cudaSuccess) {
+    cudaFree(p);
+    return nullptr;
+  }
+  return c->d_inv = p;
 }
 
 // ------------------------------------------------- in-core decomposition

@@ -17,9 +17,7 @@
 // (lower-triangle tiles, CTA-private FP64 tiles, FP64 atomics into K).  J
 // is FP64 throughout.
 //
-// FP64 path ("plain FP64 GPU path"): vectors in FP64, per block of vectors
-// the rs-packed L_J are unpacked to dense symmetric nbf x nbf matrices, the
-// half-transform is one strided-batched DGEMM and K accumulates by DSYRK.
+// The FP64 path is in jk64.cu.
 // LK screening is not applied (dense tensor work is cheaper on the GPU than
 // the screening bookkeeping); the result equals the unscreened reference.
 #include <cublas_v2.h>
@@ -48,38 +46,12 @@ __global__ void k_pack_density(const int* __restrict__ rs_a, const int* __restri
   dw[t] = (a == b ? 1.0 : 2.0) * D[(size_t)a * n + b];
 }
 
-// J[a,b] = J[b,a] = jrs[t]
-__global__ void k_unpack_sym(const int* __restrict__ rs_a, const int* __restrict__ rs_b, int64_t nrs,
-                             const double* __restrict__ v, int n, double* __restrict__ M) {
-  int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= nrs) return;
-  const int a = rs_a[t], b = rs_b[t];
-  M[(size_t)a * n + b] = v[t];
-  M[(size_t)b * n + a] = v[t];
-}
-
-// Lsq[J][a][b] = Lsq[J][b][a] = L[t + nrs*J] for a block of nb vectors
-__global__ void k_unpack_block(const int* __restrict__ rs_a, const int* __restrict__ rs_b, int64_t nrs,
-                               const double* __restrict__ L, int nb, int n, double* __restrict__ Lsq) {
-  int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (o >= nrs * nb) return;
-  const int64_t t = o % nrs;
-  const int64_t J = o / nrs;
-  const int a = rs_a[t], b = rs_b[t];
-  const double v = L[t + nrs * J];
-  double* M = Lsq + (size_t)J * n * n;
-  M[(size_t)a * n + b] = v;
-  M[(size_t)b * n + a] = v;
-}
-
 __global__ void k_symmetrize_lower(double* __restrict__ K, int n) {
   int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (o >= (int64_t)n * n) return;
   const int i = (int)(o % n), j = (int)(o / n);
   if (i > j) K[(size_t)i * n + j] = K[(size_t)j * n + i];  // column-major lower -> full
 }
-
-static inline unsigned nb256(int64_t n) { return (unsigned)((n + 255) / 256); }
 
 // F += J - factxi K (CHO_LK_SCF's FLT update)
 __global__ void k_fock_acc(double* __restrict__ F, const double* __restrict__ J, const double* __restrict__ K,
@@ -93,83 +65,6 @@ int fock_accumulate(double* F, const double* J, const double* K, double factxi, 
   g_launches.fetch_add(1, std::memory_order_relaxed);
   if (cudaGetLastError() != cudaSuccess) return MG_ERR_CUDA;
   return cudaStreamSynchronize(st) == cudaSuccess ? 0 : MG_ERR_CUDA;
-}
-
-struct JkWork {
-  int* d_rs_a = nullptr;
-  int* d_rs_b = nullptr;
-  int64_t nrs = 0;
-};
-
-int jk_fp64(Handle* h, const double* d_C, int r, double* d_J, double* d_K, cudaStream_t st, int block) {
-  return jk_fp64_batch(h, 1, &d_C, &r, &d_J, &d_K, st, block);
-}
-
-// FP64 J/K of k densities: every block of vectors is unpacked once, each
-// density runs its DGEMVs, half-transform and DSYRK on the squares.
-int jk_fp64_batch(Handle* h, int k, const double* const* Cs, const int* rs_, double* const* Js, double* const* Ks,
-                  cudaStream_t st, int block) {
-  ChoState* c = h->cho;
-  const int64_t nrs = cho_nrs(c);
-  const int M = cho_nvec(c);
-  const int n = h->nbf;
-  if (k < 1) { h->err = "FP64 J/K: no density"; return MG_ERR_ARG; }
-  int rmax = 0;
-  for (int d = 0; d < k; ++d) {
-    if (!Cs[d] || !Js[d] || !Ks[d] || rs_[d] < 1) { h->err = "FP64 J/K: a density of the batch has no factor or outputs"; return MG_ERR_ARG; }
-    rmax = std::max(rmax, rs_[d]);
-  }
-  cublasHandle_t cb = cho_cublas(c);
-  cublasSetStream(cb, st);
-  const int* d_ra = cho_rs_a_dev(c);
-  const int* d_rb = cho_rs_b_dev(c);
-  // scratch: dw (k nrs), jrs (k nrs), V (block), D (n*n), Lsq (block*n*n), X (n * block * rmax)
-  const size_t need = sizeof(double) * ((size_t)nrs * 2 * k + block + (size_t)n * n + (size_t)block * n * n +
-                                        (size_t)n * block * rmax);
-  double* ws = (double*)ws_get(h, need, st);
-  if (!ws) { h->err = "jk workspace allocation failed"; return MG_ERR_MEMORY; }
-  double* dw = ws;
-  double* jrs = dw + (size_t)nrs * k;
-  double* V = jrs + (size_t)nrs * k;
-  double* D = V + block;
-  double* Lsq = D + (size_t)n * n;
-  double* X = Lsq + (size_t)block * n * n;
-  const double one = 1.0, zero = 0.0;
-  for (int d = 0; d < k; ++d) {
-    // D = C C^T  (C column-major n x r); D symmetric so layout-agnostic
-    cublasDgemm(cb, CUBLAS_OP_N, CUBLAS_OP_T, n, n, rs_[d], &one, Cs[d], n, Cs[d], n, &zero, D, n);
-    k_pack_density<<<nb256(nrs), 256, 0, st>>>(d_ra, d_rb, nrs, D, n, dw + (size_t)d * nrs);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    cudaMemsetAsync(Ks[d], 0, sizeof(double) * n * n, st);
-    cudaMemsetAsync(Js[d], 0, sizeof(double) * n * n, st);  // AO pairs without rows stay zero
-  }
-  cudaMemsetAsync(jrs, 0, sizeof(double) * nrs * k, st);
-  // AO pairs without rows (screened-out shell pairs) stay zero in every square
-  cudaMemsetAsync(Lsq, 0, sizeof(double) * block * n * n, st);
-  for (int J0 = 0; J0 < M; J0 += block) {
-    const int nb = std::min(block, M - J0);
-    // vectors J0.. may straddle storage blocks: gather into a contiguous view
-    const double* Lb = cho_vec_ptr(c, J0, nb, st, h);
-    if (!Lb) { h->err = "vector block gather failed"; return MG_ERR_MEMORY; }
-    k_unpack_block<<<nb256(nrs * nb), 256, 0, st>>>(d_ra, d_rb, nrs, Lb, nb, n, Lsq);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    for (int d = 0; d < k; ++d) {
-      // Coulomb: V = L_b^T dw ; jrs += L_b V
-      cublasDgemv(cb, CUBLAS_OP_T, (int)nrs, nb, &one, Lb, (int)nrs, dw + (size_t)d * nrs, 1, &zero, V, 1);
-      cublasDgemv(cb, CUBLAS_OP_N, (int)nrs, nb, &one, Lb, (int)nrs, V, 1, &one, jrs + (size_t)d * nrs, 1);
-      // Exchange: X_J = Lsq_J C (n x r each), K += X X^T
-      cublasDgemmStridedBatched(cb, CUBLAS_OP_N, CUBLAS_OP_N, n, rs_[d], n, &one, Lsq, n, (long long)n * n, Cs[d], n,
-                                0, &zero, X, n, (long long)n * rs_[d], nb);
-      cublasDsyrk(cb, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_N, n, nb * rs_[d], &one, X, n, &one, Ks[d], n);
-    }
-  }
-  for (int d = 0; d < k; ++d) {
-    k_unpack_sym<<<nb256(nrs), 256, 0, st>>>(d_ra, d_rb, nrs, jrs + (size_t)d * nrs, n, Js[d]);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    k_symmetrize_lower<<<nb256((int64_t)n * n), 256, 0, st>>>(Ks[d], n);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-  }
-  return cudaGetLastError() == cudaSuccess ? 0 : MG_ERR_CUDA;
 }
 
 // ------------------------------------------------------------ mixed path
@@ -465,47 +360,6 @@ __global__ void k_row_absmax(const double* __restrict__ X, int64_t xld, int n, i
   if ((threadIdx.x & 31) == 0 && m > 0.0) atomicMax(xmax + a, (unsigned long long)__double_as_longlong(m));
 }
 
-// jrs[t] += sum_J L[t, J] V[J] over one block of nb FP64 vectors
-__global__ void k_jacc64(const double* __restrict__ L, int64_t nrs, int nb, const double* __restrict__ V,
-                         double* __restrict__ jrs) {
-  int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= nrs) return;
-  double s = 0.0;
-  for (int J = 0; J < nb; ++J) s = fma(L[t + nrs * J], V[J], s);
-  jrs[t] += s;
-}
-
-// jrs_d[t] += sum_J L[t, J] V[d nb + J] for the k densities of a batch,
-// each vector element read once (k_jacc64 for one density)
-__global__ void k_jacc_multi(const double* __restrict__ L, int64_t nrs, int nv, int nb, int k,
-                             const double* __restrict__ V, double* __restrict__ jrs) {
-  int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= nrs) return;
-  double acc[kJkMaxDens];
-#pragma unroll
-  for (int d = 0; d < kJkMaxDens; ++d) acc[d] = 0.0;
-  for (int J = 0; J < nv; ++J) {
-    const double x = L[t + nrs * J];
-#pragma unroll
-    for (int d = 0; d < kJkMaxDens; ++d)
-      if (d < k) acc[d] = fma(x, V[(size_t)d * nb + J], acc[d]);
-  }
-#pragma unroll
-  for (int d = 0; d < kJkMaxDens; ++d)
-    if (d < k) jrs[(size_t)d * nrs + t] += acc[d];
-}
-
-// inv[a*n + b] = inv[b*n + a] = t for every rs pair t (the caller fills inv
-// with -1 first: AO pairs of shell pairs without rows keep it)
-__global__ void k_rs_inverse(const int* __restrict__ rs_a, const int* __restrict__ rs_b, int64_t nrs, int n,
-                             int* __restrict__ inv) {
-  int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= nrs) return;
-  const int a = rs_a[t], b = rs_b[t];
-  inv[(size_t)a * n + b] = (int)t;
-  inv[(size_t)b * n + a] = (int)t;
-}
-
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link
 // dependency on the driver library).
 static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
@@ -660,15 +514,20 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
   int nsm = 148;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
   cublasHandle_t cb = cho_cublas(c);
+  if (!cb) { h->err = "mixed J/K: cublasCreate failed"; return MG_ERR_CUDA; }
   cublasSetStream(cb, st);
   const int* d_ra = cho_rs_a_dev(c);
   const int* d_rb = cho_rs_b_dev(c);
+  const int* inv = cho_inv_dev(c, n, st);
+  if (!inv) { h->err = "mixed J/K: inverse AO-pair table could not be stored"; return MG_ERR_MEMORY; }
   const size_t nn = (size_t)n * n;
   const int ns = (int)h->sh.size();
+  const int jsplit = jacc_splits(nrs, nb, nsm);
   // one term per take() below (each rounded up to 256 bytes)
-  size_t need = 8 * ((size_t)nb * k + 2 * nn) + 4 * nn + (size_t)s * nb * ld * ld + 4 * (size_t)nb * ld +
+  size_t need = 8 * ((size_t)nb * k + 2 * nn) + (size_t)s * nb * ld * ld + 4 * (size_t)nb * ld +
                 8 * (size_t)ld * kxmax + 8 * (size_t)ld + 8 * (size_t)nsm * 128 * 128 + sizeof(int) +
-                4 * (size_t)(ns + 1 + n) + 11 * 256;
+                4 * (size_t)(ns + 1 + n) +
+                8 * (size_t)(jsplit * (size_t)nrs + vmulti_ranges(nrs) * (size_t)nb) * k + 11 * 256;
   for (const OzDens& q : dd)
     need += 16 * (size_t)nrs + (size_t)s * q.npad * ld + 8 * (size_t)q.npad + (size_t)sk * ld * q.xs_row +
             4 * (size_t)G * ld + 6 * 256;
@@ -679,7 +538,6 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
   double* V = (double*)take(8 * (size_t)nb * k);  // V[d nb + J]
   double* D = (double*)take(8 * nn);               // D of the first density (its contraction is fused)
   double* Dt = (double*)take(8 * nn);              // D of a further density, while it is packed
-  int* inv = (int*)take(4 * nn);
   uint8_t* LS = (uint8_t*)take((size_t)s * nb * ld * ld);
   int* eA = (int*)take(4 * (size_t)nb * ld);
   double* Xf = (double*)take(8 * (size_t)ld * kxmax);  // column-major, ld rows
@@ -688,7 +546,8 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
   int* d_err = (int*)take(sizeof(int));
   int* sh_off = (int*)take(4 * (size_t)(ns + 1 + n));
   int* ao_sh = sh_off + ns + 1;
-  double* jrs_all = (double*)take(8 * (size_t)nrs * k);  // jrs of density d at d nrs
+  double* jrs_all = (double*)take(8 * (size_t)nrs * k * jsplit);  // jrs of density d at d nrs, per split
+  double* Vp = (double*)take(8 * (size_t)vmulti_ranges(nrs) * nb * k);
   double* dws = (double*)take(8 * (size_t)nrs * std::max(1, k - 1));
   for (int d = 0; d < k; ++d) {
     OzDens& q = dd[d];
@@ -752,7 +611,7 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
   }
   const double one = 1.0, zero = 0.0;
   if (cudaMemsetAsync(d_err, 0, sizeof(int), st) != cudaSuccess ||
-      cudaMemsetAsync(jrs_all, 0, 8 * nrs * k, st) != cudaSuccess) {
+      cudaMemsetAsync(jrs_all, 0, 8 * (size_t)nrs * k * jsplit, st) != cudaSuccess) {
     h->err = std::string("mixed J/K: clearing buffers: ") + cudaGetErrorString(cudaGetLastError());
     return MG_ERR_CUDA;
   }
@@ -778,9 +637,6 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
     h->err = std::string("mixed J/K: after the density products: ") + cudaGetErrorString(e);
     return MG_ERR_CUDA;
   }
-  cudaMemsetAsync(inv, 0xFF, 4 * nn, st);
-  k_rs_inverse<<<nb256(nrs), 256, 0, st>>>(d_ra, d_rb, nrs, n, inv);
-  if (!launched("k_rs_inverse")) return MG_ERR_CUDA;
   const short* eL = oz_row_exponents(h, inv, ld, st);
   if (!eL) { h->err = "mixed J/K: row exponents could not be stored"; return MG_ERR_MEMORY; }
   for (OzDens& q : dd) {
@@ -804,15 +660,12 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
                 LS, eA, V);
       });
       if (!launched("k_oz_slice_l_blocks")) return MG_ERR_CUDA;
-      if (k == 1) {
-        k_jacc64<<<nb256(nrs), 256, 0, st>>>(Lb, nrs, nv, V, dd[0].jrs);
-        if (!launched("k_jacc64")) return MG_ERR_CUDA;
-      } else {
-        launch_vmulti(Lb, nrs, nv, nb, k - 1, dws, V + nb, st);
+      if (k > 1) {
+        launch_vmulti(Lb, nrs, nv, nb, k - 1, dws, Vp, V + nb, st);
         if (!launched("k_vmulti")) return MG_ERR_CUDA;
-        k_jacc_multi<<<nb256(nrs), 256, 0, st>>>(Lb, nrs, nv, nb, k, V, jrs_all);
-        if (!launched("k_jacc_multi")) return MG_ERR_CUDA;
       }
+      launch_jacc(Lb, nrs, nv, nb, k, jsplit, V, jrs_all, st);
+      if (!launched("k_jacc_multi")) return MG_ERR_CUDA;
       for (OzDens& q : dd) {
         // a short last block: clear the columns of the missing vectors
         if (nv < nb) cudaMemsetAsync(Xf, 0, 8 * (size_t)ld * q.kx, st);
@@ -850,9 +703,8 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
   for (OzDens& q : dd) {
     k_symmetrize_lower<<<nb256((int64_t)nn), 256, 0, st>>>(q.K, n);
     if (!launched("k_symmetrize_lower")) return MG_ERR_CUDA;
-    cudaMemsetAsync(q.J, 0, 8 * nn, st);  // AO pairs without rows
-    k_unpack_sym<<<nb256(nrs), 256, 0, st>>>(d_ra, d_rb, nrs, q.jrs, n, q.J);
-    if (!launched("k_unpack_sym")) return MG_ERR_CUDA;
+    k_finish_j<<<nb256((int64_t)nn), 256, 0, st>>>(inv, q.jrs, jsplit, (int64_t)k * nrs, n, q.J);
+    if (!launched("k_finish_j")) return MG_ERR_CUDA;
   }
   if (const cudaError_t e = cudaGetLastError(); e != cudaSuccess) {
     h->err = std::string("mixed J/K: ") + cudaGetErrorString(e);

@@ -195,6 +195,9 @@ const int* cho_rs_a_dev(const ChoState* c);
 const int* cho_rs_b_dev(const ChoState* c);
 const double* cho_vec_ptr(const ChoState* c, int J0, int nb, cudaStream_t st, Handle* h);
 int cho_vec_block();
+// rs index of every AO pair (n x n device table, -1 where no row is stored),
+// built on first use and owned by the state; nullptr when it cannot be stored
+const int* cho_inv_dev(ChoState* c, int n, cudaStream_t st);
 // first rs index of every shell pair (pair_id order), device
 const int64_t* cho_sp_first_dev(const ChoState* c);
 // cached row exponents of the square Cholesky vectors (M x ld), owned by the state
@@ -206,13 +209,13 @@ int oz_selftest(Handle* h, int ld, int r, int s, const double* d_A, const double
 // (0, 101, 102, -1) or MG_ERR_*; X (n x n, column-major) is overwritten.
 int cd_incore(Handle* h, double* d_X, int n, double thr, double* d_vec, int maxvec, int* numcho, cudaStream_t st);
 int fock_accumulate(double* F, const double* J, const double* K, double factxi, int64_t n, cudaStream_t st);
-int jk_fp64(Handle* h, const double* d_C, int r, double* d_J, double* d_K, cudaStream_t st, int block);
+int jk_fp64(Handle* h, const double* d_C, int r, double* d_J, double* d_K, cudaStream_t st);
 int jk_mixed(Handle* h, const double* d_C, int r, double* d_J, double* d_K, cudaStream_t st, int block, int s, int sk);
 // J/K of k (1..8) densities over one pass of the vectors (jk.cu)
 int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs, double* const* Js, double* const* Ks,
                    cudaStream_t st, int block, int s, int sk);
 int jk_fp64_batch(Handle* h, int k, const double* const* Cs, const int* rs, double* const* Js, double* const* Ks,
-                  cudaStream_t st, int block);
+                  cudaStream_t st);
 
 inline int ncart(int l) { return (l + 1) * (l + 2) / 2; }
 inline int ncart_cum(int l) { return l <= 0 ? 0 : l * (l + 1) * (l + 2) / 6; }
