@@ -11,7 +11,7 @@
 // product, whose error dominates) and both exchange GEMMs run on the tcgen05
 // tensor cores in 8-bit integers with exact INT32 accumulation: per block of
 // vectors, a slicing kernel unpacks the rs-packed L_J into sliced dense
-// squares (and forms the Coulomb contractions V_J on the way), the
+// squares, the
 // half-transform X_J = L_J C writes X in FP64, X is sliced per row over the
 // block, and the exchange product K += X X^T runs over groups of blocks
 // (lower-triangle tiles, CTA-private FP64 tiles, FP64 atomics into K).  J
@@ -20,7 +20,6 @@
 // The FP64 path is in jk64.cu.
 // LK screening is not applied (dense tensor work is cheaper on the GPU than
 // the screening bookkeeping); the result equals the unscreened reference.
-#include <cublas_v2.h>
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -36,15 +35,6 @@
 #include "oz_gemm.cuh"
 
 namespace mg {
-
-// dw[t] = w_t D[a_t, b_t], w = 2 for a != b (both triangles), 1 on the diagonal
-__global__ void k_pack_density(const int* __restrict__ rs_a, const int* __restrict__ rs_b, int64_t nrs,
-                               const double* __restrict__ D, int n, double* __restrict__ dw) {
-  int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= nrs) return;
-  const int a = rs_a[t], b = rs_b[t];
-  dw[t] = (a == b ? 1.0 : 2.0) * D[(size_t)a * n + b];
-}
 
 __global__ void k_symmetrize_lower(double* __restrict__ K, int n) {
   int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -168,89 +158,72 @@ __global__ void k_oz_lexp(const int* __restrict__ inv, int n, int64_t nrs, const
   if (lane == 0) eL[row] = (short)max(-32000, oz_exponent(m));
 }
 
-// L slicing in blocks: one CTA per (256 AOs b, 16 AOs a0..a0+15, vector J).
-// Thread t owns b = c0 + t and loads L_J[a0..a0+16, b] straight from the
-// rs-packed vector, the rs index worked out from the shells of a and b (pair
-// (I, J') with I > J' stores a-fastest, I < J' the mirror, I = J' a
-// triangle, plf_cho_diag.F90:60-72), all 16 loads in flight at once.  L_J is
-// symmetric, so these are also row b, columns a0..a0+15: 16 consecutive K
-// bytes of row b of every slice, cut with row b's cached exponent, packed in
-// registers and written with one 16-byte store per slice (the blocked layout
-// of oz_blk_off).  The grid covers all ld columns a, so the K padding
+// L slicing: the squares of a block of rs-packed vectors, cut into slices.  One
+// CTA per (128 AOs b, 32 AOs a, kOzVecs vectors), two threads per row b with 16
+// columns a each.  The rs indices of a thread's 16 elements are looked up once
+// for all its vectors (the inverse rs table), all 16 vector elements of a
+// vector are in flight at once.  L_J is symmetric, so L_J[a, b] is row b,
+// column a: 16 consecutive K bytes of row b of every slice, cut with row b's
+// cached exponent and packed in registers; the two threads of a row write its
+// 32 bytes of a slice, so a warp's store is 512 contiguous bytes (the blocked
+// layout of oz_blk_off).  The grid covers all ld columns a, so the K padding
 // a >= n is written as zeros (as are the rows b >= n).
-// sh_off[ns + 1]: first AO of every shell (sh_off[ns] = n); ao_sh[n]: the
-// shell of every AO.
-constexpr int kOzChunk = 256;   // AOs b per CTA (= threads)
-constexpr int kOzRows = 16;     // AOs a per CTA
+// Cut: z = x 2^(8S-1-e), rounded to the nearest integer (at most half a unit of
+// the last slice; 2^(8S-1) itself, from a value just below it, becomes the
+// integer before).  For S <= 6 adding 1.5 2^52 leaves the two's-complement
+// integer in the low mantissa bits: three FP64 operations per element.
+// Bound: HBM, S bytes written per element of the squares and the packed vectors
+// read; 1250 functions, 3789 vectors, S = 6: 10.1 ms a call, 54 GB (28.6 ms with a
+// shell-pair lookup per element and vector, a floor, a rounding test and the
+// Coulomb contraction in the same kernel).
+constexpr int kOzCutRows = 128;  // AOs b per CTA
+constexpr int kOzCutCols = 32;   // AOs a per CTA: one MMA K step
+constexpr int kOzVecs = 4;       // vectors per CTA
 
 template <int S>
-__global__ void __launch_bounds__(kOzChunk) k_oz_slice_l_blocks(const int64_t* __restrict__ sp_first,
-                                                                const int* __restrict__ sh_off,
-                                                                const int* __restrict__ ao_sh, int n, int64_t nrs,
-                                                                const double* __restrict__ L, int ld, int64_t slice,
-                                                                const short* __restrict__ eL,
-                                                                const double* __restrict__ D,
-                                                                uint8_t* __restrict__ LS, int* __restrict__ eA,
-                                                                double* __restrict__ V) {
-  __shared__ int rI[kOzRows], rla[kOzRows], rnA[kOzRows];  // shell of a, index in it, its width
-  __shared__ double red[kOzChunk / 32];
-  const int c0 = blockIdx.x * kOzChunk;
-  const int a0 = blockIdx.y * kOzRows;
-  const int J = blockIdx.z;
-  const int nr = max(0, min(kOzRows, n - a0));
-  if ((int)threadIdx.x < nr) {
-    const int r = threadIdx.x, a = a0 + r;
-    const int I = ao_sh[a], aa = sh_off[I];
-    rI[r] = I;
-    rla[r] = a - aa;
-    rnA[r] = sh_off[I + 1] - aa;
-  }
-  __syncthreads();
-  const double* LJ = L + nrs * J;
-  const int b = c0 + threadIdx.x;
-  double x[kOzRows];
-  if (b < n) {
-    // rs indices fit in 32 bits (nrs < 2^31 for n < 65536)
-    const int Jp = ao_sh[b], bb = sh_off[Jp], nB = sh_off[Jp + 1] - bb, lb = b - bb, trib = Jp * (Jp + 1) / 2;
+__global__ void __launch_bounds__(2 * kOzCutRows) k_oz_slice_l(const int* __restrict__ inv, int n, int64_t nrs,
+                                                               const double* __restrict__ L, int nv, int ld,
+                                                               int64_t slice, const short* __restrict__ eL,
+                                                               uint8_t* __restrict__ LS, int* __restrict__ eA) {
+  const int b = blockIdx.x * kOzCutRows + (threadIdx.x >> 1);
+  const int a0 = blockIdx.y * kOzCutCols + 16 * (threadIdx.x & 1);
+  const int J0 = blockIdx.z * kOzVecs, J1 = min(nv, J0 + kOzVecs);
+  int idx[16];
 #pragma unroll
-    for (int r = 0; r < kOzRows; ++r) {
-      x[r] = 0.0;
-      if (r < nr) {
-        // one load for every lane (the lanes of a warp may lie on either side of I)
-        const int I = rI[r], la = rla[r];
-        const int pair = Jp < I ? I * (I + 1) / 2 + Jp : trib + I;
-        const int hi = la >= lb ? la : lb, lo = la >= lb ? lb : la;
-        const int off = Jp < I ? la + rnA[r] * lb : (Jp > I ? lb + nB * la : hi * (hi + 1) / 2 + lo);
-        const int base = (int)__ldg(sp_first + pair);  // -1: a shell pair without rows (screened out)
-        x[r] = base >= 0 ? __ldg(LJ + base + off) : 0.0;
-      }
-    }
-  } else {
-#pragma unroll
-    for (int r = 0; r < kOzRows; ++r) x[r] = 0.0;
-  }
-  // cut, and the Coulomb contraction V_J = sum_ab L_J[a, b] D[a, b] over the
-  // lower triangle (off-diagonal elements twice: L_J and D are symmetric)
-  double v = 0.0;
-  if (b < ld) {
+  for (int r = 0; r < 16; ++r) idx[r] = (b < n && a0 + r < n) ? __ldg(inv + (size_t)(a0 + r) * n + b) : -1;
+  constexpr double kM = 6755399441055744.0;                  // 1.5 2^52
+  constexpr double zmax = (double)((1ull << (8 * (S < 7 ? S : 6) - 1)) - 1);
+  for (int J = J0; J < J1; ++J) {
+    const double* LJ = L + nrs * J;
     const int64_t row = (int64_t)J * ld + b;
     const int e = eL[row];
-    if (blockIdx.y == 0) eA[row] = e;
-    const OzScale sc = oz_scale<S>(e);
-    uint32_t w[S][kOzRows / 4];  // slice p, rows 4 g .. 4 g + 3 (one byte each)
+    if (a0 == 0) eA[row] = e;
+    double x[16];
 #pragma unroll
-    for (int g = 0; g < kOzRows / 4; ++g) {
-      uint32_t lo[4], hi[4];  // the two words of Y for the four rows
+    for (int r = 0; r < 16; ++r) x[r] = idx[r] >= 0 ? __ldg(LJ + idx[r]) : 0.0;
+    // 2^(8S-1-e): one normal factor except for rows below 2^-950
+    const int k = 8 * S - 1 - e, k1 = min(k, 1000);
+    const double f1 = oz_pow2(k1);
+    if (k != k1) {
+      const double f2 = oz_pow2(k - k1);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int r = 4 * g + k, a = a0 + r;
-        if (r < nr && b <= a) v = fma(b < a ? 2.0 * x[r] : x[r], __ldg(D + (size_t)a * n + b), v);
-        const long long y = oz_fixed<S>(x[r], sc);
-        lo[k] = (uint32_t)y;
-        hi[k] = (uint32_t)((unsigned long long)y >> 32);
+      for (int r = 0; r < 16; ++r) x[r] *= f2;
+    }
+    uint32_t w[S][4];  // slice p, columns a0 + 4 g .. + 3 (one byte each)
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      uint32_t lo[4], hi[4];  // the two words of the integers of four columns
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const double z = x[4 * g + q] * f1;
+        long long y;
+        if (S <= 6) y = __double_as_longlong(fmin(z, zmax) + kM);
+        else y = __double2ll_rn(z);  // integral beyond 2^53: nothing rounds up to 2^(8S-1)
+        lo[q] = (uint32_t)y;
+        hi[q] = (uint32_t)((unsigned long long)y >> 32);
       }
-      // byte S-1-p of the four Y into one word: two byte permutes take the
-      // byte from rows (0, 1) and (2, 3), a third joins the halves
+      // byte S-1-p of the four integers into one word: two byte permutes take the
+      // byte from columns (0, 1) and (2, 3), a third joins the halves
 #pragma unroll
       for (int p = 0; p < S; ++p) {
         const int bi = S - 1 - p, kb = bi & 3;
@@ -260,18 +233,10 @@ __global__ void __launch_bounds__(kOzChunk) k_oz_slice_l_blocks(const int64_t* _
         w[p][g] = __byte_perm(s01, s23, 0x5410);
       }
     }
-    uint8_t* dst = LS + oz_blk_off(row, a0, ld, 128);  // a0 % 16 == 0: 16 bytes of one 32-byte chunk
+    uint8_t* dst = LS + oz_blk_off(row, a0, ld, 128);
 #pragma unroll
     for (int p = 0; p < S; ++p)
       *reinterpret_cast<uint4*>(dst + p * slice) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
-  }
-  v = warp_sum(v);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w8 = 0; w8 < kOzChunk / 32; ++w8) t += red[w8];
-    atomicAdd(&V[J], t);
   }
 }
 
@@ -446,7 +411,6 @@ struct OzDens {
   int nnt, Nt, npad, kx, kblk, nsub, ksub;
   int64_t xs_row;
   double* jrs;           // Coulomb in rs layout
-  double* dw;            // packed weighted density (densities after the first)
   uint8_t* CS;           // slices of C
   double* fC;            // column scale factors of C
   uint8_t* XS;           // slices of X for one group of blocks
@@ -461,10 +425,9 @@ int jk_mixed(Handle* h, const double* d_C, int r, double* d_J, double* d_K, cuda
 }
 
 // J/K of k densities over one pass of the vectors: every block of vectors is
-// unpacked and sliced once (with the first density's Coulomb contraction
-// fused), the further densities' contractions take one more read of the
-// block (k_vmulti), J accumulates for all densities in one read
-// (k_jacc_multi), and each density runs its half-transform, X slicing and
+// unpacked and sliced once, the Coulomb contractions of all densities take
+// one read of the block (k_vmulti), J accumulates for all densities in one
+// more (k_jacc_multi), and each density runs its half-transform, X slicing and
 // exchange product on the shared slices.
 int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, double* const* Js, double* const* Ks,
                    cudaStream_t st, int block, int s, int sk) {
@@ -513,46 +476,36 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
   }
   int nsm = 148;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
-  cublasHandle_t cb = cho_cublas(c);
-  if (!cb) { h->err = "mixed J/K: cublasCreate failed"; return MG_ERR_CUDA; }
-  cublasSetStream(cb, st);
   const int* d_ra = cho_rs_a_dev(c);
   const int* d_rb = cho_rs_b_dev(c);
   const int* inv = cho_inv_dev(c, n, st);
   if (!inv) { h->err = "mixed J/K: inverse AO-pair table could not be stored"; return MG_ERR_MEMORY; }
   const size_t nn = (size_t)n * n;
-  const int ns = (int)h->sh.size();
   const int jsplit = jacc_splits(nrs, nb, nsm);
   // one term per take() below (each rounded up to 256 bytes)
-  size_t need = 8 * ((size_t)nb * k + 2 * nn) + (size_t)s * nb * ld * ld + 4 * (size_t)nb * ld +
-                8 * (size_t)ld * kxmax + 8 * (size_t)ld + 8 * (size_t)nsm * 128 * 128 + sizeof(int) +
-                4 * (size_t)(ns + 1 + n) +
-                8 * (size_t)(jsplit * (size_t)nrs + vmulti_ranges(nrs) * (size_t)nb) * k + 11 * 256;
+  size_t need = 8 * (size_t)nb * k + (size_t)s * nb * ld * ld + 4 * (size_t)nb * ld + 8 * (size_t)ld * kxmax +
+                8 * (size_t)ld + 8 * (size_t)nsm * 128 * 128 + sizeof(int) +
+                8 * (size_t)(jsplit * (size_t)nrs + vmulti_ranges(nrs) * (size_t)nb) * k + 10 * 256;
   for (const OzDens& q : dd)
-    need += 16 * (size_t)nrs + (size_t)s * q.npad * ld + 8 * (size_t)q.npad + (size_t)sk * ld * q.xs_row +
+    need += 8 * (size_t)nrs + (size_t)s * q.npad * ld + 8 * (size_t)q.npad + (size_t)sk * ld * q.xs_row +
             4 * (size_t)G * ld + 6 * 256;
   char* ws = (char*)ws_get(h, need, st);
   if (!ws) { h->err = "jk workspace allocation failed"; return MG_ERR_MEMORY; }
   char* const ws_end = ws + need;
   auto take = [&](size_t bytes) { char* p = ws; ws += (bytes + 255) & ~(size_t)255; return (void*)p; };
   double* V = (double*)take(8 * (size_t)nb * k);  // V[d nb + J]
-  double* D = (double*)take(8 * nn);               // D of the first density (its contraction is fused)
-  double* Dt = (double*)take(8 * nn);              // D of a further density, while it is packed
   uint8_t* LS = (uint8_t*)take((size_t)s * nb * ld * ld);
   int* eA = (int*)take(4 * (size_t)nb * ld);
   double* Xf = (double*)take(8 * (size_t)ld * kxmax);  // column-major, ld rows
   unsigned long long* xmax = (unsigned long long*)take(8 * (size_t)ld);
   double* P = (double*)take(8 * (size_t)nsm * 128 * 128);
   int* d_err = (int*)take(sizeof(int));
-  int* sh_off = (int*)take(4 * (size_t)(ns + 1 + n));
-  int* ao_sh = sh_off + ns + 1;
   double* jrs_all = (double*)take(8 * (size_t)nrs * k * jsplit);  // jrs of density d at d nrs, per split
   double* Vp = (double*)take(8 * (size_t)vmulti_ranges(nrs) * nb * k);
-  double* dws = (double*)take(8 * (size_t)nrs * std::max(1, k - 1));
+  double* dws = (double*)take(8 * (size_t)nrs * k);      // packed weighted densities
   for (int d = 0; d < k; ++d) {
     OzDens& q = dd[d];
     q.jrs = jrs_all + (size_t)d * nrs;
-    q.dw = d > 0 ? dws + (size_t)(d - 1) * nrs : nullptr;
     q.CS = (uint8_t*)take((size_t)s * q.npad * ld);
     q.fC = (double*)take(8 * (size_t)q.npad);
     q.XS = (uint8_t*)take((size_t)sk * ld * q.xs_row);
@@ -567,17 +520,6 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
     h->err = std::string("mixed J/K: ") + what + ": " + cudaGetErrorString(e);
     return false;
   };
-  std::vector<int> hoff(ns + 1 + n);
-  for (int i = 0; i < ns; ++i) {
-    hoff[i] = h->sh[i].off;
-    for (int a = h->sh[i].off; a < h->sh[i].off + h->sh[i].nc * h->sh[i].ncomp; ++a) hoff[ns + 1 + a] = i;
-  }
-  hoff[ns] = n;
-  if (const cudaError_t e = cudaMemcpyAsync(sh_off, hoff.data(), 4 * (size_t)(ns + 1 + n), cudaMemcpyHostToDevice, st);
-      e != cudaSuccess) {
-    h->err = std::string("mixed J/K: shell table upload: ") + cudaGetErrorString(e);
-    return MG_ERR_CUDA;
-  }
   CUtensorMap map_l;
   if (!make_slice_map(&map_l, LS, ld, (int64_t)nb * ld, s, 128)) {
     h->err = "tensor maps for the exchange GEMMs could not be encoded";
@@ -609,7 +551,6 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
     ak.ld = ld; ak.n = n; ak.ntile = ntile; ak.nsub = q.nsub; ak.kblk = q.kblk; ak.ksub = q.ksub; ak.eX = q.eX;
     ak.P = P; ak.K = q.K;
   }
-  const double one = 1.0, zero = 0.0;
   if (cudaMemsetAsync(d_err, 0, sizeof(int), st) != cudaSuccess ||
       cudaMemsetAsync(jrs_all, 0, 8 * (size_t)nrs * k * jsplit, st) != cudaSuccess) {
     h->err = std::string("mixed J/K: clearing buffers: ") + cudaGetErrorString(cudaGetLastError());
@@ -621,21 +562,8 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
       h->err = std::string("mixed J/K: clearing K: ") + cudaGetErrorString(cudaGetLastError());
       return MG_ERR_CUDA;
     }
-    // D = C C^T: the first density's is read by the L unpacking, the others are packed over rs
-    double* Dd = d == 0 ? D : Dt;
-    if (const cublasStatus_t bs = cublasDgemm(cb, CUBLAS_OP_N, CUBLAS_OP_T, n, n, q.r, &one, q.C, n, q.C, n, &zero, Dd, n);
-        bs != CUBLAS_STATUS_SUCCESS) {
-      h->err = "mixed J/K: density product (cublasDgemm) failed, status " + std::to_string((int)bs);
-      return MG_ERR_CUDA;
-    }
-    if (d > 0) {
-      k_pack_density<<<nb256(nrs), 256, 0, st>>>(d_ra, d_rb, nrs, Dt, n, q.dw);
-      if (!launched("k_pack_density")) return MG_ERR_CUDA;
-    }
-  }
-  if (const cudaError_t e = cudaGetLastError(); e != cudaSuccess) {
-    h->err = std::string("mixed J/K: after the density products: ") + cudaGetErrorString(e);
-    return MG_ERR_CUDA;
+    k_density_rs<<<nb256(nrs), 256, 0, st>>>(d_ra, d_rb, nrs, q.C, n, q.r, dws + (size_t)d * nrs);
+    if (!launched("k_density_rs")) return MG_ERR_CUDA;
   }
   const short* eL = oz_row_exponents(h, inv, ld, st);
   if (!eL) { h->err = "mixed J/K: row exponents could not be stored"; return MG_ERR_MEMORY; }
@@ -652,18 +580,14 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
       const int nv = std::min(nb, M - J0);
       const double* Lb = cho_vec_ptr(c, J0, nv, st, h);
       if (!Lb) { h->err = "vector block straddles storage blocks"; return MG_ERR_ARG; }
-      cudaMemsetAsync(V, 0, 8 * (size_t)nb * k, st);
       oz_with_slices(s, [&](auto S) {
-        k_oz_slice_l_blocks<decltype(S)::value>
-            <<<dim3((ld + kOzChunk - 1) / kOzChunk, ld / kOzRows, nv), kOzChunk, 0, st>>>(
-                cho_sp_first_dev(c), sh_off, ao_sh, n, nrs, Lb, ld, (int64_t)nb * ld * ld, eL + (size_t)J0 * ld, D,
-                LS, eA, V);
+        k_oz_slice_l<decltype(S)::value>
+            <<<dim3(ld / kOzCutRows, ld / kOzCutCols, (nv + kOzVecs - 1) / kOzVecs), 2 * kOzCutRows, 0, st>>>(
+                inv, n, nrs, Lb, nv, ld, (int64_t)nb * ld * ld, eL + (size_t)J0 * ld, LS, eA);
       });
-      if (!launched("k_oz_slice_l_blocks")) return MG_ERR_CUDA;
-      if (k > 1) {
-        launch_vmulti(Lb, nrs, nv, nb, k - 1, dws, Vp, V + nb, st);
-        if (!launched("k_vmulti")) return MG_ERR_CUDA;
-      }
+      if (!launched("k_oz_slice_l")) return MG_ERR_CUDA;
+      launch_vmulti(Lb, nrs, nv, nb, k, dws, Vp, V, st);
+      if (!launched("k_vmulti")) return MG_ERR_CUDA;
       launch_jacc(Lb, nrs, nv, nb, k, jsplit, V, jrs_all, st);
       if (!launched("k_jacc_multi")) return MG_ERR_CUDA;
       for (OzDens& q : dd) {
