@@ -343,17 +343,21 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 // 8-bit tensor map over s blocked slices of a rows x kx matrix (layout of
 // oz_blk_off: tiles of br rows x 32 bytes, each contiguous), as a 5D tensor
 // (32 bytes, br rows, kx / 32 K steps, rows / br row tiles, s slices); a box
-// is one tile, placed in shared memory with the 32-byte swizzle.
-static bool make_slice_map(CUtensorMap* m, const uint8_t* base, int64_t kx, int64_t rows, int s, int br) {
+// is one tile of the first nbox slices, placed in shared memory one after
+// another with the 32-byte swizzle.
+static bool make_slice_map(CUtensorMap* m, const uint8_t* base, int64_t kx, int64_t rows, int s, int br, int nbox) {
   auto enc = tensor_map_encoder();
-  if (!enc || ((uintptr_t)base & 15) || kx % 32 || br < 8 || br > 256 || br % 8 || rows % br) return false;
+  if (!enc || ((uintptr_t)base & 15) || nbox < 1 || nbox > s || kx % 32 || br < 8 || br > 256 || br % 8 || rows % br) return false;
   cuuint64_t gdim[5] = {32u, (cuuint64_t)br, (cuuint64_t)(kx / 32), (cuuint64_t)(rows / br), (cuuint64_t)s};
   cuuint64_t gstr[4] = {32u, (cuuint64_t)br * 32, (cuuint64_t)(kx * br), (cuuint64_t)(kx * rows)};
-  cuuint32_t box[5] = {32u, (cuuint32_t)br, 1u, 1u, 1u}, es[5] = {1, 1, 1, 1, 1};
+  cuuint32_t box[5] = {32u, (cuuint32_t)br, 1u, 1u, (cuuint32_t)nbox}, es[5] = {1, 1, 1, 1, 1};
   return enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, (void*)base, gdim, gstr, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
              CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
+
+// slices that the second pass of the exchange product loads (its low diagonals)
+static inline int oz_lo_slices(int s) { return std::max(1, s - std::min(s, 4)); }
 
 static inline int rup(int x, int m) { return (x + m - 1) / m * m; }
 
@@ -373,7 +377,7 @@ static void oz_plan(OzArgs& a, int s, int Nt) {
   a.Nt = Nt;
   a.acc_stride = Nt;
   a.nd = std::min(s, 512 / a.acc_stride);
-  a.b_bytes = rup(32 * Nt, 1024);
+  a.b_bytes = 32 * Nt;  // the tiles of a box lie one after another (a multiple of the 256-byte swizzle atom)
   a.stage_bytes = s * (kOzABytes + a.b_bytes);
   a.stages = std::min(kOzMaxStages, (kOzSmemLimit - 1024) / a.stage_bytes);
 }
@@ -415,7 +419,7 @@ struct OzDens {
   double* fC;            // column scale factors of C
   uint8_t* XS;           // slices of X for one group of blocks
   int* eX;               // their row exponents
-  CUtensorMap map_c, map_x;
+  CUtensorMap map_c, map_x, map_xlo;
   OzArgs ax, ak;
 };
 
@@ -521,12 +525,14 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
     return false;
   };
   CUtensorMap map_l;
-  if (!make_slice_map(&map_l, LS, ld, (int64_t)nb * ld, s, 128)) {
+  if (!make_slice_map(&map_l, LS, ld, (int64_t)nb * ld, s, 128, s)) {
     h->err = "tensor maps for the exchange GEMMs could not be encoded";
     return MG_ERR_CUDA;
   }
   for (OzDens& q : dd)
-    if (!make_slice_map(&q.map_c, q.CS, ld, q.npad, s, q.Nt) || !make_slice_map(&q.map_x, q.XS, q.xs_row, ld, sk, 128)) {
+    if (!make_slice_map(&q.map_c, q.CS, ld, q.npad, s, q.Nt, s) ||
+        !make_slice_map(&q.map_x, q.XS, q.xs_row, ld, sk, 128, sk) ||
+        !make_slice_map(&q.map_xlo, q.XS, q.xs_row, ld, sk, 128, oz_lo_slices(sk))) {
       h->err = "tensor maps for the exchange GEMMs could not be encoded";
       return MG_ERR_CUDA;
     }
@@ -601,7 +607,7 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
         const int gx = std::min(ax.nitems, nsm);
         oz_with_slices(s, [&](auto S) {
           oz_gemm_kernel<false, decltype(S)::value><<<gx, kOzThreads, ax.stages * ax.stage_bytes + 1024, st>>>(
-              map_l, q.map_c, ax);
+              map_l, q.map_c, map_l, ax);
         });
         if (!launched("oz_gemm_kernel<false>")) return MG_ERR_CUDA;
         oz_with_slices(sk, [&](auto S) {
@@ -619,7 +625,7 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
       const int gk = std::min(ak.nitems, nsm);
       oz_with_slices(sk, [&](auto S) {
         oz_gemm_kernel<true, decltype(S)::value><<<gk, kOzThreads, ak.stages * ak.stage_bytes + 1024, st>>>(
-            q.map_x, q.map_x, ak);
+            q.map_x, q.map_x, q.map_xlo, ak);
       });
       if (!launched("oz_gemm_kernel<true>")) return MG_ERR_CUDA;
     }
@@ -677,9 +683,10 @@ int oz_selftest(Handle* h, int ld, int r, int s, const double* d_A, const double
   unsigned long long* xmax = (unsigned long long*)take(8 * (size_t)ld);
   double* P = (double*)take(8 * (size_t)nsm * 128 * 128);
   int* d_err = (int*)take(sizeof(int));
-  CUtensorMap map_l, map_c, map_x;
-  if (!make_slice_map(&map_l, LS, ld, ld, s, 128) || !make_slice_map(&map_c, CS, ld, npad, s, Nt) ||
-      !make_slice_map(&map_x, XS, kblk, ld, s, 128))
+  CUtensorMap map_l, map_c, map_x, map_xlo;
+  if (!make_slice_map(&map_l, LS, ld, ld, s, 128, s) || !make_slice_map(&map_c, CS, ld, npad, s, Nt, s) ||
+      !make_slice_map(&map_x, XS, kblk, ld, s, 128, s) ||
+      !make_slice_map(&map_xlo, XS, kblk, ld, s, 128, oz_lo_slices(s)))
     return MG_ERR_CUDA;
   OzArgs ax{}, ak{};
   oz_plan(ax, s, Nt);
@@ -711,7 +718,7 @@ int oz_selftest(Handle* h, int ld, int r, int s, const double* d_A, const double
   });
   oz_with_slices(s, [&](auto S) {
     oz_gemm_kernel<false, decltype(S)::value>
-        <<<std::min(ax.nitems, nsm), kOzThreads, ax.stages * ax.stage_bytes + 1024, st>>>(map_l, map_c, ax);
+        <<<std::min(ax.nitems, nsm), kOzThreads, ax.stages * ax.stage_bytes + 1024, st>>>(map_l, map_c, map_l, ax);
   });
   oz_with_slices(s, [&](auto S) {
     k_oz_slice_x<decltype(S)::value><<<nb256((int64_t)ld * (kblk / 32)), 256, 0, st>>>(d_X, ld, ld, r, ld, kblk, kblk,
@@ -719,7 +726,7 @@ int oz_selftest(Handle* h, int ld, int r, int s, const double* d_A, const double
   });
   oz_with_slices(s, [&](auto S) {
     oz_gemm_kernel<true, decltype(S)::value>
-        <<<std::min(ak.nitems, nsm), kOzThreads, ak.stages * ak.stage_bytes + 1024, st>>>(map_x, map_x, ak);
+        <<<std::min(ak.nitems, nsm), kOzThreads, ak.stages * ak.stage_bytes + 1024, st>>>(map_x, map_x, map_xlo, ak);
   });
   g_launches.fetch_add(6, std::memory_order_relaxed);
   if (cudaGetLastError() != cudaSuccess) return MG_ERR_CUDA;
