@@ -298,18 +298,29 @@ int setup_pairs(Handle* h) {
   return 0;
 }
 
-void* ws_get(Handle* h, size_t bytes, cudaStream_t st) {
-  if (bytes <= h->ws.size) return h->ws.ptr;
-  if (h->ws.ptr) {
+void* keep_get(Workspace& w, size_t bytes, cudaStream_t st) {
+  if (bytes <= w.size) return w.ptr;
+  if (w.ptr) {
     cudaStreamSynchronize(st);
-    cudaFree(h->ws.ptr);
+    cudaFree(w.ptr);
   }
-  h->ws.ptr = nullptr;
-  h->ws.size = 0;
-  size_t sz = std::max(bytes, (size_t)1 << 20);
-  if (dev_malloc(&h->ws.ptr, sz) != cudaSuccess) return nullptr;
-  h->ws.size = sz;
-  return h->ws.ptr;
+  w = Workspace{};
+  const size_t sz = std::max(bytes, (size_t)1 << 20);
+  if (dev_malloc(&w.ptr, sz) != cudaSuccess) return nullptr;
+  w.size = sz;
+  return w.ptr;
+}
+
+void* ws_get(Handle* h, size_t bytes, cudaStream_t st) { return keep_get(h->ws, bytes, st); }
+
+void* pin_get(Handle* h, size_t bytes) {
+  if (bytes <= h->pin.size) return h->pin.ptr;
+  if (h->pin.ptr) cudaFreeHost(h->pin.ptr);
+  h->pin.ptr = nullptr;
+  h->pin.size = 0;
+  if (cudaMallocHost(&h->pin.ptr, bytes) != cudaSuccess) return nullptr;
+  h->pin.size = bytes;
+  return h->pin.ptr;
 }
 
 }  // namespace mg

@@ -22,6 +22,33 @@ std::atomic<long long> g_allocs{0};
 // Accumulator budget (doubles) of one work item: nc * nef <= this.
 static const int kAccBudget = 12288;
 
+// One counter per class (at most 64 classes) ahead of the work items, and the
+// number of items up to which both go up in one copy from the stack.
+static constexpr size_t kCounterBytes = 64 * sizeof(int);
+static constexpr size_t kSmallUpload = 64;
+
+
+int eri_ket_chunk(int nij, int nef) { return nij * nef > kAccBudget ? 0 : std::max(1, kAccBudget / (nij * nef)); }
+
+void eri_class_stats(ClassStats& cs, int nij, int nklc, int ne, int nf, int nsab, int npab, int npcd) {
+  const int nef = ne * nf;
+  cs.max_acc = std::max(cs.max_acc, nij * nklc * nef);
+  cs.max_nef = std::max(cs.max_nef, nef);
+  cs.max_tmp = std::max(cs.max_tmp, nij * nklc * nsab * nf);
+  cs.max_nij = std::max(cs.max_nij, nij);
+  cs.max_npab = std::max(cs.max_npab, npab);
+  cs.max_npcd = std::max(cs.max_npcd, npcd);
+  cs.max_cab = std::max(cs.max_cab, nij * npab);
+  cs.max_ccd = std::max(cs.max_ccd, nklc * npcd);
+  cs.max_ne = std::max(cs.max_ne, ne);
+  cs.max_nf = std::max(cs.max_nf, nf);
+  cs.max_nc = std::max(cs.max_nc, nij * nklc);
+}
+
+ClassPlan eri_plan_for(const Handle* h, int nab, int ncd, const ClassStats& cs, int count) {
+  const int key = nab * 8 + ncd;
+  return eri_plan(nab, ncd, cs, h->eri_tpq[key], h->eri_order[key]);
+}
 
 // Split quartets into work items grouped by (la+lb, lc+ld) class; a work
 // item covers a range of the ket contracted-pair index kl.
@@ -42,11 +69,11 @@ int build_eri_items(Handle* h, const int32_t* q4, int64_t nq, const int64_t* off
     const int nab = P.la + P.lb, ncd = Q.la + Q.lb;
     const int nef = P.ne * Q.ne;
     const int nij = P.nci * P.ncj, nkl = Q.nci * Q.ncj;
-    if (nij * nef > kAccBudget) {
+    const int chunk = eri_ket_chunk(nij, nef);
+    if (!chunk) {
       h->err = "mg_eri_quartets: bra contraction block too large";
       return MG_ERR_ARG;
     }
-    const int chunk = std::max(1, kAccBudget / (nij * nef));
     const int key = nab * 8 + ncd;
     ClassStats& cs = st[key];
     for (int c0 = 0; c0 < nkl; c0 += chunk) {
@@ -58,17 +85,7 @@ int build_eri_items(Handle* h, const int32_t* q4, int64_t nq, const int64_t* off
       it.out_off = offsets[t];
       byc[key].push_back(it);
       const int nklc = it.c1 - it.c0;
-      cs.max_acc = std::max(cs.max_acc, nij * nklc * nef);
-      cs.max_nef = std::max(cs.max_nef, nef);
-      cs.max_tmp = std::max(cs.max_tmp, nij * nklc * P.nsa * P.nsb * Q.ne);
-      cs.max_nij = std::max(cs.max_nij, nij);
-      cs.max_npab = std::max(cs.max_npab, P.np);
-      cs.max_npcd = std::max(cs.max_npcd, Q.np);
-      cs.max_cab = std::max(cs.max_cab, nij * P.np);
-      cs.max_ccd = std::max(cs.max_ccd, nklc * Q.np);
-      cs.max_ne = std::max(cs.max_ne, P.ne);
-      cs.max_nf = std::max(cs.max_nf, Q.ne);
-      cs.max_nc = std::max(cs.max_nc, nij * nklc);
+      eri_class_stats(cs, nij, nklc, P.ne, Q.ne, P.nsa * P.nsb, P.np, Q.np);
       // primitive quartets x roots x (e0|f0) components, plus the contraction
       cs.work += (double)P.np * Q.np * (nab + ncd + 2) / 2 * nef + (double)nij * nklc * nef;
     }
@@ -83,7 +100,7 @@ int build_eri_items(Handle* h, const int32_t* q4, int64_t nq, const int64_t* off
     c.ncd = key % 8;
     c.begin = items.size();
     c.count = v.size();
-    c.plan = eri_plan(c.nab, c.ncd, st[key], h->eri_tpq[key], h->eri_order[key]);
+    c.plan = eri_plan_for(h, c.nab, c.ncd, st[key], c.count);
     c.work = st[key].work;
     if (c.plan.PAB < 1) {
       h->err = "mg_eri_quartets: class does not fit in shared memory";
@@ -104,18 +121,26 @@ int build_eri_items(Handle* h, const int32_t* q4, int64_t nq, const int64_t* off
 int run_eri_items(Handle* h, const std::vector<EriItem>& items, const std::vector<EriClass>& classes, double* d_out,
                   cudaStream_t st) {
   if (items.empty()) return 0;
-  if (!h->d_eri_counters && dev_malloc(&h->d_eri_counters, sizeof(int) * 64) != cudaSuccess) {
-    h->err = "ERI work counters: allocation failed";
-    return MG_ERR_MEMORY;
+  // work counters of the classes (64 zeros), then the items: one upload
+  char* d = (char*)ws_get(h, kCounterBytes + sizeof(EriItem) * items.size(), st);
+  if (!d) { h->err = "workspace allocation failed"; return MG_ERR_MEMORY; }
+  int* d_counters = (int*)d;
+  EriItem* d_items = (EriItem*)(d + kCounterBytes);
+  if (items.size() <= kSmallUpload) {
+    char up[kCounterBytes + sizeof(EriItem) * kSmallUpload];
+    memset(up, 0, kCounterBytes);
+    memcpy(up + kCounterBytes, items.data(), sizeof(EriItem) * items.size());
+    cudaMemcpyAsync(d, up, kCounterBytes + sizeof(EriItem) * items.size(), cudaMemcpyHostToDevice, st);
+  } else {
+    cudaMemsetAsync(d, 0, kCounterBytes, st);
+    cudaMemcpyAsync(d_items, items.data(), sizeof(EriItem) * items.size(), cudaMemcpyHostToDevice, st);
   }
-  EriItem* d_items = (EriItem*)ws_get(h, sizeof(EriItem) * items.size(), st);
-  if (!d_items) { h->err = "workspace allocation failed"; return MG_ERR_MEMORY; }
-  cudaMemcpyAsync(d_items, items.data(), sizeof(EriItem) * items.size(), cudaMemcpyHostToDevice, st);
-  cudaMemsetAsync(h->d_eri_counters, 0, sizeof(int) * 64, st);
   // The class kernels are independent (own counter, own output blocks): spread them over
   // the handle's side streams so that the tail of one class overlaps the next class,
-  // the largest classes first (the small ones fill in behind them).
-  int rc = side_streams_fork(h, st);
+  // the largest classes first (the small ones fill in behind them).  One class stays on
+  // the caller's stream (a fork and join of the streams costs as much as its launch).
+  const int nside = (h->eri_profile || classes.size() == 1) ? 0 : std::min<int>((int)classes.size(), MG_ERI_STREAMS);
+  int rc = nside ? side_streams_fork(h, st, nside) : 0;
   if (rc) return rc;
   std::vector<int> order(classes.size());
   for (size_t k = 0; k < order.size(); ++k) order[k] = (int)k;
@@ -134,43 +159,39 @@ int run_eri_items(Handle* h, const std::vector<EriItem>& items, const std::vecto
   for (size_t k = 0; k < order.size(); ++k) {
     const int ci = order[k];
     const EriClass& c = classes[ci];
-    const cudaStream_t ks = h->eri_profile ? st : h->eri_streams[k % MG_ERI_STREAMS];
+    const cudaStream_t ks = nside ? h->eri_streams[k % nside] : st;
     if (h->eri_profile) {
       h->eri_ev_key[k] = c.nab * 8 + c.ncd;
       h->eri_ev_plan[k] = c.plan;
       cudaEventRecord(h->eri_ev[2 * k], ks);
     }
-    if (eri_launch_class(h, d_items + c.begin, c.count, c.nab, c.ncd, c.plan, d_out, h->d_eri_counters + ci, ks)) {
+    if (eri_launch_class(h, d_items + c.begin, c.count, c.nab, c.ncd, c.plan, d_out, d_counters + ci, ks)) {
       h->err = std::string("ERI kernel launch failed: ") + cudaGetErrorString(cudaGetLastError());
       return MG_ERR_CUDA;
     }
     if (h->eri_profile) cudaEventRecord(h->eri_ev[2 * k + 1], ks);
   }
-  side_streams_join(h, st);
+  side_streams_join(h, st, nside);
   return 0;
 }
 
-int side_streams_fork(Handle* h, cudaStream_t st) {
-  if (!h->eri_streams[0]) {
-    for (int k = 0; k < MG_ERI_STREAMS; ++k) {
-      if (cudaStreamCreateWithFlags(&h->eri_streams[k], cudaStreamNonBlocking) != cudaSuccess ||
-          cudaEventCreateWithFlags(&h->eri_events[k], cudaEventDisableTiming) != cudaSuccess) {
-        h->err = "side streams could not be created";
-        return MG_ERR_CUDA;
-      }
-    }
-    if (cudaEventCreateWithFlags(&h->eri_fork, cudaEventDisableTiming) != cudaSuccess) {
-      h->err = "side streams could not be created";
-      return MG_ERR_CUDA;
-    }
+int side_streams_fork(Handle* h, cudaStream_t st, int n) {
+  bool ok = h->eri_fork || cudaEventCreateWithFlags(&h->eri_fork, cudaEventDisableTiming) == cudaSuccess;
+  for (int k = 0; k < n && ok; ++k)  // (a stream costs some 130 us to create)
+    if (!h->eri_streams[k])
+      ok = cudaStreamCreateWithFlags(&h->eri_streams[k], cudaStreamNonBlocking) == cudaSuccess &&
+           cudaEventCreateWithFlags(&h->eri_events[k], cudaEventDisableTiming) == cudaSuccess;
+  if (!ok) {
+    h->err = "side streams could not be created";
+    return MG_ERR_CUDA;
   }
   cudaEventRecord(h->eri_fork, st);
-  for (int k = 0; k < MG_ERI_STREAMS; ++k) cudaStreamWaitEvent(h->eri_streams[k], h->eri_fork, 0);
+  for (int k = 0; k < n; ++k) cudaStreamWaitEvent(h->eri_streams[k], h->eri_fork, 0);
   return 0;
 }
 
-void side_streams_join(Handle* h, cudaStream_t st) {
-  for (int k = 0; k < MG_ERI_STREAMS; ++k) {
+void side_streams_join(Handle* h, cudaStream_t st, int n) {
+  for (int k = 0; k < n; ++k) {
     cudaEventRecord(h->eri_events[k], h->eri_streams[k]);
     cudaStreamWaitEvent(st, h->eri_events[k], 0);
   }
@@ -188,6 +209,10 @@ int mg_create(const char* rys_table_path, int device, mg_handle** out) {
   if (cudaSetDevice(device) != cudaSuccess) return MG_ERR_CUDA;
   mg_handle* H = new mg_handle;
   H->h.device = device;
+  if (cudaDeviceGetAttribute(&H->h.nsm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+    delete H;
+    return MG_ERR_CUDA;
+  }
   int rc = load_rys_table(&H->h, rys_table_path);
   if (rc) {
     delete H;
@@ -213,7 +238,6 @@ int mg_destroy(mg_handle* H) {
   cudaSetDevice(h->device);
   free_basis(h);
   cudaFree(h->d_rys);
-  cudaFree(h->d_eri_counters);
   cudaFree(h->d_lk);
   cudaFree(h->d_dcd);
   for (int k = 0; k < MG_ERI_STREAMS; ++k) {
@@ -223,7 +247,8 @@ int mg_destroy(mg_handle* H) {
   if (h->eri_fork) cudaEventDestroy(h->eri_fork);
   for (cudaEvent_t e : h->grad_ev) cudaEventDestroy(e);
   for (cudaEvent_t e : h->eri_ev) cudaEventDestroy(e);
-  if (h->ws.ptr) cudaFree(h->ws.ptr);
+  for (Workspace* w : {&h->ws, &h->cho_scr, &h->cho_buf, &h->cho_lq, &h->cho_upd}) cudaFree(w->ptr);
+  if (h->pin.ptr) cudaFreeHost(h->pin.ptr);
   delete H;
   return 0;
 }
@@ -466,7 +491,7 @@ int mg_cho_drv(mg_handle* H, const mg_cho_cfg* cfg, void* stream) {
   Handle* h = &H->h;
   if (h->pairs.empty()) { h->err = "mg_cho_drv: no basis"; return MG_ERR_ARG; }
   cudaSetDevice(h->device);
-  cho_free(h->cho);
+  cho_recycle(h, h->cho);
   h->cho = nullptr;
   ChoCfgH c;
   c.thrcom = cfg->thrcom;

@@ -8,16 +8,17 @@
 //   columns    (CD|AB) all CD      cho_mca_calcint_1.F90 + PLF_Cho
 //   Dec_Qual   Q = MQ - LQ LQ^T    cho_dec_qual.F90:57-83 (Thr = max(ThrCom, Dmax Span))
 //   CD_InCore_1p pivot rule        cd_incore_1p.F90:33-85 (Acc tie rule, host FP64)
-//   Subtr      X -= L LQ^T         cho_vecbuf_subtr.F90:188-215 (DGEMM)
+//   Subtr      X -= L LQ^T         cho_vecbuf_subtr.F90:188-215
 //   CompVec    scale/diag update   cho_compvec.F90:40-120 + Cho_ChkDia_A4
 //   SetRed     damped screening    cho_setred.F90:72-100 (MODE_SCREEN 1)
 //
-// Device work: ERI diagonal and columns (eri.cu kernels), column gather,
-// DGEMM, row-parallel CompVec, reductions.  Host work per pass: the choice
-// of shell pair, the qualification list and the in-core CD of the <=100 x 100
-// qualified block (sequential, exact reference semantics).  Vectors are FP64
-// in reduced-set ("rs") layout, blocks of kVecBlock columns.
-#include <cublas_v2.h>
+// Device work: ERI diagonal and columns (eri.cu kernels), the reduced set and
+// the choice of shell pair, the qualified block, and one fused kernel for the
+// new vectors.  Host work per pass: the qualification list, the work items and
+// the in-core CD of the <=100 x 100 qualified block (sequential, exact
+// reference semantics); it waits for the device twice (the chosen pair, the
+// qualified block).  Vectors are FP64 in reduced-set ("rs") layout, blocks of
+// kVecBlock columns.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -31,7 +32,9 @@
 
 namespace mg {
 
-// from capi.cu
+constexpr int kVecBlock = 1024;  // vectors per storage block
+// largest buffer of a decomposition that the handle keeps for the next one
+constexpr size_t kKeepBytes = (size_t)256 << 20;
 
 // ------------------------------------------------------------------ kernels
 // rs descriptor: AO pair (a,b) with its shell pair and local indices
@@ -58,119 +61,357 @@ __global__ void k_extract_diag(const RsDev* __restrict__ rs, int64_t nrs, const 
   diag[t] = blk[blk_off[r.sp] + ijkl + nijkl * (sab + (int64_t)nsab * sab)];
 }
 
-// xint[t + nrs*q] = (row_t | col_q) from the (CD|AB) blocks; 0 outside the
-// reduced set.  col: the rs index of each qualified column (all in pair AB).
-__global__ void k_gather_columns(const RsDev* __restrict__ rs, int64_t nrs, const unsigned char* __restrict__ inred,
-                                 const DPair* __restrict__ pairs, const int64_t* __restrict__ blk_off,
-                                 const double* __restrict__ blk, const int* __restrict__ cols, int ncol, int spab,
-                                 double* __restrict__ xint) {
-  int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= nrs) return;
-  if (!inred[t]) {
-    for (int q = 0; q < ncol; ++q) xint[t + nrs * q] = 0.0;
-    return;
+// Element (row | col) of the (CD|AB) block of row's shell pair (Eval_IJKL
+// layout); col belongs to the ket pair A.
+__device__ __forceinline__ double cho_blk(const double* __restrict__ blk, const RsDev& r, const DPair& C, const RsDev& c,
+                                          const DPair& A) {
+  const int nij = C.nci * C.ncj, nijkl = nij * A.nci * A.ncj;
+  return __ldg(blk + r.ka + C.nci * r.kb + (int64_t)nij * (c.ka + A.nci * c.kb) +
+               (int64_t)nijkl * (r.ma + C.nsa * r.mb + (int64_t)C.nsa * C.nsb * (c.ma + A.nsa * c.mb)));
+}
+
+// One warp per shell pair: Cho_SetRed mode 1 of the pass just done (no abs:
+// keep diag > 0 with sqrt(diag xm) damp > thrcom, xm the largest |diagonal|,
+// nothing once xm <= thrcom; apply = 0 before the first pass), then the
+// pair's maxima (CHO_SETMAXSHL): diash[sp] = max(0, largest diagonal) over its
+// members in the reduced set, -1 when none is in it, diash[nsp + sp] their
+// largest |diagonal|; alive[sp] = some member is in the reduced set.
+__global__ void k_cho_scan(const double* __restrict__ diag, unsigned char* __restrict__ inred,
+                           const int64_t* __restrict__ sp_first, const int* __restrict__ sp_count, int nsp,
+                           const unsigned long long* __restrict__ xmbits, int apply, double damp, double thrcom,
+                           double* __restrict__ diash, unsigned char* __restrict__ alive) {
+  const int sp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (sp >= nsp) return;
+  const double xm = __longlong_as_double((long long)*xmbits);
+  const bool conv = !(xm > thrcom);
+  double m = -1.0, ma = 0.0;
+  const int64_t f = sp_first[sp];
+  for (int i = lane; i < sp_count[sp]; i += 32) {
+    if (!inred[f + i]) continue;
+    const double d = diag[f + i];
+    if (apply && (conv || !(d > 0.0 && sqrt(d * xm) * damp > thrcom))) {
+      inred[f + i] = 0;
+      continue;
+    }
+    m = fmax(m, fmax(d, 0.0));
+    ma = fmax(ma, fabs(d));
   }
-  const RsDev r = rs[t];
-  const DPair& C = pairs[r.sp];
-  const DPair& A = pairs[spab];
-  const int64_t base = blk_off[r.sp];
-  const int nij = C.nci * C.ncj, nkl = A.nci * A.ncj;
-  const int64_t nijkl = (int64_t)nij * nkl;
-  const int ij = r.ka + C.nci * r.kb;
-  const int sab = r.ma + C.nsa * r.mb, nsab = C.nsa * C.nsb;
-  for (int q = 0; q < ncol; ++q) {
-    const RsDev c = rs[cols[q]];
-    const int kl = c.ka + A.nci * c.kb;
-    const int scd = c.ma + A.nsa * c.mb;
-    xint[t + nrs * q] = blk[base + ij + (int64_t)nij * kl + nijkl * (sab + (int64_t)nsab * scd)];
+  for (int o = 16; o > 0; o >>= 1) {
+    m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    ma = fmax(ma, __shfl_xor_sync(0xffffffffu, ma, o));
+  }
+  if (lane == 0) {
+    diash[sp] = m;
+    diash[nsp + sp] = ma;
+    alive[sp] = m >= 0.0;
   }
 }
 
-// block max over the reduced set: out[0] = max |diag|, out[1] = max diag
-__global__ void k_red_max(const double* __restrict__ diag, const unsigned char* __restrict__ inred, int64_t n,
-                          double* __restrict__ out) {
-  __shared__ double s0[256], s1[256];
-  double m0 = 0.0, m1 = -1e300;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x)
-    if (inred[t]) {
-      m0 = fmax(m0, fabs(diag[t]));
-      m1 = fmax(m1, diag[t]);
-    }
-  s0[threadIdx.x] = m0;
-  s1[threadIdx.x] = m1;
+// What the host reads once per pass, at the head of one buffer: then the
+// diagonals (maxcnt doubles) and reduced-set flags (maxcnt bytes) of the chosen
+// shell pair and alive[nsp].
+struct ChoSel {
+  double dgmax, smax;  // largest |diagonal|; the chosen pair's maximum
+  int spab, flags;     // the chosen pair; error flags of the update kernel
+  long long pad;
+};
+
+// Cho_SetPass / Cho_GetMaxShl: the largest |diagonal|, and the shell pair of
+// the largest diagonal above thrcom (the first of equal ones; diagonals at or
+// below thrcom count as 0).  One CTA; clears xm for the next pass.
+__global__ void __launch_bounds__(1024) k_cho_select(const double* __restrict__ diash, int nsp, double thrcom,
+                                                     const int64_t* __restrict__ sp_first,
+                                                     const int* __restrict__ sp_count, const double* __restrict__ diag,
+                                                     const unsigned char* __restrict__ inred,
+                                                     const int* __restrict__ flags, unsigned long long* __restrict__ xm,
+                                                     ChoSel* __restrict__ sel, double* __restrict__ dpair,
+                                                     unsigned char* __restrict__ rpair) {
+  __shared__ double sg[32], sv[32];
+  __shared__ int si[32];
+  double g = 0.0, v = -1.0;
+  int idx = 0x7fffffff;
+  for (int sp = threadIdx.x; sp < nsp; sp += blockDim.x) {
+    const double x = diash[sp] > thrcom ? diash[sp] : 0.0;
+    if (x > v) { v = x; idx = sp; }
+    g = fmax(g, diash[nsp + sp]);
+  }
+  auto join = [&](double g2, double v2, int i2) {
+    g = fmax(g, g2);
+    if (v2 > v || (v2 == v && i2 < idx)) { v = v2; idx = i2; }
+  };
+  for (int o = 16; o > 0; o >>= 1) {
+    const double g2 = __shfl_xor_sync(0xffffffffu, g, o), v2 = __shfl_xor_sync(0xffffffffu, v, o);
+    const int i2 = __shfl_xor_sync(0xffffffffu, idx, o);
+    join(g2, v2, i2);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    sg[threadIdx.x >> 5] = g;
+    sv[threadIdx.x >> 5] = v;
+    si[threadIdx.x >> 5] = idx;
+  }
   __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) {
-      s0[threadIdx.x] = fmax(s0[threadIdx.x], s0[threadIdx.x + w]);
-      s1[threadIdx.x] = fmax(s1[threadIdx.x], s1[threadIdx.x + w]);
+  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) join(sg[w], sv[w], si[w]);
+  if (threadIdx.x == 0) {
+    sel->dgmax = g;
+    sel->smax = v;
+    sel->spab = idx;
+    sel->flags = *flags;
+    *xm = 0;
+  }
+  const int64_t f = sp_first[idx];
+  for (int i = threadIdx.x; i < sp_count[idx]; i += blockDim.x) {
+    dpair[i] = diag[f + i];
+    rpair[i] = inred[f + i];
+  }
+}
+
+// LQ: the rows of the previous vectors at the nq qualified AO pairs,
+// lq[J nq + i] = L[rows[i], J], and this CTA's share of LQ LQ^T (lower
+// triangle, jb vectors at a time, in part[blockIdx.x nq^2 ..]).  Lt: the
+// storage blocks of kVecBlock vectors.
+__global__ void __launch_bounds__(256) k_cho_lq(const double* const* __restrict__ Lt, int64_t nrs, int M,
+                                                const int* __restrict__ rows, int nq, int jb,
+                                                double* __restrict__ lq, double* __restrict__ part) {
+  extern __shared__ double cq_sl[];  // jb x nq
+  double* pb = part + (size_t)blockIdx.x * nq * nq;
+  bool first = true;
+  for (int j0 = blockIdx.x * jb; j0 < M; j0 += gridDim.x * jb, first = false) {
+    const int nj = min(jb, M - j0);
+    for (int o = threadIdx.x; o < nj * nq; o += blockDim.x) {
+      const int jj = o / nq, i = o - jj * nq, J = j0 + jj;
+      const double v = Lt[J / kVecBlock][rows[i] + nrs * (J % kVecBlock)];
+      cq_sl[o] = v;
+      lq[(size_t)J * nq + i] = v;
+    }
+    __syncthreads();
+    for (int o = threadIdx.x; o < nq * nq; o += blockDim.x) {
+      const int j = o / nq, i = o - j * nq;
+      if (i < j) continue;
+      double s = first ? 0.0 : pb[o];
+      for (int jj = 0; jj < nj; ++jj) s = fma(cq_sl[jj * nq + i], cq_sl[jj * nq + j], s);
+      pb[o] = s;
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
-    out[2 * blockIdx.x] = s0[0];
-    out[2 * blockIdx.x + 1] = s1[0];
-  }
 }
 
-// per shell pair max diag over the reduced set (CHO_SETMAXSHL)
-__global__ void k_sp_max(const double* __restrict__ diag, const unsigned char* __restrict__ inred,
-                         const int64_t* __restrict__ sp_first, const int* __restrict__ sp_count, int nsp,
-                         double* __restrict__ diash) {
-  int sp = blockIdx.x * blockDim.x + threadIdx.x;
-  if (sp >= nsp) return;
-  // diash[sp]: max(0, largest diagonal) over the pair's members in the
-  // reduced set, -1 when none is in it; diash[nsp + sp]: their largest |diagonal|
-  double m = -1.0, ma = 0.0;
-  const int64_t f = sp_first[sp];
-  for (int i = 0; i < sp_count[sp]; ++i)
-    if (inred[f + i]) {
-      m = fmax(m, fmax(diag[f + i], 0.0));
-      ma = fmax(ma, fabs(diag[f + i]));
+// Cho_Dec_Qual: Q = MQ - LQ LQ^T, MQ the integrals among the qualified AO
+// pairs (all of shell pair spab), the shares summed in a fixed order.
+__global__ void k_cho_q(const RsDev* __restrict__ rs, const DPair* __restrict__ pairs,
+                        const double* __restrict__ blk, const int* __restrict__ rows, int nq, int spab,
+                        const double* __restrict__ part, int nparts, double* __restrict__ Q) {
+  const int o = blockIdx.x * blockDim.x + threadIdx.x;
+  if (o >= nq * nq) return;
+  const int j = o / nq, i = o - j * nq;
+  const DPair& A = pairs[spab];
+  const RsDev r = rs[rows[i]], c = rs[rows[j]];
+  const size_t lo = i >= j ? (size_t)j * nq + i : (size_t)i * nq + j;
+  double s = 0.0;
+  for (int p = 0; p < nparts; ++p) s += part[(size_t)p * nq * nq + lo];
+  Q[o] = cho_blk(blk, r, A, c, A) - s;
+}
+
+// Cho_Subtr and Cho_CompVec of one pass, for the pivots i0 .. i0 + ni (at most
+// 32 at a time; later launches count the earlier pivots' vectors as previous
+// ones, their LQ rows being those of K):
+//   k_cho_subtr    s_i = sum_J L[t, J] LQ[i, J] over a range of the previous
+//                  vectors (blockIdx.y), two rows per thread, into part[range]
+//   k_cho_compvec  gather the integral columns straight from the ERI blocks,
+//                  x_i -= s_i (the ranges in order), scale, diagonal update,
+//                  Cho_ChkDia_A4, x_j -= K_ji x_i, and store the new columns
+// Rows are independent: the reference's per-vector steps touch each row only
+// through its own diagonal.  Rows outside the reduced set read nothing and get
+// zeros.  The previous vectors are the only large operand, read once against
+// NK FMAs per element, so HBM bounds k_cho_subtr up to NK = 16 and the FP64 pipe
+// above; the ranges are there for small systems, whose rows alone neither fill
+// the chip nor hide the latency of one serial pass over the vectors.
+// par: fac[nk] | K[nk x nk] (column i: vector i); ipar: qrs[nk] | colsel[nk].
+constexpr int kUpdThreads = 128;
+constexpr int kUpdRows = 2 * kUpdThreads;  // rows per CTA of k_cho_subtr
+constexpr int kUpdJ = 32;                  // vectors per shared-memory chunk (divides kVecBlock)
+
+struct ChoUpd {
+  double* const* Lt;
+  int64_t nrs;
+  int M, i0, ni, nk, nq, spab, last;
+  int jper, nrange;     // previous vectors per range (a multiple of kUpdJ), ranges
+  double* part;         // [range][i][nrs]
+  const double* lq;
+  const double* blk;
+  const int64_t* base;  // first element of a shell pair's bra block (times ksz)
+  int64_t ksz;          // elements of the ket block
+  const RsDev* rs;
+  const DPair* pairs;
+  const unsigned char* inred;
+  double* diag;
+  const double* par;
+  const int* ipar;
+  double qdmax, damp, thrcom, thrneg, tooneg;
+  int* flags;
+  unsigned long long* xm;
+};
+
+template <int NK>
+__global__ void __launch_bounds__(kUpdThreads) k_cho_subtr(const ChoUpd u) {
+  constexpr int KV = (kUpdJ * NK + kUpdThreads - 1) / kUpdThreads;  // LQ values a thread stages
+  __shared__ __align__(16) double sl[2][kUpdJ][NK];
+  __shared__ int ssel[NK];
+  const int tid = threadIdx.x;
+  const int64_t t0 = blockIdx.x * (int64_t)kUpdRows + tid, t1 = t0 + kUpdThreads;
+  const bool a0 = t0 < u.nrs && u.inred[t0], a1 = t1 < u.nrs && u.inred[t1];
+  if (tid < NK) ssel[tid] = tid < u.ni ? u.ipar[u.nk + u.i0 + tid] : 0;
+  const int jb = blockIdx.y * u.jper, je = min(u.M + u.i0, jb + u.jper);
+  if (!__syncthreads_or(a0 || a1)) return;
+  double acc[2][NK], lqv[KV];
+#pragma unroll
+  for (int i = 0; i < NK; ++i) acc[0][i] = acc[1][i] = 0.0;
+  auto stage = [&](int j0) {
+#pragma unroll
+    for (int v = 0; v < KV; ++v) {
+      const int o = tid + v * kUpdThreads, jj = o / NK, i = o - jj * NK;
+      lqv[v] = (o < kUpdJ * NK && j0 + jj < je && i < u.ni) ? __ldg(u.lq + (size_t)(j0 + jj) * u.nq + ssel[i]) : 0.0;
     }
-  diash[sp] = m;
-  diash[nsp + sp] = ma;
-}
-
-// Cho_CompVec for one pass, one thread per rs row (rows are independent:
-// the reference's per-vector steps touch each row only through its own
-// diagonal).  X: nrs x nk (column-major, this pass's columns after Subtr).
-// K: nk x nk lower triangular in-block vectors; fac[i] = 1/sqrt(|QDiag_i|);
-// qrs[i]: parent rs of vector i.  flags[0] set if a diagonal < TooNeg.
-__global__ void k_compvec(double* __restrict__ X, int64_t nrs, int nk, const double* __restrict__ K,
-                          const double* __restrict__ fac, const int* __restrict__ qrs, double* __restrict__ diag,
-                          const unsigned char* __restrict__ inred, double qdmax, double damp, double thrcom,
-                          double thrneg, double tooneg, int* __restrict__ flags) {
-  int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= nrs) return;
-  if (!inred[t]) {  // vectors are zero outside the reduced set of their pass
-    for (int i = 0; i < nk; ++i) X[t + nrs * i] = 0.0;
-    return;
-  }
-  double d = diag[t];
-  for (int i = 0; i < nk; ++i) {
-    double x = X[t + nrs * i] * fac[i];
-    if (d == 0.0) x = 0.0;
-    d -= x * x;
-    if (t == qrs[i]) d = 0.0;  // Cho_P_ZeroDiag
-    if (d < 0.0 && d < thrneg) {  // Cho_ChkDia_A4
-      if (d < tooneg) atomicOr(flags, 1);
-      d = 0.0;
+  };
+  stage(jb);
+  int s = 0;
+  for (int j0 = jb; j0 < je; j0 += kUpdJ, s ^= 1) {
+    double* sf = &sl[s][0][0];
+#pragma unroll
+    for (int v = 0; v < KV; ++v)
+      if (tid + v * kUpdThreads < kUpdJ * NK) sf[tid + v * kUpdThreads] = lqv[v];
+    __syncthreads();
+    if (j0 + kUpdJ < je) stage(j0 + kUpdJ);
+    const int nj = min(kUpdJ, je - j0);
+    const double* Lp = u.Lt[j0 / kVecBlock] + u.nrs * (j0 % kVecBlock);
+    for (int q = 0; q < nj; q += 8) {
+      double x0[8], x1[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const double* p = Lp + u.nrs * (q + e);
+        x0[e] = a0 && q + e < nj ? __ldg(p + t0) : 0.0;
+        x1[e] = a1 && q + e < nj ? __ldg(p + t1) : 0.0;
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+#pragma unroll
+        for (int i = 0; i < NK; ++i) {
+          const double l = sl[s][q + e][i];
+          acc[0][i] = fma(x0[e], l, acc[0][i]);
+          acc[1][i] = fma(x1[e], l, acc[1][i]);
+        }
     }
-    if (sqrt(fabs(d) * qdmax) * damp <= thrcom) d = 0.0;
-    X[t + nrs * i] = x;
-    for (int j = i + 1; j < nk; ++j) X[t + nrs * j] -= K[j + nk * i] * x;
   }
-  diag[t] = d;
+  double* p = u.part + (size_t)blockIdx.y * u.ni * u.nrs;
+#pragma unroll
+  for (int i = 0; i < NK; ++i) {
+    if (i >= u.ni) break;
+    if (a0) p[(size_t)i * u.nrs + t0] = acc[0][i];
+    if (a1) p[(size_t)i * u.nrs + t1] = acc[1][i];
+  }
 }
 
-// Cho_SetRed mode 1 (no abs): keep diag > 0 with sqrt(diag*xm)*damp > thrcom
-__global__ void k_setred(const double* __restrict__ diag, unsigned char* __restrict__ inred, int64_t n, double xm,
-                         double damp, double thrcom, int conv) {
-  int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  if (!inred[t]) return;
-  const double d = diag[t];
-  inred[t] = (!conv && d > 0.0 && sqrt(d * xm) * damp > thrcom) ? 1 : 0;
+template <int NK>
+__global__ void __launch_bounds__(kUpdThreads) k_cho_compvec(const ChoUpd u) {
+  __shared__ double sK[NK * NK], sfac[NK], smax[kUpdThreads / 32];
+  __shared__ int sq[NK];
+  const int tid = threadIdx.x;
+  const int64_t t = blockIdx.x * (int64_t)kUpdThreads + tid;
+  const bool act = t < u.nrs && u.inred[t];
+  for (int o = tid; o < NK; o += kUpdThreads) {
+    const bool ok = o < u.ni;
+    sfac[o] = ok ? u.par[u.i0 + o] : 0.0;
+    sq[o] = ok ? u.ipar[u.i0 + o] : -1;
+  }
+  for (int o = tid; o < NK * NK; o += kUpdThreads) {
+    const int j = o % NK, i = o / NK;
+    sK[o] = (i < u.ni && j < u.ni) ? u.par[u.nk + (size_t)u.nk * (u.i0 + i) + u.i0 + j] : 0.0;
+  }
+  __syncthreads();
+  double acc[NK];
+#pragma unroll
+  for (int i = 0; i < NK; ++i) acc[i] = 0.0;
+  if (act) {
+    for (int r = 0; r < u.nrange; ++r)
+#pragma unroll
+      for (int i = 0; i < NK; ++i)
+        if (i < u.ni) acc[i] += __ldg(u.part + ((size_t)r * u.ni + i) * u.nrs + t);
+    const RsDev rt = u.rs[t];
+    const DPair& C = u.pairs[rt.sp];
+    const DPair& A = u.pairs[u.spab];
+    const double* b = u.blk + u.base[rt.sp] * u.ksz;
+#pragma unroll
+    for (int i = 0; i < NK; ++i)
+      if (i < u.ni) acc[i] = cho_blk(b, rt, C, u.rs[sq[i]], A) - acc[i];
+  }
+  double dabs = 0.0;
+  if (t < u.nrs) {
+    double d = act ? u.diag[t] : 0.0;
+    const int Mp = u.M + u.i0;
+#pragma unroll
+    for (int i = 0; i < NK; ++i) {
+      if (i >= u.ni) break;
+      double x = 0.0;
+      if (act) {
+        x = acc[i] * sfac[i];
+        if (d == 0.0) x = 0.0;
+        d -= x * x;
+        if (t == sq[i]) d = 0.0;  // Cho_P_ZeroDiag
+        if (d < 0.0 && d < u.thrneg) {  // Cho_ChkDia_A4
+          if (d < u.tooneg) atomicOr(u.flags, 1);
+          d = 0.0;
+        }
+        if (sqrt(fabs(d) * u.qdmax) * u.damp <= u.thrcom) d = 0.0;
+#pragma unroll
+        for (int j = 0; j < NK; ++j)
+          if (j > i) acc[j] -= sK[j + NK * i] * x;
+      }
+      const int c = Mp + i;
+      u.Lt[c / kVecBlock][t + u.nrs * (c % kVecBlock)] = x;
+    }
+    if (act) {
+      u.diag[t] = d;
+      dabs = fabs(d);
+    }
+  }
+  if (u.last) {  // the largest |diagonal| left (a maximum: independent of the order)
+    for (int o = 16; o > 0; o >>= 1) dabs = fmax(dabs, __shfl_xor_sync(0xffffffffu, dabs, o));
+    if ((tid & 31) == 0) smax[tid >> 5] = dabs;
+    __syncthreads();
+    if (tid == 0) {
+      for (int w = 1; w < kUpdThreads / 32; ++w) dabs = fmax(dabs, smax[w]);
+      if (dabs > 0.0) atomicMax(u.xm, (unsigned long long)__double_as_longlong(dabs));
+    }
+  }
+}
+
+// ranges of the previous vectors: about 6 CTAs per SM in all, at least 64
+// vectors each
+static int upd_ranges(int64_t nrs, int M, int nsm) {
+  const int64_t rows = (nrs + kUpdRows - 1) / kUpdRows;
+  const int64_t r = std::min<int64_t>(6 * (int64_t)nsm / rows, M / 64);
+  return (int)std::max<int64_t>(1, r);
+}
+
+template <int NK>
+static void launch_update_nk(const ChoUpd& u, cudaStream_t st) {
+  if (u.nrange)
+    k_cho_subtr<NK><<<dim3((unsigned)((u.nrs + kUpdRows - 1) / kUpdRows), u.nrange), kUpdThreads, 0, st>>>(u);
+  k_cho_compvec<NK><<<(unsigned)((u.nrs + kUpdThreads - 1) / kUpdThreads), kUpdThreads, 0, st>>>(u);
+  g_launches.fetch_add(u.nrange ? 2 : 1, std::memory_order_relaxed);
+}
+static void launch_update(ChoUpd u, int nsm, cudaStream_t st) {
+  const int Mp = u.M + u.i0;
+  const int want = Mp ? upd_ranges(u.nrs, Mp, nsm) : 0;
+  u.jper = want ? ((Mp + want - 1) / want + kUpdJ - 1) / kUpdJ * kUpdJ : kUpdJ;
+  u.nrange = (Mp + u.jper - 1) / u.jper;
+  if (u.ni <= 2) launch_update_nk<2>(u, st);
+  else if (u.ni <= 4) launch_update_nk<4>(u, st);
+  else if (u.ni <= 6) launch_update_nk<6>(u, st);
+  else if (u.ni <= 8) launch_update_nk<8>(u, st);
+  else if (u.ni <= 12) launch_update_nk<12>(u, st);
+  else if (u.ni <= 16) launch_update_nk<16>(u, st);
+  else if (u.ni <= 24) launch_update_nk<24>(u, st);
+  else launch_update_nk<32>(u, st);
 }
 
 __global__ void k_init_red(double* __restrict__ diag, unsigned char* __restrict__ inred, int64_t n, double scrmax) {
@@ -184,16 +425,6 @@ __global__ void k_init_red(double* __restrict__ diag, unsigned char* __restrict_
   }
 }
 
-// gather LQ rows: lq[i + nq*J] = L[qrow[i] + nrs*J]
-__global__ void k_gather_rows(const double* __restrict__ L, int64_t nrs, int ncol, const int* __restrict__ rows, int nq,
-                              double* __restrict__ lq) {
-  int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (o >= (int64_t)nq * ncol) return;
-  const int i = (int)(o % nq);
-  const int64_t J = o / nq;
-  lq[o] = L[rows[i] + nrs * J];
-}
-
 static inline unsigned nblk(int64_t n, int b = 256) { return (unsigned)((n + b - 1) / b); }
 
 // --------------------------------------------------------------- host side
@@ -202,6 +433,8 @@ struct ChoState {
   std::vector<int> rs_a, rs_b, rs_sp;
   std::vector<int64_t> sp_first;
   std::vector<int> sp_count;
+  std::vector<RsDev> rsd;       // host copy of d_rs while the state is built
+  char* d_tab = nullptr;        // one allocation holding the tables below
   RsDev* d_rs = nullptr;
   int* d_rs_a = nullptr;        // AO indices of each rs entry (device)
   int* d_rs_b = nullptr;
@@ -214,20 +447,24 @@ struct ChoState {
   int M = 0;
   std::vector<int> piv, pass_of;
   int npass = 0;
-  cublasHandle_t cublas = nullptr;
   short* d_lexp = nullptr;      // row exponents of the square L_J (mixed J/K), M x lexp_ld
   int lexp_ld = 0;
   int* d_inv = nullptr;         // rs index of every AO pair (n x n, -1: no row), J/K
 };
 
-static const int kVecBlock = 1024;
+// The vectors' storage of a state about to be replaced, for the next
+// decomposition of the same list (which frees what it does not use).
+void cho_recycle(Handle* h, ChoState* c) {
+  if (!c) return;
+  h->cho_spare.swap(c->Lblk);
+  h->cho_spare_bytes = sizeof(double) * (size_t)c->nrs * kVecBlock;
+  cho_free(c);
+}
 
 void cho_free(ChoState* c) {
   if (!c) return;
-  cudaFree(c->d_rs); cudaFree(c->d_sp_first); cudaFree(c->d_sp_count); cudaFree(c->d_rs_a); cudaFree(c->d_rs_b);
-  cudaFree(c->d_diag); cudaFree(c->d_diag0); cudaFree(c->d_inred); cudaFree(c->d_lexp); cudaFree(c->d_inv);
+  cudaFree(c->d_tab); cudaFree(c->d_lexp); cudaFree(c->d_inv);
   for (auto p : c->Lblk) cudaFree(p);
-  if (c->cublas) cublasDestroy(c->cublas);
   delete c;
 }
 
@@ -235,10 +472,8 @@ void cho_free(ChoState* c) {
 // every shell pair (keep == nullptr) or the shell pairs with keep[sp] set
 // (the others get sp_first = -1 and no rows).  Replaces a previous list.
 static void make_rs(Handle* h, ChoState* c, const std::vector<char>* keep = nullptr) {
-  cudaFree(c->d_rs_a); cudaFree(c->d_rs_b); cudaFree(c->d_rs); cudaFree(c->d_sp_first); cudaFree(c->d_sp_count);
-  c->rs_a.clear(); c->rs_b.clear(); c->rs_sp.clear(); c->sp_first.clear(); c->sp_count.clear();
+  c->rs_a.clear(); c->rs_b.clear(); c->rs_sp.clear(); c->sp_first.clear(); c->sp_count.clear(); c->rsd.clear();
   const int ns = h->sh.size();
-  std::vector<RsDev> rsd;
   for (int i = 0; i < ns; ++i)
     for (int j = 0; j <= i; ++j) {
       const int sp = pair_id(i, j);
@@ -258,7 +493,7 @@ static void make_rs(Handle* h, ChoState* c, const std::vector<char>* keep = null
         r.sp = sp;
         r.ma = la / A.nc; r.ka = la % A.nc;
         r.mb = lb / B.nc; r.kb = lb % B.nc;
-        rsd.push_back(r);
+        c->rsd.push_back(r);
       };
       if (i != j) {
         for (int lb = 0; lb < nB; ++lb)
@@ -270,21 +505,37 @@ static void make_rs(Handle* h, ChoState* c, const std::vector<char>* keep = null
       c->sp_count.push_back((int)(c->rs_a.size() - c->sp_first.back()));
     }
   c->nrs = c->rs_a.size();
-  dev_malloc(&c->d_rs_a, sizeof(int) * c->nrs);
-  dev_malloc(&c->d_rs_b, sizeof(int) * c->nrs);
+}
+
+// The state's device tables, in one allocation; the rs list goes up.
+static bool upload_rs(ChoState* c) {
+  const size_t n = std::max<int64_t>(c->nrs, 1), nsp = c->sp_first.size();
+  size_t need = 0;
+  auto place = [&](size_t bytes) { const size_t o = need; need += (bytes + 255) & ~(size_t)255; return o; };
+  const size_t o_rs = place(sizeof(RsDev) * n), o_a = place(sizeof(int) * n), o_b = place(sizeof(int) * n),
+               o_f = place(sizeof(int64_t) * nsp), o_c = place(sizeof(int) * nsp), o_d = place(sizeof(double) * n),
+               o_d0 = place(sizeof(double) * n), o_in = place(n);
+  if (dev_malloc(&c->d_tab, need) != cudaSuccess) return false;
+  c->d_rs = (RsDev*)(c->d_tab + o_rs);
+  c->d_rs_a = (int*)(c->d_tab + o_a);
+  c->d_rs_b = (int*)(c->d_tab + o_b);
+  c->d_sp_first = (int64_t*)(c->d_tab + o_f);
+  c->d_sp_count = (int*)(c->d_tab + o_c);
+  c->d_diag = (double*)(c->d_tab + o_d);
+  c->d_diag0 = (double*)(c->d_tab + o_d0);
+  c->d_inred = (unsigned char*)(c->d_tab + o_in);
+  cudaMemcpy(c->d_rs, c->rsd.data(), sizeof(RsDev) * c->nrs, cudaMemcpyHostToDevice);
   cudaMemcpy(c->d_rs_a, c->rs_a.data(), sizeof(int) * c->nrs, cudaMemcpyHostToDevice);
   cudaMemcpy(c->d_rs_b, c->rs_b.data(), sizeof(int) * c->nrs, cudaMemcpyHostToDevice);
-  dev_malloc(&c->d_rs, sizeof(RsDev) * c->nrs);
-  cudaMemcpy(c->d_rs, rsd.data(), sizeof(RsDev) * c->nrs, cudaMemcpyHostToDevice);
-  dev_malloc(&c->d_sp_first, sizeof(int64_t) * c->sp_first.size());
-  cudaMemcpy(c->d_sp_first, c->sp_first.data(), sizeof(int64_t) * c->sp_first.size(), cudaMemcpyHostToDevice);
-  dev_malloc(&c->d_sp_count, sizeof(int) * c->sp_count.size());
-  cudaMemcpy(c->d_sp_count, c->sp_count.data(), sizeof(int) * c->sp_count.size(), cudaMemcpyHostToDevice);
+  cudaMemcpy(c->d_sp_first, c->sp_first.data(), sizeof(int64_t) * nsp, cudaMemcpyHostToDevice);
+  cudaMemcpy(c->d_sp_count, c->sp_count.data(), sizeof(int) * nsp, cudaMemcpyHostToDevice);
+  std::vector<RsDev>().swap(c->rsd);
+  return true;
 }
 
 // ERI blocks (q4 quartets) into a scratch buffer; offsets per quartet
-static double* eri_blocks(Handle* h, const std::vector<int32_t>& q4, std::vector<int64_t>& off, double*& buf,
-                          size_t& bufsz, cudaStream_t st, int& rc) {
+static double* eri_blocks(Handle* h, const std::vector<int32_t>& q4, std::vector<int64_t>& off, cudaStream_t st,
+                          int& rc) {
   const int64_t nq = q4.size() / 4;
   off.assign(nq + 1, 0);
   for (int64_t t = 0; t < nq; ++t) {
@@ -292,14 +543,8 @@ static double* eri_blocks(Handle* h, const std::vector<int32_t>& q4, std::vector
     for (int x = 0; x < 4; ++x) n *= (int64_t)h->sh[q4[4 * t + x]].nc * h->sh[q4[4 * t + x]].ncomp;
     off[t + 1] = off[t] + n;
   }
-  const size_t need = sizeof(double) * std::max<int64_t>(off[nq], 1);
-  if (need > bufsz) {
-    cudaStreamSynchronize(st);
-    cudaFree(buf);
-    buf = nullptr;
-    if (dev_malloc(&buf, need) != cudaSuccess) { rc = MG_ERR_MEMORY; bufsz = 0; return nullptr; }
-    bufsz = need;
-  }
+  double* buf = (double*)keep_get(h->cho_buf, sizeof(double) * std::max<int64_t>(off[nq], 1), st);
+  if (!buf) { rc = MG_ERR_MEMORY; return nullptr; }
   std::vector<EriItem> items;
   std::vector<EriClass> classes;
   rc = build_eri_items(h, q4.data(), nq, off.data(), items, classes);
@@ -356,17 +601,84 @@ static int cd_incore_1p(std::vector<double>& X, int n, std::vector<double>& Vec,
   return 0;
 }
 
-static double red_max(const double* d_diag, const unsigned char* d_inred, int64_t n, double* d_tmp, int which,
-                      cudaStream_t st) {
-  const int nb = 296;
-  k_red_max<<<nb, 256, 0, st>>>(d_diag, d_inred, n, d_tmp);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  std::vector<double> h(2 * nb);
-  cudaMemcpyAsync(h.data(), d_tmp, sizeof(double) * 2 * nb, cudaMemcpyDeviceToHost, st);
-  cudaStreamSynchronize(st);
-  double m = which == 0 ? 0.0 : -1e300;
-  for (int b = 0; b < nb; ++b) m = std::max(m, h[2 * b + which]);
-  return m;
+// Static side of the per-pass integral batches: the kept shell pairs grouped by
+// la + lb, heaviest (most primitive pairs) first, their block sizes and the
+// distinct kinds of pair in each group, from which a pass's class statistics
+// follow.  The ket of a pass is one shell pair, so nothing is sorted per pass.
+struct ChoKind {
+  int nij, ne, nsab, maxnp;
+};
+struct ChoItemPlan {
+  std::vector<int> order[2 * MG_MAX_L + 1];       // shell pairs of la + lb = nab
+  std::vector<ChoKind> kinds[2 * MG_MAX_L + 1];
+  std::vector<int> kind_of;                        // per shell pair, in its group
+  std::vector<int64_t> base;                       // first element of the bra block
+  int64_t total = 0;                               // elements of all bra blocks
+};
+
+static void make_item_plan(const Handle* h, const ChoState* c, ChoItemPlan& p) {
+  const int nsp = c->sp_count.size();
+  p.kind_of.assign(nsp, 0);
+  p.base.assign(nsp, 0);
+  for (int sp = 0; sp < nsp; ++sp) {
+    if (!c->sp_count[sp]) continue;
+    const DPair& P = h->pairs[sp];
+    const int nij = P.nci * P.ncj, nsab = P.nsa * P.nsb, nab = P.la + P.lb;
+    p.base[sp] = p.total;
+    p.total += (int64_t)nij * nsab;
+    p.order[nab].push_back(sp);
+    auto& ks = p.kinds[nab];
+    size_t k = 0;
+    while (k < ks.size() && !(ks[k].nij == nij && ks[k].ne == P.ne && ks[k].nsab == nsab)) ++k;
+    if (k == ks.size()) ks.push_back({nij, P.ne, nsab, 0});
+    ks[k].maxnp = std::max(ks[k].maxnp, P.np);
+    p.kind_of[sp] = (int)k;
+  }
+  for (auto& o : p.order)
+    std::stable_sort(o.begin(), o.end(), [&](int a, int b) { return h->pairs[a].np > h->pairs[b].np; });
+}
+
+// The (CD|AB) work items of one pass (bra pairs with alive[sp] != 0, ket spab)
+static int pass_items(Handle* h, const ChoItemPlan& p, const unsigned char* alive, int spab,
+                      std::vector<EriItem>& items, std::vector<EriClass>& classes) {
+  const DPair& Q = h->pairs[spab];
+  const int nkl = Q.nci * Q.ncj, ncd = Q.la + Q.lb;
+  const int64_t ksz = (int64_t)nkl * Q.nsa * Q.nsb;
+  items.clear();
+  classes.clear();
+  std::vector<char> seen;
+  std::vector<int> chunk;
+  for (int nab = 0; nab <= 2 * MG_MAX_L; ++nab) {
+    if (p.order[nab].empty()) continue;
+    const auto& ks = p.kinds[nab];
+    seen.assign(ks.size(), 0);
+    chunk.resize(ks.size());
+    for (size_t k = 0; k < ks.size(); ++k) chunk[k] = eri_ket_chunk(ks[k].nij, ks[k].ne * Q.ne);
+    EriClass c;
+    c.nab = nab;
+    c.ncd = ncd;
+    c.begin = (int)items.size();
+    c.work = 0;
+    for (int sp : p.order[nab]) {
+      if (!alive[sp]) continue;
+      const int kd = p.kind_of[sp];
+      if (chunk[kd] < 1) { h->err = "mg_cho_drv: bra contraction block too large"; return MG_ERR_ARG; }
+      seen[kd] = 1;
+      c.work += h->pairs[sp].np;
+      for (int c0 = 0; c0 < nkl; c0 += chunk[kd])
+        items.push_back({sp, spab, c0, std::min(nkl, c0 + chunk[kd]), (long long)(p.base[sp] * ksz)});
+    }
+    c.count = (int)items.size() - c.begin;
+    if (!c.count) continue;
+    ClassStats cs;
+    for (size_t k = 0; k < ks.size(); ++k)
+      if (seen[k]) eri_class_stats(cs, ks[k].nij, std::min(nkl, chunk[k]), ks[k].ne, Q.ne, ks[k].nsab, ks[k].maxnp, Q.np);
+    c.work *= (double)Q.np * cs.max_nef;
+    c.plan = eri_plan_for(h, nab, ncd, cs, c.count);
+    if (c.plan.PAB < 1) { h->err = "mg_cho_drv: class does not fit in shared memory"; return MG_ERR_ARG; }
+    classes.push_back(c);
+  }
+  return 0;
 }
 
 int cho_decompose(Handle* h, const ChoCfgH& cfg, ChoState*& out, cudaStream_t st, std::string& err) {
@@ -375,12 +687,19 @@ int cho_decompose(Handle* h, const ChoCfgH& cfg, ChoState*& out, cudaStream_t st
   make_rs(h, c);
   const int nsp = c->sp_count.size();
   const double damp = cho_default_damp(cfg.thrcom);
-  if (cublasCreate(&c->cublas) != CUBLAS_STATUS_SUCCESS) { err = "cublasCreate failed"; return MG_ERR_CUDA; }
-  cublasSetStream(c->cublas, st);
-  double* d_tmp = nullptr;
-  dev_malloc(&d_tmp, sizeof(double) * std::max<int64_t>(2 * 296, 2 * (int64_t)nsp));
-  double* buf = nullptr;
-  size_t bufsz = 0;
+  // the handle's buffers, kept for the next decomposition unless they are large
+  struct GiveBack {
+    Handle* h;
+    ~GiveBack() {
+      for (Workspace* w : {&h->cho_scr, &h->cho_buf, &h->cho_lq, &h->cho_upd})
+        if (w->size > kKeepBytes) {
+          cudaFree(w->ptr);
+          *w = Workspace{};
+        }
+      for (double* p : h->cho_spare) cudaFree(p);
+      h->cho_spare.clear();
+    }
+  } give_back{h};
   int rc = 0;
   // ---- diagonal (CHO_GETDIAG): (AB|AB) for every shell pair, then the initial
   // screening (cho_calcdiag.F90:255-300): elements below
@@ -395,20 +714,22 @@ int cho_decompose(Handle* h, const ChoCfgH& cfg, ChoState*& out, cudaStream_t st
       q4.insert(q4.end(), {i, j, i, j});
     }
     std::vector<int64_t> off;
-    eri_blocks(h, q4, off, buf, bufsz, st, rc);
-    if (rc) { err = "diagonal integrals failed: " + err; cudaFree(buf); cudaFree(d_tmp); return rc; }
-    int64_t* d_off = nullptr;
-    dev_malloc(&d_off, sizeof(int64_t) * nsp);
-    cudaMemcpyAsync(d_off, off.data(), sizeof(int64_t) * nsp, cudaMemcpyHostToDevice, st);
+    double* buf = eri_blocks(h, q4, off, st, rc);
+    if (rc) { err = "diagonal integrals failed: " + err; return rc; }
     // full diagonal, every shell pair
-    double* d_full = nullptr;
-    dev_malloc(&d_full, sizeof(double) * c->nrs);
-    k_extract_diag<<<nblk(c->nrs), 256, 0, st>>>(c->d_rs, c->nrs, h->d_pairs, d_off, buf, d_full);
+    const size_t rs_bytes = (sizeof(RsDev) * c->nrs + 255) & ~(size_t)255;
+    char* d = (char*)keep_get(h->cho_scr, rs_bytes + sizeof(int64_t) * nsp + sizeof(double) * c->nrs, st);
+    if (!d) { err = "diagonal: out of device memory"; return MG_ERR_MEMORY; }
+    RsDev* d_rs = (RsDev*)d;
+    int64_t* d_off = (int64_t*)(d + rs_bytes);
+    double* d_full = (double*)(d_off + nsp);
+    cudaMemcpyAsync(d_rs, c->rsd.data(), sizeof(RsDev) * c->nrs, cudaMemcpyHostToDevice, st);
+    cudaMemcpyAsync(d_off, off.data(), sizeof(int64_t) * nsp, cudaMemcpyHostToDevice, st);
+    k_extract_diag<<<nblk(c->nrs), 256, 0, st>>>(d_rs, c->nrs, h->d_pairs, d_off, buf, d_full);
     g_launches.fetch_add(1, std::memory_order_relaxed);
     std::vector<double> hd(c->nrs);
     cudaMemcpyAsync(hd.data(), d_full, sizeof(double) * c->nrs, cudaMemcpyDeviceToHost, st);
     cudaStreamSynchronize(st);
-    cudaFree(d_full);
     double dm = 0;
     for (double v : hd) dm = std::max(dm, std::fabs(v));
     if (dm > 0) scrmax = cfg.thrcom * cfg.thrcom / damp / dm;
@@ -417,170 +738,179 @@ int cho_decompose(Handle* h, const ChoCfgH& cfg, ChoState*& out, cudaStream_t st
       if (!(hd[t] < scrmax)) keep[c->rs_sp[t]] = 1;
     make_rs(h, c, &keep);
     // the diagonal over the kept shell pairs, from the same integral blocks
-    dev_malloc(&c->d_diag, sizeof(double) * std::max<int64_t>(c->nrs, 1));
-    dev_malloc(&c->d_diag0, sizeof(double) * std::max<int64_t>(c->nrs, 1));
-    dev_malloc(&c->d_inred, std::max<int64_t>(c->nrs, 1));
+    if (!upload_rs(c)) { err = "diagonal: out of device memory"; return MG_ERR_MEMORY; }
     k_extract_diag<<<nblk(std::max<int64_t>(c->nrs, 1)), 256, 0, st>>>(c->d_rs, c->nrs, h->d_pairs, d_off, buf,
                                                                         c->d_diag0);
     g_launches.fetch_add(1, std::memory_order_relaxed);
     cudaMemcpyAsync(c->d_diag, c->d_diag0, sizeof(double) * c->nrs, cudaMemcpyDeviceToDevice, st);
     cudaStreamSynchronize(st);
-    cudaFree(d_off);
   }
   const int64_t nrs = c->nrs;
+  const size_t blk_bytes = sizeof(double) * (size_t)nrs * kVecBlock;
+  if (h->cho_spare_bytes != blk_bytes) {  // storage of the previous vectors, usable for the same list only
+    for (double* p : h->cho_spare) cudaFree(p);
+    h->cho_spare.clear();
+  }
+  ChoItemPlan plan;
+  make_item_plan(h, c, plan);
+  int maxcnt = 1;
+  for (int sp = 0; sp < nsp; ++sp) maxcnt = std::max(maxcnt, c->sp_count[sp]);
+  const int MQ = std::min(cfg.maxqual, maxcnt);  // the qualified columns belong to one shell pair
+  const int maxblk = cfg.maxvec / kVecBlock + 2;
+  // CTAs of k_cho_lq (each holds a partial qualified block), at most 64 MB of them
+  const int kParts = (int)std::max<int64_t>(1, std::min<int64_t>(148, ((int64_t)8 << 20) / ((int64_t)MQ * MQ)));
+  if (!smem_attr_once((const void*)k_cho_lq, 200 * 1024)) { err = "shared-memory limit could not be raised"; return MG_ERR_CUDA; }
+  // ---- scratch of the passes, one allocation
+  size_t need = 0;
+  auto place = [&](size_t bytes) { const size_t o = need; need += (bytes + 255) & ~(size_t)255; return o; };
+  const size_t sel_bytes = sizeof(ChoSel) + sizeof(double) * maxcnt + (size_t)(maxcnt + 7) / 8 * 8 + nsp;
+  const size_t par_bytes = sizeof(double) * ((size_t)MQ + (size_t)MQ * MQ) + sizeof(int) * 2 * MQ;
+  const size_t o_sel = place(sel_bytes), o_diash = place(sizeof(double) * 2 * nsp), o_par = place(par_bytes),
+               o_base = place(sizeof(int64_t) * nsp), o_lt = place(sizeof(double*) * maxblk), o_xm = place(16),
+               o_cols = place(sizeof(int) * MQ), o_q = place(sizeof(double) * MQ * MQ),
+               o_part = place(sizeof(double) * MQ * MQ * kParts);
+  char* scr = (char*)keep_get(h->cho_scr, need, st);
+  // partial sums of the update kernels
+  const int nrow = (int)((nrs + kUpdRows - 1) / kUpdRows);
+  const size_t upd = sizeof(double) * std::max<size_t>(1, 6 * h->nsm / std::max(nrow, 1)) * std::min(32, MQ) * std::max<int64_t>(nrs, 1);
+  double* d_upd = (double*)keep_get(h->cho_upd, upd, st);
+  if (!scr || !d_upd) { err = "out of device memory for the passes' scratch"; return MG_ERR_MEMORY; }
+  ChoSel* d_sel = (ChoSel*)(scr + o_sel);
+  double* d_dpair = (double*)(d_sel + 1);
+  unsigned char* d_rpair = (unsigned char*)(d_dpair + maxcnt);
+  unsigned char* d_alive = d_rpair + (size_t)(maxcnt + 7) / 8 * 8;
+  double* d_diash = (double*)(scr + o_diash);
+  double* d_par = (double*)(scr + o_par);
+  int64_t* d_base = (int64_t*)(scr + o_base);
+  double** d_lt = (double**)(scr + o_lt);
+  unsigned long long* d_xm = (unsigned long long*)(scr + o_xm);
+  int* d_flags = (int*)(d_xm + 1);
+  int* d_cols = (int*)(scr + o_cols);
+  double* d_Q = (double*)(scr + o_q);
+  double* d_part = (double*)(scr + o_part);
+  // host side of the same, pinned: the select buffer, Q, the parameters
+  const size_t pin_sel = (sel_bytes + 255) & ~(size_t)255, pin_q = sizeof(double) * MQ * MQ;
+  char* pin = (char*)pin_get(h, pin_sel + ((pin_q + 255) & ~(size_t)255) + par_bytes);
+  if (!pin) { err = "pinned host memory for the passes"; return MG_ERR_MEMORY; }
+  const ChoSel* hsel = (const ChoSel*)pin;
+  const double* hdpair = (const double*)(hsel + 1);
+  const unsigned char* hrpair = (const unsigned char*)(hdpair + maxcnt);
+  const unsigned char* halive = hrpair + (size_t)(maxcnt + 7) / 8 * 8;
+  double* hQ = (double*)(pin + pin_sel);
+  double* hpar = (double*)(pin + pin_sel + ((pin_q + 255) & ~(size_t)255));
   k_init_red<<<nblk(std::max<int64_t>(nrs, 1)), 256, 0, st>>>(c->d_diag, c->d_inred, nrs, scrmax);
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  int* d_flags = nullptr;
-  dev_malloc(&d_flags, sizeof(int));
-  cudaMemsetAsync(d_flags, 0, sizeof(int), st);
-  double *d_xint = nullptr, *d_X = nullptr, *d_K = nullptr, *d_fac = nullptr, *d_lq = nullptr, *d_Q = nullptr;
-  int *d_cols = nullptr, *d_qrs = nullptr;
-  int64_t* d_off = nullptr;
-  dev_malloc(&d_off, sizeof(int64_t) * nsp);
-  const int MQ = cfg.maxqual;
-  dev_malloc(&d_xint, sizeof(double) * nrs * MQ);
-  dev_malloc(&d_X, sizeof(double) * nrs * MQ);
-  dev_malloc(&d_K, sizeof(double) * MQ * MQ);
-  dev_malloc(&d_fac, sizeof(double) * MQ);
-  dev_malloc(&d_cols, sizeof(int) * MQ);
-  dev_malloc(&d_qrs, sizeof(int) * MQ);
-  dev_malloc(&d_Q, sizeof(double) * MQ * MQ);
-  dev_malloc(&d_lq, sizeof(double) * (size_t)MQ * kVecBlock);
-  std::vector<double> hdiash(2 * (size_t)nsp), hq;
-  std::vector<int64_t> off_sp(nsp);
-  auto Lcol = [&](int J) -> double* { return c->Lblk[J / kVecBlock] + (size_t)nrs * (J % kVecBlock); };
+  cudaMemsetAsync(d_xm, 0, 16, st);
+  cudaMemcpyAsync(d_base, plan.base.data(), sizeof(int64_t) * nsp, cudaMemcpyHostToDevice, st);
+  std::vector<EriItem> items;
+  std::vector<EriClass> classes;
+  std::vector<double> Q, Vec;
+  std::vector<int> iD;
   for (int pass = 0; pass <= nrs; ++pass) {
-    // ---- Cho_SetPass: the largest reduced-set diagonal of every shell pair
-    // (-1: no member in the reduced set); their maximum is the pass's DGMax
-    k_sp_max<<<nblk(nsp), 256, 0, st>>>(c->d_diag, c->d_inred, c->d_sp_first, c->d_sp_count, nsp, d_tmp);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    cudaMemcpyAsync(hdiash.data(), d_tmp, sizeof(double) * 2 * nsp, cudaMemcpyDeviceToHost, st);
-    cudaStreamSynchronize(st);
-    double dgmax = 0.0;  // max |diagonal| over the reduced set
-    for (int sp = 0; sp < nsp; ++sp) dgmax = std::max(dgmax, hdiash[nsp + sp]);
+    // ---- Cho_SetRed of the previous pass, Cho_SetPass and Cho_GetMaxShl; the
+    // diagonal and the reduced-set flags of the chosen shell pair come along
+    k_cho_scan<<<(nsp + 7) / 8, 256, 0, st>>>(c->d_diag, c->d_inred, c->d_sp_first, c->d_sp_count, nsp, d_xm, pass > 0,
+                                              damp, cfg.thrcom, d_diash, d_alive);
+    k_cho_select<<<1, 1024, 0, st>>>(d_diash, nsp, cfg.thrcom, c->d_sp_first, c->d_sp_count, c->d_diag, c->d_inred,
+                                     d_flags, d_xm, d_sel, d_dpair, d_rpair);
+    g_launches.fetch_add(2, std::memory_order_relaxed);
+    cudaMemcpyAsync(pin, d_sel, sel_bytes, cudaMemcpyDeviceToHost, st);
+    if (cudaStreamSynchronize(st) != cudaSuccess) { rc = MG_ERR_CUDA; err = "CUDA error in Cholesky pass"; break; }
+    if (hsel->flags) { rc = MG_ERR_DECOMP; err = "diagonal too negative (Cho_ChkDia_A4 TooNeg)"; break; }
+    const double dgmax = hsel->dgmax;  // max |diagonal| over the reduced set
     if (dgmax < cfg.thrcom) break;
     const double diamin = std::max(dgmax * cfg.span, cfg.thrcom);
-    double smax = -1e9;
-    int spab = -1;
-    for (int sp = 0; sp < nsp; ++sp) {
-      const double v = hdiash[sp] > cfg.thrcom ? hdiash[sp] : 0.0;
-      if (v > smax) { smax = v; spab = sp; }
-    }
+    const double smax = hsel->smax;
+    const int spab = hsel->spab;
     if (smax == 0.0 || std::fabs(smax) < diamin) { rc = MG_ERR_DECOMP; err = "no qualifying diagonal (Cho_GetInt 104)"; break; }
-    // ---- Cho_Qualify_2 within shell pair spab (cho_qualify.h)
-    const int64_t f = c->sp_first[spab];
-    const int cnt = c->sp_count[spab];
-    std::vector<double> dpair(cnt);
-    std::vector<unsigned char> rpair(cnt);
-    cudaMemcpyAsync(dpair.data(), c->d_diag + f, sizeof(double) * cnt, cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(rpair.data(), c->d_inred + f, cnt, cudaMemcpyDeviceToHost, st);
-    cudaStreamSynchronize(st);
-    // positions t inside the pair, then rs indices
-    std::vector<int> qual = cho_qualify_2(dpair.data(), rpair.data(), cnt, diamin, cfg.maxqual);
-    for (int& t : qual) t = (int)(f + t);
+    // ---- Cho_Qualify_2 within shell pair spab (cho_qualify.h): positions t
+    // inside the pair, then rs indices
+    std::vector<int> qual = cho_qualify_2(hdpair, hrpair, c->sp_count[spab], diamin, cfg.maxqual);
+    for (int& t : qual) t = (int)(c->sp_first[spab] + t);
     const int nq = qual.size();
     if (nq == 0) { rc = MG_ERR_DECOMP; err = "empty qualification (Cho_GetInt 104)"; break; }
     // ---- integral columns (CD|AB) for every CD pair touching the reduced set
-    // (the reduced set has not changed since the shell-pair maxima above)
-    std::vector<int32_t> q4;
-    std::vector<int> qsp;
-    for (int sp = 0; sp < nsp; ++sp) {
-      if (hdiash[sp] < 0.0) continue;
-      q4.insert(q4.end(), {h->pairs[sp].i, h->pairs[sp].j, h->pairs[spab].i, h->pairs[spab].j});
-      qsp.push_back(sp);
-    }
-    std::vector<int64_t> off;
-    eri_blocks(h, q4, off, buf, bufsz, st, rc);
+    const DPair& A = h->pairs[spab];
+    const int64_t ksz = (int64_t)A.nci * A.ncj * A.nsa * A.nsb;
+    double* buf = (double*)keep_get(h->cho_buf, sizeof(double) * std::max<int64_t>(plan.total * ksz, 1), st);
+    if (!buf) { rc = MG_ERR_MEMORY; err = "column integrals failed: out of device memory"; break; }
+    rc = pass_items(h, plan, halive, spab, items, classes);
+    if (!rc) rc = run_eri_items(h, items, classes, buf, st);
     if (rc) { err = "column integrals failed: " + err; break; }
-    std::fill(off_sp.begin(), off_sp.end(), -1);
-    for (size_t t = 0; t < qsp.size(); ++t) off_sp[qsp[t]] = off[t];
-    cudaMemcpyAsync(d_off, off_sp.data(), sizeof(int64_t) * nsp, cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(d_cols, qual.data(), sizeof(int) * nq, cudaMemcpyHostToDevice, st);
-    k_gather_columns<<<nblk(nrs), 256, 0, st>>>(c->d_rs, nrs, c->d_inred, h->d_pairs, d_off, buf, d_cols, nq, spab,
-                                                d_xint);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    // ---- Cho_Dec_Qual: Q = MQ - LQ LQ^T  (MQ = xint rows at the qualified positions)
+    // ---- Cho_Dec_Qual: Q = MQ - LQ LQ^T  (MQ: the columns' rows at the qualified positions)
     const int M = c->M;
-    // MQ (rows of the qualified columns) then Q -= LQ LQ^T on the device
-    std::vector<double> Q((size_t)nq * nq);
-    k_gather_rows<<<nblk((int64_t)nq * nq), 256, 0, st>>>(d_xint, nrs, nq, d_cols, nq, d_Q);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    for (int b = 0; b * kVecBlock < M; ++b) {
-      const int nc = std::min(kVecBlock, M - b * kVecBlock);
-      k_gather_rows<<<nblk((int64_t)nq * nc), 256, 0, st>>>(c->Lblk[b], nrs, nc, d_cols, nq, d_lq);
-      g_launches.fetch_add(1, std::memory_order_relaxed);
-      const double one = 1.0, mone = -1.0;
-      cublasDgemm(c->cublas, CUBLAS_OP_N, CUBLAS_OP_T, nq, nq, nc, &mone, d_lq, nq, d_lq, nq, &one, d_Q, nq);
+    double* d_lq = (double*)h->cho_lq.ptr;
+    if (h->cho_lq.size < sizeof(double) * (size_t)nq * (M + nq)) {  // grows with the vectors
+      d_lq = (double*)keep_get(h->cho_lq, sizeof(double) * (size_t)MQ * (M + kVecBlock + MQ), st);
+      if (!d_lq) { rc = MG_ERR_MEMORY; err = "out of device memory for the LQ rows"; break; }
     }
-    cudaMemcpyAsync(Q.data(), d_Q, sizeof(double) * nq * nq, cudaMemcpyDeviceToHost, st);
-    cudaStreamSynchronize(st);
-    std::vector<double> qdiag(nq);
-    for (int q = 0; q < nq; ++q) qdiag[q] = Q[q + (size_t)nq * q];
-    const double dmax = red_max(c->d_diag, c->d_inred, nrs, d_tmp, 1, st);  // Cho_P_MaxDX
-    const double thr = std::max(cfg.thrcom, dmax * cfg.span);
-    std::vector<double> Vec((size_t)nq * nq, 0.0);
-    std::vector<int> iD;
+    cudaMemcpyAsync(d_cols, qual.data(), sizeof(int) * nq, cudaMemcpyHostToDevice, st);
+    int nparts = 0;
+    if (M > 0) {
+      const int jb = std::max(1, std::min(64, 6144 / nq));
+      nparts = std::min((M + jb - 1) / jb, kParts);
+      k_cho_lq<<<nparts, 256, sizeof(double) * jb * nq, st>>>(d_lt, nrs, M, d_cols, nq, jb, d_lq, d_part);
+      g_launches.fetch_add(1, std::memory_order_relaxed);
+    }
+    k_cho_q<<<nblk((int64_t)nq * nq, 128), 128, 0, st>>>(c->d_rs, h->d_pairs, buf + plan.base[spab] * ksz, d_cols, nq,
+                                                         spab, d_part, nparts, d_Q);
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    cudaMemcpyAsync(hQ, d_Q, sizeof(double) * nq * nq, cudaMemcpyDeviceToHost, st);
+    if (cudaStreamSynchronize(st) != cudaSuccess) { rc = MG_ERR_CUDA; err = "CUDA error in Cholesky pass"; break; }
+    Q.assign(hQ, hQ + (size_t)nq * nq);
+    // Cho_P_MaxDX is the largest diagonal of the reduced set, all of them positive: dgmax
+    const double thr = std::max(cfg.thrcom, dgmax * cfg.span);
+    Vec.assign((size_t)nq * nq, 0.0);
+    iD.clear();
     int nk = 0;
     if (cd_incore_1p(Q, nq, Vec, nk, thr, iD)) { rc = MG_ERR_DECOMP; err = "CD_InCore_1p failed (negative diagonal)"; break; }
     if (nk == 0) { rc = MG_ERR_DECOMP; err = "no vector from qualified block"; break; }
     if (M + nk > cfg.maxvec) { rc = MG_ERR_MEMORY; err = "too many Cholesky vectors (MaxVec)"; break; }
     // pivot order (cho_decom_a4.F90:120-170)
-    std::vector<double> K((size_t)nk * nk), fac(nk), qd(nk);
-    std::vector<int> qrs(nk), colsel(nk);
+    double *fac = hpar, *K = hpar + nk;
+    int *qrs = (int*)(K + (size_t)nk * nk), *colsel = qrs + nk;
+    std::vector<double> qd(nk);
     for (int i = 0; i < nk; ++i)
       for (int j = 0; j < nk; ++j) K[j + (size_t)nk * i] = Vec[iD[j] + (size_t)nq * i];
-    for (int i = 0; i < nk; ++i) { qd[i] = qdiag[iD[i]]; qrs[i] = qual[iD[i]]; colsel[i] = iD[i]; }
+    for (int i = 0; i < nk; ++i) { qd[i] = hQ[iD[i] + (size_t)nq * iD[i]]; qrs[i] = qual[iD[i]]; colsel[i] = iD[i]; }
     const double qdmax = qd[0];
     for (int i = 0; i < nk; ++i) {
       fac[i] = 1.0 / std::sqrt(std::fabs(qd[i]));
       for (int j = i; j < nk; ++j) qd[j] -= K[j + (size_t)nk * i] * K[j + (size_t)nk * i];
       qd[i] = 0.0;
     }
-    // destination columns of this pass
+    // storage of this pass's vectors (every element of a column is written)
     while ((int)c->Lblk.size() * kVecBlock < M + nk) {
       double* p = nullptr;
-      if (dev_malloc(&p, sizeof(double) * nrs * kVecBlock) != cudaSuccess) { rc = MG_ERR_MEMORY; break; }
-      cudaMemsetAsync(p, 0, sizeof(double) * nrs * kVecBlock, st);
+      if (!h->cho_spare.empty()) {
+        p = h->cho_spare.back();
+        h->cho_spare.pop_back();
+      } else if (dev_malloc(&p, blk_bytes) != cudaSuccess) {
+        rc = MG_ERR_MEMORY;
+        break;
+      }
+      cudaMemcpyAsync(d_lt + c->Lblk.size(), &p, sizeof(double*), cudaMemcpyHostToDevice, st);
       c->Lblk.push_back(p);
     }
     if (rc) { err = "out of device memory for Cholesky vectors"; break; }
-    // X[:, i] = xint[:, iD[i]] (pivot order, Cho_RdQCol_Indx) in a contiguous scratch
-    for (int i = 0; i < nk; ++i)
-      cudaMemcpyAsync(d_X + nrs * i, d_xint + nrs * colsel[i], sizeof(double) * nrs, cudaMemcpyDeviceToDevice, st);
-    cudaMemcpyAsync(d_qrs, qrs.data(), sizeof(int) * nk, cudaMemcpyHostToDevice, st);
-    // ---- Cho_Subtr: X -= L_prev LQ^T  (DGEMM per vector block)
-    for (int b = 0; b * kVecBlock < M; ++b) {
-      const int ncb = std::min(kVecBlock, M - b * kVecBlock);
-      k_gather_rows<<<nblk((int64_t)nk * ncb), 256, 0, st>>>(c->Lblk[b], nrs, ncb, d_qrs, nk, d_lq);
-      g_launches.fetch_add(1, std::memory_order_relaxed);
-      const double mone = -1.0, one = 1.0;
-      cublasDgemm(c->cublas, CUBLAS_OP_N, CUBLAS_OP_T, (int)nrs, nk, ncb, &mone, c->Lblk[b], (int)nrs, d_lq, nk, &one,
-                  d_X, (int)nrs);
+    cudaMemcpyAsync(d_par, hpar, sizeof(double) * ((size_t)nk + (size_t)nk * nk) + sizeof(int) * 2 * nk,
+                    cudaMemcpyHostToDevice, st);
+    if (nk > 32)  // later launches read the LQ rows of this pass's own vectors
+      cudaMemcpyAsync(d_lq + (size_t)M * nq, Vec.data(), sizeof(double) * (size_t)nq * nk, cudaMemcpyHostToDevice, st);
+    // ---- Cho_Subtr and Cho_CompVec
+    ChoUpd u{d_lt, nrs, M, 0, 0, nk, nq, spab, 0, 0, 0, d_upd, d_lq, buf, d_base, ksz, c->d_rs, h->d_pairs, c->d_inred, c->d_diag,
+             d_par, (const int*)(d_par + nk + (size_t)nk * nk), qdmax, damp, cfg.thrcom, -1e-40, -1e-8, d_flags, d_xm};
+    for (u.i0 = 0; u.i0 < nk; u.i0 += 32) {
+      u.ni = std::min(32, nk - u.i0);
+      u.last = u.i0 + 32 >= nk;
+      launch_update(u, h->nsm, st);
     }
-    // ---- Cho_CompVec (row-parallel)
-    cudaMemcpyAsync(d_K, K.data(), sizeof(double) * nk * nk, cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(d_fac, fac.data(), sizeof(double) * nk, cudaMemcpyHostToDevice, st);
-    k_compvec<<<nblk(nrs), 256, 0, st>>>(d_X, nrs, nk, d_K, d_fac, d_qrs, c->d_diag, c->d_inred, qdmax, damp,
-                                        cfg.thrcom, -1e-40, -1e-8, d_flags);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    for (int i = 0; i < nk; ++i)
-      cudaMemcpyAsync(Lcol(M + i), d_X + nrs * i, sizeof(double) * nrs, cudaMemcpyDeviceToDevice, st);
     for (int i = 0; i < nk; ++i) { c->piv.push_back(qrs[i]); c->pass_of.push_back(pass); }
     c->M = M + nk;
     c->npass = pass + 1;
-    // ---- Cho_SetRed (damped screening)
-    const double xm = red_max(c->d_diag, c->d_inred, nrs, d_tmp, 0, st);
-    k_setred<<<nblk(nrs), 256, 0, st>>>(c->d_diag, c->d_inred, nrs, xm, damp, cfg.thrcom, xm > cfg.thrcom ? 0 : 1);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    int hflag = 0;
-    cudaMemcpyAsync(&hflag, d_flags, sizeof(int), cudaMemcpyDeviceToHost, st);
-    cudaStreamSynchronize(st);
-    if (hflag) { rc = MG_ERR_DECOMP; err = "diagonal too negative (Cho_ChkDia_A4 TooNeg)"; break; }
     if (cudaGetLastError() != cudaSuccess) { rc = MG_ERR_CUDA; err = "CUDA error in Cholesky pass"; break; }
   }
   cudaStreamSynchronize(st);
-  cudaFree(buf); cudaFree(d_tmp); cudaFree(d_flags); cudaFree(d_xint); cudaFree(d_X); cudaFree(d_K); cudaFree(d_fac);
-  cudaFree(d_lq); cudaFree(d_Q); cudaFree(d_cols); cudaFree(d_qrs); cudaFree(d_off);
   return rc;
 }
 
@@ -610,7 +940,6 @@ int cho_copy_vectors(const ChoState* c, int first, int count, double* d_out, cud
   return 0;
 }
 const double* cho_diag0(const ChoState* c) { return c->d_diag0; }
-cublasHandle_t cho_cublas(ChoState* c) { return c->cublas; }
 const int* cho_rs_a_dev(const ChoState* c) { return c->d_rs_a; }
 const int* cho_rs_b_dev(const ChoState* c) { return c->d_rs_b; }
 // contiguous FP64 vectors [J0, J0+nb) (the range must not cross a storage block)
@@ -619,7 +948,6 @@ const double* cho_vec_ptr(const ChoState* c, int J0, int nb, cudaStream_t, Handl
   return c->Lblk[J0 / kVecBlock] + (size_t)c->nrs * (J0 % kVecBlock);
 }
 int cho_vec_block() { return kVecBlock; }
-const int64_t* cho_sp_first_dev(const ChoState* c) { return c->d_sp_first; }
 short* cho_lexp(const ChoState* c, int ld) { return c->lexp_ld == ld ? c->d_lexp : nullptr; }
 void cho_set_lexp(ChoState* c, short* p, int ld) {
   cudaFree(c->d_lexp);

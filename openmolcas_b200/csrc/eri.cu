@@ -115,11 +115,13 @@ int eri_launch_class(Handle* h, const EriItem* d_items, int nitems, int nab, int
   for (int i = 0; i < MG_MAX_RYS; ++i) ra.m[i] = h->rys_meta[i];
   ra.tab = h->d_rys;
   const int groups = kEriThreads / pl.tpq;
-  int per_sm = 0, nsm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kEriThreads, pl.smem);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
-  if (per_sm < 1) return 3;
   const long long want = (nitems + groups - 1) / groups;
+  const int nsm = h->nsm;
+  int per_sm = 1;
+  if (want > nsm) {  // up to one CTA per SM: resident whatever the occupancy
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kEriThreads, pl.smem);
+    if (per_sm < 1) return 3;
+  }
   const int nblk = (int)std::min<long long>(want, (long long)per_sm * nsm);
   EriArgs a{d_items, nitems, h->d_pairs, h->d_prim, h->tot_np, h->d_coef, h->d_hrr, tab, out, d_counter,
             pl.tpq, pl.gsm, pl.PAB, pl.PCD};

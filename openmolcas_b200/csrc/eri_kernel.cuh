@@ -42,7 +42,6 @@ struct EriArgs {
 };
 using EriFn = void (*)(EriArgs, RysArgs);
 EriFn eri_kernel_pick(int nab, int ncd);
-constexpr int kEriThreads = 512;
 
 // [e0|f0] of one Cartesian shell L of the bra range for one primitive quartet
 // and one ket component f: the L + 1 values of each direction's row are loaded

@@ -249,7 +249,8 @@ int grad_build(Handle* h, double cutint, GradPlan& plan) {
   plan.d_counters = nullptr;
   // one scratch region per side stream: class kernels on different streams run concurrently
   plan.scratch_stride = (std::max<size_t>(scratch_need, 32) + 31) & ~(size_t)31;
-  if (dev_malloc(&plan.d_scratch, sizeof(double) * plan.scratch_stride * MG_ERI_STREAMS) != cudaSuccess ||
+  plan.nstreams = std::max<int>(1, std::min<int>(MG_ERI_STREAMS, (int)plan.classes.size()));
+  if (dev_malloc(&plan.d_scratch, sizeof(double) * plan.scratch_stride * plan.nstreams) != cudaSuccess ||
       dev_malloc(&plan.d_counters, sizeof(int) * std::max<size_t>(plan.classes.size(), 1)) != cudaSuccess) {
     h->err = "gradient scratch allocation failed";
     return MG_ERR_MEMORY;
@@ -272,7 +273,8 @@ int grad_run(Handle* h, const GradPlan& plan, const double* d_D, const double* d
   // The class kernels are independent (own counter, own scratch region per stream, atomic
   // accumulation into the gradient): spread them over the handle's side streams so that the
   // tail of one class overlaps the next.
-  int rc = side_streams_fork(h, st);
+  const int nside = (h->grad_profile || plan.classes.size() < 2) ? 0 : plan.nstreams;
+  int rc = nside ? side_streams_fork(h, st, nside) : 0;
   if (rc) return rc;
   // largest classes first; the scratch region follows the stream (classes on one
   // stream run one after another).  Profiled: every class on the caller's stream,
@@ -296,8 +298,8 @@ int grad_run(Handle* h, const GradPlan& plan, const double* d_D, const double* d
     const GradClass& c = plan.classes[ci];
     GradFn k = grad_kernel_m1(c.nab1, c.ncd1);
     if (!k) { h->err = "gradient class out of range"; return MG_ERR_ARG; }
-    const int sk = h->grad_profile ? 0 : (int)(pos % MG_ERI_STREAMS);
-    const cudaStream_t ks = h->grad_profile ? st : h->eri_streams[sk];
+    const int sk = nside ? (int)(pos % nside) : 0;
+    const cudaStream_t ks = nside ? h->eri_streams[sk] : st;
     GradArgs a{plan.d_items + c.begin, c.count, h->d_pairs, h->d_prim, h->tot_np, h->d_coef, d_D, h->nbf,
                plan.d_tab, d_grad, plan.d_scratch + plan.scratch_stride * sk, c.scr, plan.d_counters + ci, c.tpq,
                c.gsm, c.pab, c.pcd, c.rw, d_DS, coulfac, 0.25 * exfac};
@@ -310,7 +312,7 @@ int grad_run(Handle* h, const GradPlan& plan, const double* d_D, const double* d
     if (cudaGetLastError() != cudaSuccess) { h->err = "gradient kernel launch failed"; return MG_ERR_CUDA; }
     if (h->grad_profile) cudaEventRecord(h->grad_ev[2 * pos + 1], ks);
   }
-  side_streams_join(h, st);
+  side_streams_join(h, st, nside);
   return 0;
 }
 

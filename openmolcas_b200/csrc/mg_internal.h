@@ -62,6 +62,8 @@ struct EriItem {
   long long out_off;
 };
 
+constexpr int kEriThreads = 512;  // threads of an ERI CTA
+
 // Launch plan of one ERI class (eri.cu) and per-class statistics.
 struct ClassPlan {
   int tpq, PAB, PCD, gsm;
@@ -91,6 +93,7 @@ struct Workspace {
 
 struct Handle {
   int device = 0;
+  int nsm = 148;  // SMs of the device
   std::vector<ShellH> sh;
   int nbf = 0, natom = 0, lmax = 0;
   // pairs (canonical, iTri order: pair id of (i,j), i>=j, is i*(i+1)/2+j)
@@ -109,10 +112,15 @@ struct Handle {
   std::vector<double> tmax;   // Schwarz bound per pair (sqrt max |(ab|ab)|)
   double* d_tmax = nullptr;
   Workspace ws;
+  Workspace pin;              // pinned host memory (pin_get)
+  // buffers of the Cholesky decomposition (keep_get) and the storage of the
+  // vectors it replaces
+  Workspace cho_scr, cho_buf, cho_lq, cho_upd;
+  std::vector<double*> cho_spare;
+  size_t cho_spare_bytes = 0;
   std::string err;
   struct ChoState* cho = nullptr;  // Cholesky vectors of the current basis
   struct GradPlan* grad = nullptr; // gradient work list (per Schwarz threshold)
-  int* d_eri_counters = nullptr;   // one work counter per ERI class launch (64)
   cudaStream_t eri_streams[MG_ERI_STREAMS] = {};  // side streams of the ERI and gradient class launches
   cudaEvent_t eri_events[MG_ERI_STREAMS] = {};
   cudaEvent_t eri_fork = nullptr;
@@ -160,15 +168,16 @@ struct GradPlan {
   std::vector<GradClass> classes;
   GradItem* d_items = nullptr;
   size_t scratch_stride = 0;     // doubles of scratch per side stream
+  int nstreams = 1;              // side streams the classes are spread over
   double* d_tab = nullptr;       // per-CTA tables of the gradient kernel
   double* d_scratch = nullptr;   // per-group 2-PDM slots
   int* d_counters = nullptr;     // one work counter per class
   double cutint = -1;
 };
 int grad_build(Handle* h, double cutint, GradPlan& plan);
-// fork the handle's side streams from `st` (created on first use) / join them back into `st`
-int side_streams_fork(Handle* h, cudaStream_t st);
-void side_streams_join(Handle* h, cudaStream_t st);
+// fork the first n of the handle's side streams from `st` (created on first use) / join them back into `st`
+int side_streams_fork(Handle* h, cudaStream_t st, int n);
+void side_streams_join(Handle* h, cudaStream_t st, int n);
 int rys_eval(Handle* h, int nrys, int64_t n, const double* d_T, double* d_x, double* d_w);
 int grad_run(Handle* h, const GradPlan& plan, const double* d_D, const double* d_DS, double coulfac, double exfac,
              double* d_grad, cudaStream_t st);
@@ -182,6 +191,7 @@ struct ChoCfgH {
 };
 int cho_decompose(Handle* h, const ChoCfgH& cfg, ChoState*& out, cudaStream_t st, std::string& err);
 void cho_free(ChoState* c);
+void cho_recycle(Handle* h, ChoState* c);
 int64_t cho_nrs(const ChoState* c);
 int cho_nvec(const ChoState* c);
 int cho_npass(const ChoState* c);
@@ -189,8 +199,6 @@ void cho_pivots(const ChoState* c, int32_t* piv, int32_t* pass_of);
 void cho_rs_list(const ChoState* c, int32_t* a, int32_t* b, int32_t* sp);
 int cho_copy_vectors(const ChoState* c, int first, int count, double* d_out, cudaStream_t st);
 const double* cho_diag0(const ChoState* c);
-typedef struct cublasContext* cublasHandle_t;
-cublasHandle_t cho_cublas(ChoState* c);
 const int* cho_rs_a_dev(const ChoState* c);
 const int* cho_rs_b_dev(const ChoState* c);
 const double* cho_vec_ptr(const ChoState* c, int J0, int nb, cudaStream_t st, Handle* h);
@@ -198,8 +206,6 @@ int cho_vec_block();
 // rs index of every AO pair (n x n device table, -1 where no row is stored),
 // built on first use and owned by the state; nullptr when it cannot be stored
 const int* cho_inv_dev(ChoState* c, int n, cudaStream_t st);
-// first rs index of every shell pair (pair_id order), device
-const int64_t* cho_sp_first_dev(const ChoState* c);
 // cached row exponents of the square Cholesky vectors (M x ld), owned by the state
 short* cho_lexp(const ChoState* c, int ld);
 void cho_set_lexp(ChoState* c, short* p, int ld);
@@ -228,11 +234,22 @@ void build_sph(Handle* h, int lmax);
 std::vector<double> hrr_matrix(const Handle* h, int la, int lb, const double* A, const double* B, int& ne, int& emin);
 int setup_pairs(Handle* h);
 void* ws_get(Handle* h, size_t bytes, cudaStream_t st);
+// device memory of one of the handle's workspaces, grown when too small (after
+// waiting for the stream); nullptr when it cannot be had
+void* keep_get(Workspace& w, size_t bytes, cudaStream_t st);
+// pinned host memory of the handle, kept between calls; the caller has waited
+// for every copy of the previous use.  nullptr when it cannot be had.
+void* pin_get(Handle* h, size_t bytes);
 
 // ERI work lists (capi.cu) and launchers (eri.cu)
 ClassPlan eri_plan(int nab, int ncd, const ClassStats& cs, int tpq0 = 0, int order = 0);
 int eri_launch_class(Handle* h, const EriItem* d_items, int nitems, int nab, int ncd, const ClassPlan& pl, double* out,
                      int* d_counter, cudaStream_t st);
+// contracted ket pairs of one work item (0: even one does not fit)
+int eri_ket_chunk(int nij, int nef);
+void eri_class_stats(ClassStats& cs, int nij, int nklc, int ne, int nf, int nsab, int npab, int npcd);
+// the launch plan of `count` work items of class (nab, ncd) of this handle
+ClassPlan eri_plan_for(const Handle* h, int nab, int ncd, const ClassStats& cs, int count);
 int build_eri_items(Handle* h, const int32_t* q4, int64_t nq, const int64_t* offsets, std::vector<EriItem>& items,
                     std::vector<EriClass>& classes);
 int run_eri_items(Handle* h, const std::vector<EriItem>& items, const std::vector<EriClass>& classes, double* d_out,

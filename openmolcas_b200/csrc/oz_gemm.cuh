@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(kOzThreads, 1)
     // so that the descriptors are formed in uniform registers.  With one box per
     // operand and K step instead of one per slice: half-transform 32.2 -> 29.0 ms,
     // exchange product 19.0 -> 17.7 ms at 1250 functions (L2 reads: 5.8 TB/s of the
-    // 10 TB/s a plain read kernel gets; the MMAs alone would take 17 and 9 ms)
+    // 10 TB/s a plain read kernel gets; the MMAs alone would take 17 and 7 ms)
     const uint32_t el = tc_elect();
     const uint32_t id[4] = {tc_idesc_i8(a.Nt, false, false), tc_idesc_i8(a.Nt, false, true),
                             tc_idesc_i8(a.Nt, true, false), tc_idesc_i8(a.Nt, true, true)};
