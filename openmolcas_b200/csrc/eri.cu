@@ -67,15 +67,17 @@ static size_t eri_group_smem(int nab, int ncd, const ClassStats& cs, int pab, in
 
 // tpq0: the first group size tried (0: from the widest stage); order: the tile
 // dimension shrunk first when it does not fit (0 ket primitives, 1 bra; + 2:
-// the tile starts from 64 x 16 primitive pairs instead of 32 x 8)
+// the tile starts from 64 x 16 primitive pairs instead of 32 x 8; 4: from 64 x
+// 64 and shrinks towards four times as many bra as ket primitives: the bra sum of
+// a tile is formed in registers)
 ClassPlan eri_plan(int nab, int ncd, const ClassStats& cs, int tpq0, int order) {
   const int NR = (nab + ncd) / 2 + 1;
   ClassPlan pl{0, 0, 0, 0, 0};
   const size_t budget = (227 * 1024) / 8 - kETabD;  // one CTA per SM
-  const bool big = order >= 2;
-  order %= 2;
+  const bool square = order == 4, big = order >= 2;
+  order = square ? 0 : order % 2;
   int pab = std::max(1, std::min(cs.max_npab, big ? 64 : 32));
-  int pcd = std::max(1, std::min(cs.max_npcd, big ? 16 : 8));
+  int pcd = std::max(1, std::min(cs.max_npcd, square ? 64 : big ? 16 : 8));
   const int width = std::max({cs.max_acc, pab * pcd * cs.max_nef / 2, pab * pcd * NR * 3 * 8});
   // the kernel's multiply-high divisions are exact below 2^32: largest loop
   // extent x divisor of a tile a x c
@@ -89,10 +91,14 @@ ClassPlan eri_plan(int nab, int ncd, const ClassStats& cs, int tpq0, int order) 
     const size_t gbudget = (budget / groups) & ~(size_t)1;
     int a = pab, c = pcd;
     while ((eri_group_smem(nab, ncd, cs, a, c) > gbudget || bound(a, c) >= 4294967296.0) && (a > 1 || c > 1)) {
-      if (order == 1 && a > 1) a = (a + 1) / 2;
-      else if (c > 1) c = (c + 1) / 2;
-      else a = (a + 1) / 2;
+      if ((square && a >= 4 * c && a > 1) || (order == 1 && a > 1)) a = tile_shrink(a, cs.max_npab);
+      else if (c > 1) c = tile_shrink(c, cs.max_npcd);
+      else a = tile_shrink(a, cs.max_npab);
     }
+    // a group whose accumulators leave no room for a tile of a few quartets gives
+    // way to the next larger one (class (2, 6), f f ket pairs: 34.2 ms with 1 x 1 tiles
+    // in 256-thread groups, 6.1 ms in one group of 512)
+    if (tpq < kEriThreads && a * c < std::min(4, cs.max_npab * cs.max_npcd)) continue;
     if (eri_group_smem(nab, ncd, cs, a, c) <= gbudget) {
       pl.tpq = tpq;
       pl.PAB = a;

@@ -170,9 +170,14 @@ int grad_build(Handle* h, double cutint, GradPlan& plan) {
     {
       const size_t cta = kCtaLimit / 8 - kGTabD;
       const int nthr = GradThreads<1>::value;
-      const int order = h->grad_order[key];
-      const int cab = h->grad_cap[key] ? 32 : 16, ccd = h->grad_cap[key] ? 16 : 8;
-      const int tpq0 = h->grad_tpq[key] ? h->grad_tpq[key] : (wmax <= 512 ? 128 : 256);
+      // A class with no more items than SMs is a matter of one item's latency: the
+      // whole CTA takes one item, in the largest tile that fits (from 64 x 64 primitive
+      // pairs, the larger dimension shrinks).  Above that the table's throughput tiles
+      // are faster.  24 functions (406 quartets): 660 -> 292 us a gradient.
+      const bool small = (int)v.size() <= h->nsm && !h->grad_fixed[key];
+      const int order = small ? 3 : h->grad_order[key];
+      const int cab = small ? 64 : h->grad_cap[key] ? 32 : 16, ccd = small ? 64 : h->grad_cap[key] ? 16 : 8;
+      const int tpq0 = small ? nthr : h->grad_tpq[key] ? h->grad_tpq[key] : (wmax <= 512 ? 128 : 256);
       // a tile fits when its shared memory is within the group's share and every
       // run-time loop extent x divisor of the kernel stays below 2^32
       auto div_ok = [&](int a, int c, int rw) {
@@ -187,9 +192,10 @@ int grad_build(Handle* h, double cutint, GradPlan& plan) {
         size_t need = worst(pab, pcd, rw);
         while ((need > gb || !div_ok(pab, pcd, rw)) && (pab > 1 || pcd > 1 || rw > 1)) {
           if (order == 1 && rw > 1) --rw;
-          else if (order == 2 && pab > 1) pab = (pab + 1) / 2;
-          else if (pcd > 1) pcd = (pcd + 1) / 2;
-          else if (pab > 1) pab = (pab + 1) / 2;
+          else if (order == 2 && pab > 1) pab = tile_shrink(pab, m.npab);
+          else if (order == 3 && pab >= pcd && pab > 1) pab = tile_shrink(pab, m.npab);
+          else if (pcd > 1) pcd = tile_shrink(pcd, m.npcd);
+          else if (pab > 1) pab = tile_shrink(pab, m.npab);
           else --rw;
           need = worst(pab, pcd, rw);
         }

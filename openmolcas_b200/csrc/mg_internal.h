@@ -133,6 +133,9 @@ struct Handle {
   int grad_tpq[64] = {};
   int grad_order[64] = {};
   int grad_cap[64] = {};  // tile caps: 0 = 16 bra x 8 ket primitive pairs, 1 = 32 x 16
+  // classes whose tile the caller set and that keep it whatever their size (the
+  // choices that mg_tile_defaults was told about are throughput defaults)
+  bool grad_fixed[64] = {}, eri_fixed[64] = {};
   // profiled gradients: classes one after another on the caller's stream, an
   // event pair around each (grad_ev[2k], grad_ev[2k + 1] for class key grad_ev_key[k])
   bool grad_profile = false;
@@ -222,6 +225,12 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs, dou
                    cudaStream_t st, int block, int s, int sk);
 int jk_fp64_batch(Handle* h, int k, const double* const* Cs, const int* rs, double* const* Js, double* const* Ks,
                   cudaStream_t st);
+
+// the next smaller tile extent of n items: one tile more, of equal extents
+inline int tile_shrink(int x, int n) {
+  const int k = (n + x - 1) / x + 1;
+  return (n + k - 1) / k < x ? (n + k - 1) / k : x - 1;
+}
 
 inline int ncart(int l) { return (l + 1) * (l + 2) / 2; }
 inline int ncart_cum(int l) { return l <= 0 ? 0 : l * (l + 1) * (l + 2) / 6; }

@@ -76,6 +76,7 @@ def lib():
     L.mg_grad_plan_info.argtypes = [vp, i, i, i, i, i, C.c_int]
     L.mg_eri_set_tile.argtypes = [vp, C.c_int, C.c_int, C.c_int, C.c_int]
     L.mg_eri_profile.argtypes = [vp, C.c_int]
+    L.mg_tile_defaults.argtypes = [vp]
     L.mg_eri_class_times.argtypes = [vp, i, d, i, i, i, C.c_int]
     _lib = L
     return L
@@ -127,6 +128,7 @@ class MolGpu:
                 for key, t in json.load(f)["classes"].items():
                     nab, ncd = (int(x) for x in key.split(","))
                     self.set_eri_tile(nab, ncd, t["tpq"], t["order"])
+        self._check(self.L.mg_tile_defaults(self.h), "mg_tile_defaults")
 
     def _check(self, rc, what):
         if rc != 0:
