@@ -55,13 +55,15 @@ static size_t grad_group_smem(const DPair& P, const DPair& Q, int nijc, int nklc
   const size_t n1d = (size_t)(la + 1) * (lb + 1) * (lc + 1) * (ld + 1);
   const size_t nij = nijc, nc = nij * nklc;
   const bool multi = nc > 1;
-  const size_t fixed = 8 + ev2(nij * P.np) + ev2((size_t)nklc * Q.np) + (multi ? ev2(nij * pcd * ncart4) : 0) +
+  const size_t fixed = 8 + nij * ev2((size_t)P.np) + nklc * ev2((size_t)Q.np) + (multi ? ev2(nij * pcd * ncart4) : 0) +
                        ev2((ncart4 + 1) / 2);
   const size_t nt = (size_t)pab * pcd;
   const size_t w = std::min<size_t>(rw, NR);
   // padded strides of Gp and F (the kernel's Gs, J4 and St)
   const size_t gs = ncart4 | 1, j4 = 4 * n1d + 2, st = 3 * w * j4 + (w & 1 ? 0 : 2);
-  const size_t tile = ev2(nt * ((size_t)NR * 10 + 5)) + ev2(nt * gs) + nt * st;
+  // the 2D tables of the classes whose recursion goes through shared memory
+  const size_t nij2 = (size_t)(la + lb + 2) * (lc + ld + 2), g2 = nij2 <= kGradJobMax ? 0 : 3 * w * (nij2 | 1);
+  const size_t tile = ev2(nt * ((size_t)NR * 10 + 5)) + ev2(nt * gs) + nt * st + ev2(nt * g2);
   return ev2(fixed + std::max(tile, (size_t)16 * 9));
 }
 

@@ -1,7 +1,7 @@
 // Two-electron gradient kernel (FP64), one template instantiated per
 // (la+lb+1, lc+ld+1) class; MINB (resident CTAs per SM) sets the threads per
 // CTA and the register budget.  The algorithm and its reference anchors are
-// described in grad.cu; the instantiations live in grad_k1.cu.
+// described in grad.cu; the instantiations live in grad_k1.cu .. grad_k3.cu.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -40,7 +40,12 @@ struct GradArgs {
 };
 
 using GradFn = void (*)(GradArgs, RysArgs);
+// the kernel of class (nab1, ncd1): instantiated in grad_k1.cu (nab1 1..3),
+// grad_k2.cu (4, 5) and grad_k3.cu (6, 7), which compile side by side
 GradFn grad_kernel_m1(int nab1, int ncd1);
+GradFn grad_kernel_lo(int nab1, int ncd1);
+GradFn grad_kernel_mid(int nab1, int ncd1);
+GradFn grad_kernel_hi(int nab1, int ncd1);
 
 // Assg1 for one shell quartet class with la = LA, blocked over the Cartesian
 // components of centre A: a thread takes all NCA components that share one
@@ -94,6 +99,180 @@ __device__ __forceinline__ void assg1_a_block(const double* __restrict__ F, cons
         acc[7] = fma(gxz, Y23[ay].y, acc[7]);
         acc[8] = fma(gxy, Z23[az].y, acc[8]);
       }
+    }
+  }
+}
+
+// s += c[0..3] v; AL: c is 16-byte aligned (two loads instead of four)
+template <bool AL>
+__device__ __forceinline__ void axpy4(const double* __restrict__ c, double v, double (&s)[4]) {
+  double2 a, b;
+  if (AL) {
+    a = *reinterpret_cast<const double2*>(c);
+    b = *reinterpret_cast<const double2*>(c + 2);
+  } else {
+    a = make_double2(c[0], c[1]);
+    b = make_double2(c[2], c[3]);
+  }
+  s[0] = fma(a.x, v, s[0]);
+  s[1] = fma(a.y, v, s[1]);
+  s[2] = fma(b.x, v, s[2]);
+  s[3] = fma(b.y, v, s[3]);
+}
+
+// Largest NI * NJ whose recursion stage runs one thread per job with the whole
+// 2D table of the job (NI NJ doubles) and the transfer rows in registers.  Larger
+// classes (from (3, 4): the registers would spill, and their tiles have too few
+// jobs to hide one long thread) go through a table in shared memory.  460-function
+// gradient, all classes with unchanged tiles 1723 -> 1554 ms: (3, 3) 167 -> 139,
+// (2, 3) 78 -> 50, (2, 2) 28 -> 17; (3, 5) 103 -> 92, (4, 5) 120 -> 106, (5, 4) 110
+// -> 101.
+constexpr int kGradJobMax = 18;
+
+// The recursion stage with one thread per (quartet, root, direction) job.  The
+// lane-per-row form (one NI-lane segment per job, rows exchanged by shuffles)
+// spends NI lanes on values that one thread forms in as many instructions, and
+// only la + 1 of the lanes store; a thread per job needs about a fifth of the
+// instructions.  When a wave has fewer jobs than half the group's threads, up to
+// four threads share a job: each repeats the recursion and takes every nsub-th
+// (c, d) column.  A job record's stride is 2 mod 4 doubles, so the 16-byte
+// stores of consecutive threads fall in different banks.
+template <int NI, int NJ, int NR>
+__device__ __forceinline__ void grad_jobs_thread(const double* __restrict__ cf, int CFT, const double* __restrict__ hdr,
+                                                 double* __restrict__ F, int nt, int nrw, int r0, int la, int lb,
+                                                 int lc, int ld, int J4, int St, const FDiv& fnrw, int tid, int tpq) {
+  const int njobs = nt * nrw * 3;
+  const int nsub = 4 * njobs <= tpq ? 4 : 2 * njobs <= tpq ? 2 : 1;
+  for (int q = tid; q < njobs * nsub; q += tpq) {
+    const int sub = q >= njobs ? (q >= 2 * njobs ? (q >= 3 * njobs ? 3 : 2) : 1) : 0, job = q - sub * njobs;
+    const int tr = job / 3, d = job - 3 * tr, t = fq(tr, fnrw), rl = tr - t * nrw, r = r0 + rl;
+    const double* c = cf + t * CFT + r * 10;
+    const double B00 = c[0], B10 = c[1], B01 = c[2], C00 = c[3 + d], D00 = c[6 + d];
+    double G[NJ][NI];  // G[j][e]
+    G[0][0] = d == 2 ? c[9] : 1.0;
+    G[0][1] = C00 * G[0][0];
+#pragma unroll
+    for (int i = 1; i < NI - 1; ++i) G[0][i + 1] = fma(i * B10, G[0][i - 1], C00 * G[0][i]);
+#pragma unroll
+    for (int j = 0; j < NJ - 1; ++j)
+#pragma unroll
+      for (int e = 0; e < NI; ++e) {
+        double v = D00 * G[j][e];
+        if (j > 0) v = fma(j * B01, G[j > 0 ? j - 1 : 0][e], v);
+        if (e > 0) v = fma(e * B00, G[j][e > 0 ? e - 1 : 0], v);
+        G[j + 1][e] = v;
+      }
+    const double cdv = hdr[3 + d], abv = hdr[d];
+    const double* ex = cf + t * CFT + NR * 10;
+    const double e2a = ex[0], e2b = ex[1], e2c = ex[2];
+    double2* Fo = reinterpret_cast<double2*>(F + (size_t)t * St + (size_t)(job - 3 * nrw * t) * J4);
+    int col = sub;  // counts down to this thread's next (c, d) column
+#pragma unroll
+    for (int m = 0; m < NJ - 1; ++m) {  // ket level d = m: G[c][e] = V[e][c][m]
+      if (m > ld) break;
+      if (m > 0) {
+#pragma unroll
+        for (int cc = 0; cc + m < NJ; ++cc)
+#pragma unroll
+          for (int e = 0; e < NI; ++e) G[cc][e] = fma(cdv, G[cc][e], G[cc + 1][e]);
+      }
+#pragma unroll
+      for (int cc = 0; cc + m + 1 < NJ; ++cc) {
+        if (cc > lc) break;
+        if (col-- != 0) continue;
+        col = nsub - 1;
+        double u[NI], w[NI], up[NI];
+#pragma unroll
+        for (int e = 0; e < NI; ++e) {
+          u[e] = G[cc][e];
+          w[e] = e2c * G[cc + 1][e];
+          if (cc > 0) w[e] = fma((double)-cc, G[cc > 0 ? cc - 1 : 0][e], w[e]);
+          up[e] = 0.0;
+        }
+        double2* Fc = Fo + 2 * (la + 1) * (lb + 1) * (cc + (lc + 1) * m);
+#pragma unroll
+        for (int b = 0; b < NI - 1; ++b) {
+          if (b > lb) break;
+          double ud = 0.0;  // U(a-1, b)
+#pragma unroll
+          for (int e = 0; e + b < NI - 1; ++e) {
+            const double ue = u[e], un = fma(abv, ue, u[e + 1]);  // U(a, b+1)
+            if (e <= la) {
+              double2 v01, v23;
+              v01.x = ue;
+              v01.y = e2a * u[e + 1];
+              if (e > 0) v01.y = fma((double)-e, ud, v01.y);
+              v23.x = e2b * un;
+              if (b > 0) v23.x = fma((double)-b, up[e], v23.x);
+              v23.y = w[e];
+              Fc[2 * (e + (la + 1) * b)] = v01;
+              Fc[2 * (e + (la + 1) * b) + 1] = v23;
+            }
+            w[e] = fma(abv, w[e], w[e + 1]);
+            ud = ue;
+            up[e] = ue;
+            u[e] = un;
+          }
+        }
+      }
+    }
+  }
+}
+
+// One (c, d = M) ket column of a job from its 2D table G[j][e]: the ket transfer
+// in closed form, V[e][c][M] = sum_k binom(M, k) CD^(M-k) G[c+k][e], for columns
+// c-1, c, c+1, then the bra transfer and the derivative factors in registers.
+template <int NI, int NJ, int M>
+__device__ __forceinline__ void grad_column(const double* __restrict__ G, int cc, int la, int lb, double abv,
+                                            double cdv, const double* __restrict__ ex, double2* __restrict__ Fc) {
+  constexpr double bin[4][4] = {{1, 0, 0, 0}, {1, 1, 0, 0}, {1, 2, 1, 0}, {1, 3, 3, 1}};
+  const double e2a = ex[0], e2b = ex[1], e2c = ex[2];
+  double ck[M + 1], p = 1.0;
+#pragma unroll
+  for (int k = M; k >= 0; --k) {
+    ck[k] = bin[M][k] * p;
+    p *= cdv;
+  }
+  const double mc = (double)-cc;
+  const double* Gc = G + cc * NI;
+  double u[NI], w[NI], up[NI];
+#pragma unroll
+  for (int e = 0; e < NI; ++e) {
+    double v = 0.0, vp = 0.0, vm = 0.0;
+#pragma unroll
+    for (int k = 0; k <= M + 1; ++k) {  // rows c .. c + M + 1
+      const double x = Gc[k * NI + e];
+      if (k <= M) v = fma(ck[k <= M ? k : 0], x, v);
+      if (k > 0) vp = fma(ck[k > 0 ? k - 1 : 0], x, vp);
+      if (k < M) vm = fma(ck[k < M ? k + 1 : 0], x, vm);
+    }
+    if (cc > 0) vm = fma(ck[0], Gc[e - NI], vm);
+    u[e] = v;
+    w[e] = fma(mc, vm, e2c * vp);
+    up[e] = 0.0;
+  }
+#pragma unroll
+  for (int b = 0; b < NI - 1; ++b) {
+    if (b > lb) break;
+    double ud = 0.0;  // U(a-1, b)
+#pragma unroll
+    for (int e = 0; e + b < NI - 1; ++e) {
+      const double ue = u[e], un = fma(abv, ue, u[e + 1]);  // U(a, b+1)
+      if (e <= la) {
+        double2 v01, v23;
+        v01.x = ue;
+        v01.y = e2a * u[e + 1];
+        if (e > 0) v01.y = fma((double)-e, ud, v01.y);
+        v23.x = e2b * un;
+        if (b > 0) v23.x = fma((double)-b, up[e], v23.x);
+        v23.y = w[e];
+        Fc[2 * (e + (la + 1) * b)] = v01;
+        Fc[2 * (e + (la + 1) * b) + 1] = v23;
+      }
+      w[e] = fma(abv, w[e], w[e + 1]);
+      ud = ue;
+      up[e] = ue;
+      u[e] = un;
     }
   }
 }
@@ -155,9 +334,10 @@ __global__ void __launch_bounds__(GradThreads<MINB>::value, MINB) grad_kernel(co
   const int NT = PAB * PCD;
   const int CFT = NR * 10 + 5;  // per-quartet coefficient record (odd stride)
   double* hdr = sm;
-  double* Cab = hdr + 8;                              // nij * npab
-  double* Ccd = Cab + ev2(nij * npab);                // nklc * npcd
-  double* Y = Ccd + ev2(nklc * npcd);                 // [ij][pc][abcd] (multi only)
+  const int npabs = ev2(npab), npcds = ev2(npcd);     // even rows: pairs of coefficients load at once
+  double* Cab = hdr + 8;                              // nij * npabs
+  double* Ccd = Cab + nij * npabs;                    // nklc * npcds
+  double* Y = Ccd + nklc * npcds;                     // [ij][pc][abcd] (multi only)
   int* IX = reinterpret_cast<int*>(Y + (multi ? ev2(nij * PCD * ncart4) : 0));  // [abcd] packed 2D indices
   double* U0 = reinterpret_cast<double*>(IX) + ev2((ncart4 + 1) / 2);
   // padded strides: consecutive primitive quartets fall in different bank groups
@@ -167,24 +347,37 @@ __global__ void __launch_bounds__(GradThreads<MINB>::value, MINB) grad_kernel(co
   double* cf = U0;                                    // NT * CFT
   double* Gp = cf + ev2(NT * CFT);                    // [t][abcd] primitive 2-PDM, row stride Gs
   double* F = Gp + ev2(NT * Gs);                      // [t][rl][dir][e1][4], job stride J4, quartet stride St
+  constexpr int GS = (NI * NJ) | 1;                   // 2D table of one job (odd stride), large classes only
+  double* G2 = F + (size_t)NT * St;                   // [job][j][e]
   double* Gam = Gg;                                   // [il][abcd] (global scratch)
   double* Tmp = Gg + ev2(nc * ncart4);                // stage-0 temp (global scratch)
   if (tid < 3) {
     hdr[tid] = P.A[tid] - P.B[tid];
     hdr[3 + tid] = Q.A[tid] - Q.B[tid];
   }
-  for (int o = tid; o < nij * npab; o += tpq) Cab[o] = a.coef[P.coef_off + (size_t)it.i0 * npab + o];
-  for (int o = tid; o < nklc * npcd; o += tpq) Ccd[o] = a.coef[Q.coef_off + (size_t)it.c0 * npcd + o];
+  {
+    const FDiv fab = fdiv(npab), fcd = fdiv(npcd);
+    for (int o = tid; o < nij * npab; o += tpq) {
+      const int ij = fq(o, fab);
+      Cab[o + ij * (npabs - npab)] = a.coef[P.coef_off + (size_t)it.i0 * npab + o];
+    }
+    for (int o = tid; o < nklc * npcd; o += tpq) {
+      const int kl = fq(o, fcd);
+      Ccd[o + kl * (npcds - npcd)] = a.coef[Q.coef_off + (size_t)it.c0 * npcd + o];
+    }
+  }
   // ---- stage 0: contracted 2-PDM (PGet1), spherical, then -> Cartesian
   {
     const double* Dm = a.Dm;
     const size_t nbf = a.nbf;
     const int nsp4 = nsa * nsb * nsc * nsd;
+    const SDiv dnc = sdiv(nc), dnsa = sdiv(nsa), dnsb = sdiv(nsb), dnsc = sdiv(nsc), dnij = sdiv(nij),
+               dpi = sdiv(P.nci), dqi = sdiv(Q.nci);
     for (int o = tid; o < nc * nsp4; o += tpq) {
-      const int il = o % nc, r1 = o / nc;
-      const int sa = r1 % nsa, r2 = r1 / nsa, sb = r2 % nsb, r3 = r2 / nsb, sc = r3 % nsc, sd = r3 / nsc;
-      const int ij = it.i0 + il % nij, kl = it.c0 + il / nij;
-      const int ki = ij % P.nci, kj = ij / P.nci, kk = kl % Q.nci, kq = kl / Q.nci;
+      int il, sa, sb, sc, ijl, ki, kk;
+      const int r1 = sq(o, dnc, il), r2 = sq(r1, dnsa, sa), r3 = sq(r2, dnsb, sb), sd = sq(r3, dnsc, sc);
+      const int kl = it.c0 + sq(il, dnij, ijl), ij = it.i0 + ijl;
+      const int kj = sq(ij, dpi, ki), kq = sq(kl, dqi, kk);
       const int pa = P.ao_a + sa * P.nci + ki, pb = P.ao_b + sb * P.ncj + kj;
       const int pc = Q.ao_a + sc * Q.nci + kk, pd = Q.ao_b + sd * Q.ncj + kq;
       // D is symmetric: index it with the fastest-varying AO (pa, then pb) as the
@@ -204,8 +397,10 @@ __global__ void __launch_bounds__(GradThreads<MINB>::value, MINB) grad_kernel(co
     double* nxt = Gam;
     if (ld >= 2) {  // d: [il][sa][sb][sc][sd] -> [il][sa][sb][sc][cd]
       const int inner = nc * nsa * nsb * nsc;
+      const SDiv din = sdiv(inner);
       for (int o = tid; o < inner * ncd; o += tpq) {
-        const int in = o % inner, cd = o / inner;
+        int in;
+        const int cd = sq(o, din, in);
         double s = 0;
         for (int m = 0; m < nsd; ++m) s = fma(Sd[cd + ncd * m], cur[in + inner * m], s);
         nxt[o] = s;
@@ -215,8 +410,10 @@ __global__ void __launch_bounds__(GradThreads<MINB>::value, MINB) grad_kernel(co
     }
     if (lc >= 2) {  // c
       const int inner = nc * nsa * nsb;
+      const SDiv din = sdiv(inner), dcc = sdiv(ncc);
       for (int o = tid; o < inner * ncc * ncd; o += tpq) {
-        const int in = o % inner, r1 = o / inner, cc = r1 % ncc, cd = r1 / ncc;
+        int in, cc;
+        const int cd = sq(sq(o, din, in), dcc, cc);
         double s = 0;
         for (int m = 0; m < nsc; ++m) s = fma(Sc[cc + ncc * m], cur[in + inner * (m + nsc * cd)], s);
         nxt[o] = s;
@@ -227,8 +424,10 @@ __global__ void __launch_bounds__(GradThreads<MINB>::value, MINB) grad_kernel(co
     if (lb >= 2) {  // b
       const int inner = nc * nsa;
       const int outer = ncc * ncd;
+      const SDiv din = sdiv(inner), dcb = sdiv(ncb);
       for (int o = tid; o < inner * ncb * outer; o += tpq) {
-        const int in = o % inner, r1 = o / inner, cb = r1 % ncb, ou = r1 / ncb;
+        int in, cb;
+        const int ou = sq(sq(o, din, in), dcb, cb);
         double s = 0;
         for (int m = 0; m < nsb; ++m) s = fma(Sb[cb + ncb * m], cur[in + inner * (m + nsb * ou)], s);
         nxt[o] = s;
@@ -238,8 +437,10 @@ __global__ void __launch_bounds__(GradThreads<MINB>::value, MINB) grad_kernel(co
     }
     if (la >= 2) {  // a
       const int outer = ncb * ncc * ncd;
+      const SDiv dca = sdiv(nca);
       for (int o = tid; o < nc * nca * outer; o += tpq) {
-        const int il = o % nc, r1 = o / nc, ca = r1 % nca, ou = r1 / nca;
+        int il, ca;
+        const int ou = sq(sq(o, dnc, il), dca, ca);
         double s = 0;
         for (int m = 0; m < nsa; ++m) s = fma(Sa[ca + nca * m], cur[il + nc * (m + nsa * ou)], s);
         nxt[o] = s;
@@ -247,8 +448,10 @@ __global__ void __launch_bounds__(GradThreads<MINB>::value, MINB) grad_kernel(co
       gsync(g, tpq);
       double* t = cur; cur = nxt; nxt = t;
     }
+    const SDiv dn4 = sdiv(ncart4);
     for (int o = tid; o < nc * ncart4; o += tpq) {  // transpose to [il][abcd]
-      const int il = o / ncart4, abcd = o - il * ncart4;
+      int abcd;
+      const int il = sq(o, dn4, abcd);
       nxt[o] = cur[il + nc * abcd];
     }
     Gam = nxt;
@@ -289,20 +492,18 @@ __global__ void __launch_bounds__(GradThreads<MINB>::value, MINB) grad_kernel(co
         const int r1 = fq(o, f4), abcd = o - r1 * ncart4, ij = fq(r1, fpc), pc0 = 4 * (r1 - ij * npc4);
         const double* gm = Gam + (size_t)ij * ncart4 + abcd;
         const double* cc = Ccd + pcd0 + pc0;
-        double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-        for (int klc = 0; klc < nklc; ++klc) {
-          const double gv = gm[(size_t)nij * klc * ncart4];
-          const double* ck = cc + klc * npcd;
-          s0 = fma(ck[0], gv, s0);
-          if (pc0 + 1 < npc) s1 = fma(ck[1], gv, s1);
-          if (pc0 + 2 < npc) s2 = fma(ck[2], gv, s2);
-          if (pc0 + 3 < npc) s3 = fma(ck[3], gv, s3);
+        double s[4] = {0.0, 0.0, 0.0, 0.0};
+        // (coefficients past the chunk belong to sums that are not stored)
+        if (pcd0 & 1) {
+          for (int klc = 0; klc < nklc; ++klc) axpy4<false>(cc + klc * npcds, gm[(size_t)nij * klc * ncart4], s);
+        } else {
+          for (int klc = 0; klc < nklc; ++klc) axpy4<true>(cc + klc * npcds, gm[(size_t)nij * klc * ncart4], s);
         }
         double* y = Y + abcd + ncart4 * (pc0 + PCD * ij);
-        y[0] = s0;
-        if (pc0 + 1 < npc) y[ncart4] = s1;
-        if (pc0 + 2 < npc) y[2 * ncart4] = s2;
-        if (pc0 + 3 < npc) y[3 * ncart4] = s3;
+        y[0] = s[0];
+        if (pc0 + 1 < npc) y[ncart4] = s[1];
+        if (pc0 + 2 < npc) y[2 * ncart4] = s[2];
+        if (pc0 + 3 < npc) y[3 * ncart4] = s[3];
       }
     }
     for (int pab0 = 0; pab0 < npab; pab0 += PAB) {
@@ -318,12 +519,14 @@ __global__ void __launch_bounds__(GradThreads<MINB>::value, MINB) grad_kernel(co
         const double zeta = prim[ia], eta = prim[ic];
         const double px = prim[2 * tot_np + ia], py = prim[3 * tot_np + ia], pz = prim[4 * tot_np + ia];
         const double qx = prim[2 * tot_np + ic], qy = prim[3 * tot_np + ic], qz = prim[4 * tot_np + ic];
-        const double ze = zeta + eta, zei = 1.0 / ze, rho = zeta * eta * zei;
+        double zei, rzei;  // 1 / (zeta + eta) and its root
+        recip_root(zeta + eta, zei, rzei);
+        const double rho = zeta * eta * zei;
         const double dx = px - qx, dy = py - qy, dz = pz - qz;
         const double T = rho * (dx * dx + dy * dy + dz * dz);
         double x, w;
         rys_one<NR>(ra, T, r, x, w);
-        const double fact = prim[tot_np + ia] * prim[tot_np + ic] * sqrt(zei);
+        const double fact = prim[tot_np + ia] * prim[tot_np + ic] * rzei;
         const double U2 = x * zei;
         double* c = cf + t * CFT + r * 10;
         c[0] = 0.5 * U2;
@@ -353,54 +556,49 @@ __global__ void __launch_bounds__(GradThreads<MINB>::value, MINB) grad_kernel(co
         const FDiv f4 = fdiv(ncart4), fpa = fdiv(npa4);
         for (int o = tid; o < npa4 * npc * ncart4; o += tpq) {
           const int r1 = fq(o, f4), abcd = o - r1 * ncart4, pc = fq(r1, fpa), pa0 = 4 * (r1 - pc * npa4);
-          double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+          double s[4] = {0.0, 0.0, 0.0, 0.0};
+          const double* ca = Cab + pab0 + pa0;
           if (multi) {
             const double* y = Y + abcd + ncart4 * pc;
-            const double* ca = Cab + pab0 + pa0;
-            for (int ij = 0; ij < nij; ++ij) {
-              const double yv = y[(size_t)ncart4 * PCD * ij];
-              const double* ci = ca + ij * npab;
-              s0 = fma(ci[0], yv, s0);
-              if (pa0 + 1 < npa) s1 = fma(ci[1], yv, s1);
-              if (pa0 + 2 < npa) s2 = fma(ci[2], yv, s2);
-              if (pa0 + 3 < npa) s3 = fma(ci[3], yv, s3);
+            if (pab0 & 1) {
+              for (int ij = 0; ij < nij; ++ij) axpy4<false>(ca + ij * npabs, y[ncart4 * PCD * ij], s);
+            } else {
+              for (int ij = 0; ij < nij; ++ij) axpy4<true>(ca + ij * npabs, y[ncart4 * PCD * ij], s);
             }
           } else {
-            const double gv = Gam[abcd] * Ccd[pcd0 + pc];
-            const double* ca = Cab + pab0 + pa0;
-            s0 = ca[0] * gv;
-            if (pa0 + 1 < npa) s1 = ca[1] * gv;
-            if (pa0 + 2 < npa) s2 = ca[2] * gv;
-            if (pa0 + 3 < npa) s3 = ca[3] * gv;
+            axpy4<false>(ca, Gam[abcd] * Ccd[pcd0 + pc], s);
           }
           double* gp = Gp + (size_t)(pa0 + npa * pc) * Gs + abcd;
-          gp[0] = s0;
-          if (pa0 + 1 < npa) gp[Gs] = s1;
-          if (pa0 + 2 < npa) gp[2 * Gs] = s2;
-          if (pa0 + 3 < npa) gp[3 * Gs] = s3;
+          gp[0] = s[0];
+          if (pa0 + 1 < npa) gp[Gs] = s[1];
+          if (pa0 + 2 < npa) gp[2 * Gs] = s[2];
+          if (pa0 + 3 < npa) gp[3 * Gs] = s[3];
         }
       }
       gsync(g, tpq);
       for (int r0 = 0; r0 < NR; r0 += RW) {
         const int nrw = min(RW, NR - r0);
         const FDiv fnrw = fdiv(nrw);
-        // ---- (2) one NI-lane segment of a warp per (quartet, root, direction) job (32/NI jobs
-        //      per warp), all in registers:
-        //      2D recursion: lane e holds the row G[e][0..NJ-1] and takes G[e-1][j] from its
-        //        neighbour,  G[e][j+1] = D00 G[e][j] + j B01 G[e][j-1] + e B00 G[e-1][j];
-        //      ket 2D-level HRR (HRR2Db) in the lane:  V[e][c][0] = G[e][c],
+        // ---- (2) 2D integrals of every (quartet, root, direction) job:
+        //      2D recursion  G[e][j+1] = D00 G[e][j] + j B01 G[e][j-1] + e B00 G[e-1][j];
+        //      ket 2D-level HRR (HRR2Db):  V[e][c][0] = G[e][c],
         //        V[e][c][d+1] = V[e][c+1][d] + CD V[e][c][d];
-        //      bra 2D-level HRR (HRR2Da) across the lanes of the group (a shift along e):
+        //      bra 2D-level HRR (HRR2Da):
         //        U(a,0) = V[a][c][d],  U(a,b+1) = U(a+1,b) + AB U(a,b);
         //      derivative factors (Rys2Dg): F = U, dA = 2alpha U(a+1,b) - a U(a-1,b),
         //        dB = 2beta U(a,b+1) - b U(a,b-1), dC = the same transfer of
         //        W[a] = 2gamma V[a][c+1][d] - c V[a][c-1][d]
-        {
+        if constexpr (NI * NJ <= kGradJobMax) {
+          grad_jobs_thread<NI, NJ, NR>(cf, CFT, hdr, F, nt, nrw, r0, la, lb, lc, ld, J4, St, fnrw, tid, tpq);
+        } else {
+          // the recursion by one NI-lane segment of a warp per job (32/NI jobs per warp; lane e
+          // holds the row G[e][0..NJ-1] and takes G[e-1][j] from its neighbour) into the
+          // job's table, then one thread per job and (c, d) column
           constexpr int JPW = 32 / NI;  // jobs per warp
           const int njobs = nt * nrw * 3;
           const int lane = tid & 31;
           const int seg = lane / NI, e = lane - seg * NI;  // seg >= JPW: spare lanes
-          const int lup = (lane + 31) & 31, ldn = (lane + 1) & 31;
+          const int lup = (lane + 31) & 31;
           for (int jb = (tid >> 5) * JPW; jb < njobs; jb += (tpq >> 5) * JPW) {  // warp-uniform trip count
             const bool valid = seg < JPW && jb + seg < njobs;
             const int job = min(jb + seg, njobs - 1);
@@ -414,60 +612,37 @@ __global__ void __launch_bounds__(GradThreads<MINB>::value, MINB) grad_kernel(co
               gm1 = g0;
               g0 = gn;
             }
-            double L[NJ];
-            L[0] = g0;
+            double* Go = G2 + (size_t)job * GS + e;
+            double L = g0, Lm = 0.0;
+            if (valid) Go[0] = L;
 #pragma unroll
             for (int j = 0; j < NJ - 1; ++j) {
-              const double up = __shfl_sync(0xffffffffu, L[j], lup);  // G[e-1][j]
-              double v = D00 * L[j];
-              if (j > 0) v = fma(j * B01, L[j > 0 ? j - 1 : 0], v);
+              const double up = __shfl_sync(0xffffffffu, L, lup);  // G[e-1][j]
+              double v = D00 * L;
+              if (j > 0) v = fma(j * B01, Lm, v);
               if (e > 0) v = fma(e * B00, up, v);
-              L[j + 1] = v;
+              Lm = L;
+              L = v;
+              if (valid) Go[(j + 1) * NI] = v;
             }
-            const double cdv = hdr[3 + d], abv = hdr[d];
+          }
+          gsync(g, tpq);
+          const int ncol = (lc + 1) * (ld + 1);
+          const FDiv fjobs = fdiv(njobs), flc = fdiv(lc + 1);
+          for (int w = tid; w < njobs * ncol; w += tpq) {
+            const int col = fq(w, fjobs), job = w - col * njobs;
+            const int m = fq(col, flc), cc = col - m * (lc + 1);
+            const int d = job % 3, tr = job / 3, t = fq(tr, fnrw);
             const double* ex = cf + t * CFT + NR * 10;
-            const double e2a = ex[0], e2b = ex[1], e2c = ex[2];
-            double2* Fo = reinterpret_cast<double2*>(F + (size_t)t * St + (size_t)(job - 3 * nrw * t) * J4);
-            const bool wr = valid && e <= la;
-#pragma unroll
-            for (int m = 0; m < NJ; ++m) {  // ket level: L[c] = V[e][c][m]
-              if (m > ld) break;
-              if (m > 0) {
-#pragma unroll
-                for (int cc = 0; cc + m < NJ; ++cc) L[cc] = fma(cdv, L[cc], L[cc + 1]);
-              }
-#pragma unroll
-              for (int cc = 0; cc + m + 1 < NJ; ++cc) {
-                if (cc > lc) break;
-                double u = L[cc];
-                double w = e2c * L[cc + 1] - (cc > 0 ? cc * L[cc > 0 ? cc - 1 : 0] : 0.0);
-                double uprev = 0.0;
-                // U(e-1, 0) from the neighbour once; later levels by the transfer itself,
-                // U(e-1, b+1) = U(e, b) + AB U(e-1, b), so each level needs two shuffles
-                double ud = __shfl_sync(0xffffffffu, u, lup);
-                const int ebase = (la + 1) * (lb + 1) * (cc + (lc + 1) * m);
-#pragma unroll
-                for (int b = 0; b < NI - 1; ++b) {
-                  if (b > lb) break;
-                  const double un = __shfl_sync(0xffffffffu, u, ldn);  // U(e+1, b)
-                  const double wn = __shfl_sync(0xffffffffu, w, ldn);
-                  const double unext = fma(abv, u, un);                       // U(e, b+1)
-                  if (wr) {
-                    double2 v01, v23;
-                    v01.x = u;
-                    v01.y = e2a * un - (e > 0 ? e * ud : 0.0);
-                    v23.x = e2b * unext - (b > 0 ? b * uprev : 0.0);
-                    v23.y = w;
-                    const int e1 = e + (la + 1) * b + ebase;
-                    Fo[2 * e1] = v01;
-                    Fo[2 * e1 + 1] = v23;
-                  }
-                  ud = fma(abv, ud, u);  // U(e-1, b+1)
-                  uprev = u;
-                  u = unext;
-                  w = fma(abv, w, wn);
-                }
-              }
+            double2* Fc = reinterpret_cast<double2*>(F + (size_t)t * St + (size_t)(job - 3 * nrw * t) * J4) +
+                          2 * (la + 1) * (lb + 1) * col;
+            const double* Gj = G2 + (size_t)job * GS;
+            const double abv = hdr[d], cdv = hdr[3 + d];
+            switch (m) {
+              case 0: grad_column<NI, NJ, 0>(Gj, cc, la, lb, abv, cdv, ex, Fc); break;
+              case 1: grad_column<NI, NJ, 1>(Gj, cc, la, lb, abv, cdv, ex, Fc); break;
+              case 2: grad_column<NI, NJ, 2>(Gj, cc, la, lb, abv, cdv, ex, Fc); break;
+              case 3: grad_column<NI, NJ, 3>(Gj, cc, la, lb, abv, cdv, ex, Fc); break;
             }
           }
         }
@@ -557,18 +732,4 @@ GradFn grad_fn_b(int b) {
   }
   return nullptr;
 }
-template <int MINB>
-GradFn grad_pick(int a, int b) {
-  switch (a) {
-    case 1: return grad_fn_b<MINB, 1>(b);
-    case 2: return grad_fn_b<MINB, 2>(b);
-    case 3: return grad_fn_b<MINB, 3>(b);
-    case 4: return grad_fn_b<MINB, 4>(b);
-    case 5: return grad_fn_b<MINB, 5>(b);
-    case 6: return grad_fn_b<MINB, 6>(b);
-    case 7: return grad_fn_b<MINB, 7>(b);
-  }
-  return nullptr;
-}
-
 }  // namespace mg

@@ -11,8 +11,11 @@
 //              CTAs so that a small matrix still fills the chip; every split
 //              keeps its own partial tiles, summed in order by k_finish_k
 // All sums run in a fixed order: a call gives the same bits every time.
-// Measured, 300 functions, 1400 vectors, rank 41 (cuBLAS DGEMM/DSYRK over
-// blocks of 32 unpacked squares before): see the figures at each kernel.
+// Measured, 300 functions, 1400 vectors, rank 41 (cuBLAS over blocks of 32
+// unpacked squares before): half-transform 0.52 ms, 20 TFLOP/s (1.12 ms and 0.38
+// ms of unpacking); exchange product 0.25 ms, 21 TFLOP/s (1.26 ms); whole Fock
+// update 4.55 -> 1.78 ms.  1250 functions, 3789 vectors, rank 167: 146.8 -> 117.1
+// ms (25 TFLOP/s; the FP64 pipe peaks at 37).
 #include <cuda_runtime.h>
 
 #include <algorithm>

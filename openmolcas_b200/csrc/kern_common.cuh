@@ -58,6 +58,30 @@ __device__ __forceinline__ FDiv fdiv(unsigned n) {
 }
 __device__ __forceinline__ unsigned fq(unsigned o, const FDiv& f) { return __umulhi(o, f.m) + (o & f.k); }
 
+// The same with a correction step: exact for every o < 2^32, whatever n
+// (floor(2^32 / n) o / 2^32 is at most one below the quotient).
+struct SDiv {
+  unsigned m, n;
+};
+__device__ __forceinline__ SDiv sdiv(unsigned n) { return {n == 1 ? 0xFFFFFFFFu : 0xFFFFFFFFu / n + (0xFFFFFFFFu % n == n - 1), n}; }
+__device__ __forceinline__ int sq(int o, const SDiv& f, int& rem) {
+  unsigned q = __umulhi((unsigned)o, f.m), r = (unsigned)o - q * f.n;
+  if (r >= f.n) {
+    ++q;
+    r -= f.n;
+  }
+  rem = (int)r;
+  return (int)q;
+}
+
+// x^-1 and x^-1/2: one reciprocal root, its square with one Newton step (both
+// within a unit in the last place, as the division and the root they replace)
+__device__ __forceinline__ void recip_root(double x, double& xi, double& rxi) {
+  rxi = rsqrt(x);
+  const double y = rxi * rxi;
+  xi = fma(y, fma(-x, y, 1.0), y);
+}
+
 // one Rys root/weight of order N at T (table or asymptotic)
 template <int N>
 __device__ __forceinline__ void rys_one(const RysArgs& ra, double T, int r, double& x, double& w) {
