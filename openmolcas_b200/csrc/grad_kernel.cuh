@@ -47,57 +47,76 @@ GradFn grad_kernel_lo(int nab1, int ncd1);
 GradFn grad_kernel_mid(int nab1, int ncd1);
 GradFn grad_kernel_hi(int nab1, int ncd1);
 
-// Assg1 for one shell quartet class with la = LA, blocked over the Cartesian
-// components of centre A: a thread takes all NCA components that share one
-// (b, c, d) component and one primitive quartet, loads the LA + 1 interleaved
-// 2D records (I, dA, dB, dC) per direction once and reuses them across the NCA
-// components (component 0 is (LA, 0, 0), so the x records start LA before it).
-template <int LA>
-__device__ __forceinline__ void assg1_a_block(const double* __restrict__ F, const double* __restrict__ Gp,
-                                              const int* __restrict__ IX, int nt, int nrest, int St, int Gs, int J4,
-                                              int nrw, int tid, int tpq, double* acc) {
-  constexpr int NCA = (LA + 1) * (LA + 2) / 2;
-  constexpr CartExp<LA> ce{};
+// Assg1 for one shell quartet class whose fastest component indices run over
+// shells of LA and LB (LB = 0: one shell), sum-factorised over the directions.
+// With G the primitive density and X, Y, Z the 2D integrals of a component,
+//   U[x] = sum G Y Z,  V[y] = sum G X Z,  W[z] = sum G X Y
+// over the components that share the 2D index x (y, z), and a derivative
+// factor multiplies U, V or W once per 2D index instead of once per component:
+// five FP64 operations per component and root and nine per 2D index and
+// direction, against fourteen per component for the products one by one, and the
+// derivative factors (three of the four values of a record) are read once per 2D
+// index.  A thread takes all NCA x NCB components of one (quartet, rest) and
+// loops over the roots.  abcd0, the first component, is (LA, 0, 0) x (LB, 0, 0),
+// so its packed x index lies LA + (LA + 1) LB after the block's first.
+template <int LA, int LB>
+__device__ __forceinline__ void assg1_block(const double* __restrict__ F, const double* __restrict__ Gp,
+                                            const int* __restrict__ IX, int nt, int nrest, int St, int Gs, int J4,
+                                            int nrw, int tid, int tpq, double* acc) {
+  constexpr int NCA = (LA + 1) * (LA + 2) / 2, NCB = (LB + 1) * (LB + 2) / 2;
+  constexpr int N = (LA + 1) * (LB + 1);  // 2D indices per direction
+  constexpr CartExp<LA> ca{};
+  constexpr CartExp<LB> cb{};
   const FDiv fnt = fdiv(nt);
   for (int w = tid; w < nt * nrest; w += tpq) {
     const int rest = fq(w, fnt), t = w - rest * nt;
-    const int abcd0 = NCA * rest;
-    double gm[NCA];
-    bool any = false;
-#pragma unroll
-    for (int ca = 0; ca < NCA; ++ca) {
-      gm[ca] = Gp[t * Gs + abcd0 + ca];
-      any |= gm[ca] != 0.0;
-    }
-    if (!any) continue;
+    const int abcd0 = NCA * NCB * rest;
+    const double* g = Gp + t * Gs + abcd0;
     const int pk = IX[abcd0];
-    const int bx = 4 * ((pk & 255) - LA), by = J4 + 4 * ((pk >> 8) & 255), bz = 2 * J4 + 4 * (pk >> 16);
-    const double* Fb = F + (size_t)t * St;
-    for (int rl = 0; rl < nrw; ++rl, Fb += 3 * J4) {
-      double2 X01[LA + 1], X23[LA + 1], Y01[LA + 1], Y23[LA + 1], Z01[LA + 1], Z23[LA + 1];
+    const double* Fx = F + (size_t)t * St + 4 * ((pk & 255) - (LA + (LA + 1) * LB));
+    const double* Fy = F + (size_t)t * St + J4 + 4 * ((pk >> 8) & 255);
+    const double* Fz = F + (size_t)t * St + 2 * J4 + 4 * (pk >> 16);
+    constexpr bool kHold = NCA * NCB <= 6;  // the densities stay in registers over the roots
+    double gh[kHold ? NCA * NCB : 1];
+    if (kHold) {
 #pragma unroll
-      for (int k = 0; k <= LA; ++k) {
-        X01[k] = *reinterpret_cast<const double2*>(Fb + bx + 4 * k);
-        X23[k] = *reinterpret_cast<const double2*>(Fb + bx + 4 * k + 2);
-        Y01[k] = *reinterpret_cast<const double2*>(Fb + by + 4 * k);
-        Y23[k] = *reinterpret_cast<const double2*>(Fb + by + 4 * k + 2);
-        Z01[k] = *reinterpret_cast<const double2*>(Fb + bz + 4 * k);
-        Z23[k] = *reinterpret_cast<const double2*>(Fb + bz + 4 * k + 2);
+      for (int c = 0; c < NCA * NCB; ++c) gh[kHold ? c : 0] = g[c];
+    }
+    for (int rl = 0; rl < nrw; ++rl, Fx += 3 * J4, Fy += 3 * J4, Fz += 3 * J4) {
+      double X[N], Y[N], Z[N], U[N], V[N], W[N];
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        X[i] = Fx[4 * i];
+        Y[i] = Fy[4 * i];
+        Z[i] = Fz[4 * i];
+        U[i] = V[i] = W[i] = 0.0;
       }
 #pragma unroll
-      for (int ca = 0; ca < NCA; ++ca) {
-        const int ax = ce.e[ca][0], ay = ce.e[ca][1], az = ce.e[ca][2];
-        const double g = gm[ca];
-        const double gyz = g * Y01[ay].x * Z01[az].x, gxz = g * X01[ax].x * Z01[az].x, gxy = g * X01[ax].x * Y01[ay].x;
-        acc[0] = fma(gyz, X01[ax].y, acc[0]);
-        acc[1] = fma(gxz, Y01[ay].y, acc[1]);
-        acc[2] = fma(gxy, Z01[az].y, acc[2]);
-        acc[3] = fma(gyz, X23[ax].x, acc[3]);
-        acc[4] = fma(gxz, Y23[ay].x, acc[4]);
-        acc[5] = fma(gxy, Z23[az].x, acc[5]);
-        acc[6] = fma(gyz, X23[ax].y, acc[6]);
-        acc[7] = fma(gxz, Y23[ay].y, acc[7]);
-        acc[8] = fma(gxy, Z23[az].y, acc[8]);
+      for (int jb = 0; jb < NCB; ++jb)
+#pragma unroll
+        for (int ja = 0; ja < NCA; ++ja) {
+          const int x = ca.e[ja][0] + (LA + 1) * cb.e[jb][0], y = ca.e[ja][1] + (LA + 1) * cb.e[jb][1],
+                    z = ca.e[ja][2] + (LA + 1) * cb.e[jb][2];
+          const double gm = kHold ? gh[kHold ? ja + NCA * jb : 0] : g[ja + NCA * jb];
+          const double gx = gm * X[x], gy = gm * Y[y];
+          U[x] = fma(gy, Z[z], U[x]);
+          V[y] = fma(gx, Z[z], V[y]);
+          W[z] = fma(gx, Y[y], W[z]);
+        }
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        const double2 dx = *reinterpret_cast<const double2*>(Fx + 4 * i + 2);
+        const double2 dy = *reinterpret_cast<const double2*>(Fy + 4 * i + 2);
+        const double2 dz = *reinterpret_cast<const double2*>(Fz + 4 * i + 2);
+        acc[0] = fma(U[i], Fx[4 * i + 1], acc[0]);
+        acc[1] = fma(V[i], Fy[4 * i + 1], acc[1]);
+        acc[2] = fma(W[i], Fz[4 * i + 1], acc[2]);
+        acc[3] = fma(U[i], dx.x, acc[3]);
+        acc[4] = fma(V[i], dy.x, acc[4]);
+        acc[5] = fma(W[i], dz.x, acc[5]);
+        acc[6] = fma(U[i], dx.y, acc[6]);
+        acc[7] = fma(V[i], dy.y, acc[7]);
+        acc[8] = fma(W[i], dz.y, acc[8]);
       }
     }
   }
@@ -648,14 +667,22 @@ __global__ void __launch_bounds__(GradThreads<MINB>::value, MINB) grad_kernel(co
         }
         gsync(g, tpq);
         // ---- (4) Assg1: sum over Cartesian components and roots; consecutive threads
-        //      take consecutive primitive quartets of one Cartesian quartet (blocked over
-        //      the components of centre A for la = 1, 2; over those of centre B when
-        //      la = 0, which puts B first in the component order with unit stride)
+        //      take consecutive primitive quartets of one component block (the components
+        //      of centre A for la = 1, 2, with those of B where possible; those of centre
+        //      B when la = 0, which puts B first in the component order with unit stride)
         const int lblk = la > 0 ? la : lb;
-        if (lblk == 1) {
-          assg1_a_block<1>(F, Gp, IX, nt, ncart4 / 3, St, Gs, J4, nrw, tid, tpq, acc);
+        // both bra shells of (p p| in one block where the ket components still give every
+        // thread something to do ((p d| that way: 24 instead of 12 values per direction
+        // in registers, and class (4, 3) of the 460-function gradient 222 instead of
+        // 180 ms)
+        const int nket = ncc * ncd;
+        const bool two = la == 1 && lb == 1 && nt * nket >= tpq;
+        if (NAB1 == 3 && two) {
+          assg1_block<1, 1>(F, Gp, IX, nt, nket, St, Gs, J4, nrw, tid, tpq, acc);
+        } else if (lblk == 1) {
+          assg1_block<1, 0>(F, Gp, IX, nt, ncart4 / 3, St, Gs, J4, nrw, tid, tpq, acc);
         } else if (lblk == 2) {
-          assg1_a_block<2>(F, Gp, IX, nt, ncart4 / 6, St, Gs, J4, nrw, tid, tpq, acc);
+          assg1_block<2, 0>(F, Gp, IX, nt, ncart4 / 6, St, Gs, J4, nrw, tid, tpq, acc);
         } else {
           const FDiv fnt = fdiv(nt);
           for (int w = tid; w < nt * ncart4; w += tpq) {
