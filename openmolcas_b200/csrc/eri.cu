@@ -61,8 +61,8 @@ static size_t eri_group_smem(int nab, int ncd, const ClassStats& cs, int pab, in
   const size_t nt = (size_t)pab * pcd;
   const size_t tile = ev2s((size_t)cs.max_nij * pcd * cs.max_nef) + ev2s(nt * cfs) + nt * gst +
                       nt * (size_t)(cs.max_nef | 1);
-  return 2 + ev2s(cs.max_acc) + ev2s(cs.max_cab) + ev2s(cs.max_ccd) + ev2s((cs.max_ne + cs.max_nf + 1) / 2) +
-         std::max(tile, ev2s(cs.max_tmp));
+  return ev2s(2 + ev2s(cs.max_acc) + ev2s(cs.max_cab) + ev2s(cs.max_ccd) + ev2s((cs.max_ne + cs.max_nf + 1) / 2) +
+              std::max(tile, ev2s(cs.max_tmp)));
 }
 
 // tpq0: the first group size tried (0: from the widest stage); order: the tile

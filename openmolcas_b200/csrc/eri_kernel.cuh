@@ -74,6 +74,121 @@ __device__ __forceinline__ void ef_shell(const double* __restrict__ Ib, int fxo,
   for (int c = 0; c < NCL; ++c) out[c] = acc[c];
 }
 
+// [e0|f0] of the Cartesian shells LO and HI = LO + 1 together: the HI + 1 values
+// of a row serve both.
+template <int LO, int HI, int NR, int RS, int DS>
+__device__ __forceinline__ void ef_shells(const double* __restrict__ Ib, int fxo, int fyo, int fzo,
+                                          double* __restrict__ out) {
+  constexpr int NL = (LO + 1) * (LO + 2) / 2, NH = (HI + 1) * (HI + 2) / 2;
+  constexpr CartExp<LO> cl{};
+  constexpr CartExp<HI> ch{};
+  double acc[NL + NH];
+#pragma unroll
+  for (int c = 0; c < NL + NH; ++c) acc[c] = 0.0;
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    const double* px = Ib + r * RS + fxo;
+    const double* py = Ib + DS + r * RS + fyo;
+    const double* pz = Ib + 2 * DS + r * RS + fzo;
+    double X[HI + 1], Y[HI + 1], Z[HI + 1];
+#pragma unroll
+    for (int k = 0; k <= HI; ++k) {
+      X[k] = px[k];
+      Y[k] = py[k];
+      Z[k] = pz[k];
+    }
+#pragma unroll
+    for (int c = 0; c < NL; ++c) acc[c] = fma(X[cl.e[c][0]] * Y[cl.e[c][1]], Z[cl.e[c][2]], acc[c]);
+#pragma unroll
+    for (int c = 0; c < NH; ++c) acc[NL + c] = fma(X[ch.e[c][0]] * Y[ch.e[c][1]], Z[ch.e[c][2]], acc[NL + c]);
+  }
+#pragma unroll
+  for (int c = 0; c < NL + NH; ++c) out[c] = acc[c];
+}
+
+// s += c[0..3] v; AL: c is 16-byte aligned (two loads instead of four).  Where
+// fewer than four ij are left, the values past them belong to sums that are not
+// stored.
+template <bool AL>
+__device__ __forceinline__ void eri_load4(const double* __restrict__ c, double (&v)[4]) {
+  if (AL) {
+    const double2 a = *reinterpret_cast<const double2*>(c), b = *reinterpret_cast<const double2*>(c + 2);
+    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = c[k];
+  }
+}
+template <bool AL>
+__device__ __forceinline__ void eri_axpy4(const double* __restrict__ c, double x, double (&s)[4]) {
+  double v[4];
+  eri_load4<AL>(c, v);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) s[k] = fma(v[k], x, s[k]);
+}
+template <bool AL>
+__device__ __forceinline__ void eri_axpy42(const double* __restrict__ c, double x0, double x1, double (&s0)[4],
+                                           double (&s1)[4]) {
+  double v[4];
+  eri_load4<AL>(c, v);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    s0[k] = fma(v[k], x0, s0[k]);
+    s1[k] = fma(v[k], x1, s1[k]);
+  }
+}
+// x[0], x[st], .. += s, the first n of four
+__device__ __forceinline__ void eri_add4(double* __restrict__ x, int st, int n, const double (&s)[4]) {
+  x[0] += s[0];
+  if (n > 1) x[st] += s[1];
+  if (n > 2) x[2 * st] += s[2];
+  if (n > 3) x[3 * st] += s[3];
+}
+
+// Largest NI * NJ whose recursion may run one thread per job (the large tables
+// have few quartets per tile, and the second form costs them registers).
+constexpr int kEriJobMax = 20;
+
+// The 2D recursion with one thread per (direction, root, quartet) job, the
+// quartet fastest (the odd quartet stride keeps the 32 lanes' accesses in
+// different banks): two columns of NI values in registers, no exchange between
+// lanes.  It needs about a fifth of the instructions of the NI-lane form, which
+// stays for waves whose jobs would leave more than half of the group idle.
+template <int NI, int NJ, int NR, int RS, int DS, int GST, int CFS>
+__device__ __forceinline__ void eri_jobs_thread(const double* __restrict__ cf, double* __restrict__ I, int nt,
+                                                const FDiv& fnt, int tid, int tpq) {
+  for (int job = tid; job < nt * NR * 3; job += tpq) {
+    const int u = fq(job, fnt), t = job - u * nt, d = u / NR, r = u - d * NR;
+    const double* c = cf + t * CFS + r * 10;
+    const double B00 = c[0], B10 = c[1], B01 = c[2], C00 = c[3 + d], D00 = c[6 + d];
+    double* Io = I + (size_t)t * GST + d * DS + r * RS;
+    double cur[NI], prev[NI];
+    cur[0] = d == 2 ? c[9] : 1.0;
+    if (NI > 1) cur[NI > 1 ? 1 : 0] = C00 * cur[0];
+#pragma unroll
+    for (int i = 1; i < NI - 1; ++i) cur[i + 1] = fma(i * B10, cur[i - 1], C00 * cur[i]);
+#pragma unroll
+    for (int e = 0; e < NI; ++e) {
+      Io[e] = cur[e];
+      prev[e] = 0.0;
+    }
+#pragma unroll
+    for (int j = 0; j < NJ - 1; ++j) {
+      double below = 0.0;  // I[e-1][j]
+#pragma unroll
+      for (int e = 0; e < NI; ++e) {
+        double v = D00 * cur[e];
+        if (j > 0) v = fma(j * B01, prev[e], v);
+        if (e > 0) v = fma(e * B00, below, v);
+        below = cur[e];
+        prev[e] = below;
+        cur[e] = v;
+        Io[(j + 1) * NI + e] = v;
+      }
+    }
+  }
+}
+
 // Per-group shared layout (doubles, every region even):
 //   hdr[2] | acc | Cab | Ccd | Ft (ints) | union{ HRR temp | X | tile: cf | I | E }
 // I holds per primitive quartet [dir][root][f][e] (stride GST, odd); E per
@@ -121,7 +236,13 @@ __global__ void __launch_bounds__(kEriThreads, 1) eri_kernel(const EriArgs a, co
     double* I = cf + ev2(NT * CFS);
     double* E = I + NT * GST;
     for (int o = tid; o < nacc; o += tpq) acc[o] = 0.0;
-    for (int o = tid; o < nij * npab; o += tpq) Cab[o] = a.coef[P.coef_off + o];
+    {
+      const FDiv fab = fdiv(npab);
+      for (int o = tid; o < nij * npab; o += tpq) {  // bra coefficients as [primitive pair][ij]
+        const int ij = fq(o, fab);
+        Cab[(o - ij * npab) * nij + ij] = a.coef[P.coef_off + o];
+      }
+    }
     for (int o = tid; o < nklc * npcd; o += tpq) Ccd[o] = a.coef[Q.coef_off + (size_t)it.c0 * npcd + o];
     {  // packed offsets of the Cartesian f components (f * NI per direction) into one root of I
       const int foff = d_ccum(Q.emin);
@@ -149,12 +270,14 @@ __global__ void __launch_bounds__(kEriThreads, 1) eri_kernel(const EriArgs a, co
           const double zeta = prim[ia], eta = prim[ic];
           const double px = prim[2 * tot_np + ia], py = prim[3 * tot_np + ia], pz = prim[4 * tot_np + ia];
           const double qx = prim[2 * tot_np + ic], qy = prim[3 * tot_np + ic], qz = prim[4 * tot_np + ic];
-          const double ze = zeta + eta, zei = 1.0 / ze, rho = zeta * eta * zei;
+          double zei, rzei;  // 1 / (zeta + eta) and its root
+          recip_root(zeta + eta, zei, rzei);
+          const double rho = zeta * eta * zei;
           const double dx = px - qx, dy = py - qy, dz = pz - qz;
           const double T = rho * (dx * dx + dy * dy + dz * dz);
           double x, w;
           rys_one<NR>(ra, T, r, x, w);
-          const double fact = prim[tot_np + ia] * prim[tot_np + ic] * sqrt(zei);
+          const double fact = prim[tot_np + ia] * prim[tot_np + ic] * rzei;
           const double U2 = x * zei;
           double* c = cf + t * CFS + r * 10;
           c[0] = 0.5 * U2;
@@ -170,10 +293,14 @@ __global__ void __launch_bounds__(kEriThreads, 1) eri_kernel(const EriArgs a, co
         }
         gsync(g, tpq);
         if (NI * NJ > 1) {
-          // ---- 1b: 2D recursion, one NI-lane warp segment per (quartet, root, direction)
-          //      (32/NI jobs per warp): I[e][f+1] = D00 I[e][f] + f B01 I[e][f-1] + e B00 I[e-1][f]
-          constexpr int JPW = 32 / NI;
+          // ---- 1b: 2D recursion I[e][f+1] = D00 I[e][f] + f B01 I[e][f-1] + e B00 I[e-1][f],
+          //      a thread per (quartet, root, direction) when that fills half of the group,
+          //      else one NI-lane warp segment each (32/NI jobs per warp)
           const int njobs = nt * NR * 3;
+          if (NI * NJ <= kEriJobMax && 2 * njobs >= tpq) {
+            if constexpr (NI * NJ <= kEriJobMax) eri_jobs_thread<NI, NJ, NR, RS, DS, GST, CFS>(cf, I, nt, fdiv(nt), tid, tpq);
+          } else {
+          constexpr int JPW = 32 / NI;
           const int lane = tid & 31;
           const int seg = lane / NI, e = lane - seg * NI;  // seg >= JPW: spare lanes
           const int lup = (lane + 31) & 31;
@@ -204,10 +331,23 @@ __global__ void __launch_bounds__(kEriThreads, 1) eri_kernel(const EriArgs a, co
               if (valid) Io[(j + 1) * NI] = v;
             }
           }
+          }
           gsync(g, tpq);
           // ---- 2a: [e0|f0] = sum_r Ix Iy Iz, one thread per (quartet, f, bra shell L);
           //      consecutive lanes on consecutive quartets
-          {
+          // all shells of the bra range in one thread where (quartet, f) alone fills the group
+          const int emin_ = P.emin;
+          if ((NAB == 2 && emin_ == 1 && nt * nf >= tpq) || (NAB == 3 && emin_ == 2 && nt * nf >= tpq)) {
+            if constexpr (NAB == 2 || NAB == 3) {
+              const FDiv fnt = fdiv(nt);
+              for (int w = tid; w < nt * nf; w += tpq) {
+                const int jf = fq(w, fnt), t = w - jf * nt;
+                const int pf = Ft[jf];
+                ef_shells<NAB - 1, NAB, NR, RS, DS>(I + (size_t)t * GST, pf & 255, (pf >> 8) & 255, pf >> 16,
+                                                    E + (size_t)t * Est + (size_t)ne * jf);
+              }
+            }
+          } else {
             const int emin = P.emin, nsh = NAB - emin + 1;
             const int c0 = d_ccum(emin);
             const FDiv fnt = fdiv(nt), fnf = fdiv(nf);
@@ -234,29 +374,48 @@ __global__ void __launch_bounds__(kEriThreads, 1) eri_kernel(const EriArgs a, co
           for (int t = tid; t < nt; t += tpq) E[(size_t)t * Est] = cf[t * CFS + 9];
         }
         gsync(g, tpq);
-        // ---- 2b1: bra half-transform  X[ij][pc][ef] += sum_pa Cab[ij][pa] E[pa,pc][ef];
-        //      a thread makes 4 consecutive ij of one (pc, ef), each E load feeds 4 FMAs
+        // ---- 2b1: bra half-transform  X[ij][pc][ef] += sum_pa Cab[pa][ij] E[pa,pc][ef]
         {
-          const int nij4 = (nij + 3) >> 2;
-          const FDiv fnef = fdiv(nef), fnpc = fdiv(npc);
-          for (int o = tid; o < nij4 * npc * nef; o += tpq) {
-            const int r1 = fq(o, fnef), ef = o - r1 * nef, q = fq(r1, fnpc), pc = r1 - q * npc;
-            const int ij0 = 4 * q;
-            const double* ca = Cab + ij0 * npab + pab0;
+          const int nij4 = (nij + 3) >> 2, nout = nij4 * npc * nef;
+          const FDiv fnpc = fdiv(npc);
+          const double* Cb = Cab + pab0 * nij;
+          // few outputs (classes with s shells): 2^sh lanes share one, each every 2^sh-th pa
+          int sh = 0;
+          while (sh < 5 && (nout << (sh + 1)) <= tpq && (2 << sh) <= npa) ++sh;
+          if (sh > 0) {
+            const FDiv fnef = fdiv(nef);
+            const int o = tid >> sh, l = tid & ((1 << sh) - 1), oc = min(o, nout - 1);
+            const int r1 = fq(oc, fnef), ef = oc - r1 * nef, q = fq(r1, fnpc), pc = r1 - q * npc;
             const double* e = E + (size_t)pc * npa * Est + ef;
-            double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-            for (int pa = 0; pa < npa; ++pa) {
-              const double ev = e[(size_t)pa * Est];
-              s0 = fma(ca[pa], ev, s0);
-              if (ij0 + 1 < nij) s1 = fma(ca[npab + pa], ev, s1);
-              if (ij0 + 2 < nij) s2 = fma(ca[2 * npab + pa], ev, s2);
-              if (ij0 + 3 < nij) s3 = fma(ca[3 * npab + pa], ev, s3);
+            double s[4] = {0.0, 0.0, 0.0, 0.0};
+            for (int pa = l; pa < npa; pa += 1 << sh) eri_axpy4<false>(Cb + pa * nij + 4 * q, e[(size_t)pa * Est], s);
+            for (int w = 1 << (sh - 1); w > 0; w >>= 1) {
+#pragma unroll
+              for (int k = 0; k < 4; ++k) s[k] += __shfl_xor_sync(0xffffffffu, s[k], w);
             }
-            double* x = X + ef + nef * (pc + PCD * ij0);
-            x[0] += s0;
-            if (ij0 + 1 < nij) x[nef * PCD] += s1;
-            if (ij0 + 2 < nij) x[2 * nef * PCD] += s2;
-            if (ij0 + 3 < nij) x[3 * nef * PCD] += s3;
+            if (l == 0 && o < nout) eri_add4(X + ef + nef * (pc + PCD * 4 * q), nef * PCD, nij - 4 * q, s);
+          } else {
+            // four ij and two ef per thread: two coefficient and two E loads feed eight FMAs
+            const int half = (nef + 1) >> 1;
+            const FDiv fhalf = fdiv(half);
+            for (int o = tid; o < nij4 * npc * half; o += tpq) {
+              const int r1 = fq(o, fhalf), ef = o - r1 * half, q = fq(r1, fnpc), pc = r1 - q * npc;
+              const bool two = ef + half < nef;
+              const double* e = E + (size_t)pc * npa * Est + ef;
+              const double* e1 = two ? e + half : e;
+              const double* c = Cb + 4 * q;
+              double s0[4] = {0.0, 0.0, 0.0, 0.0}, s1[4] = {0.0, 0.0, 0.0, 0.0};
+              if (nij & 1) {
+#pragma unroll 2
+                for (int pa = 0; pa < npa; ++pa, c += nij, e += Est, e1 += Est) eri_axpy42<false>(c, *e, *e1, s0, s1);
+              } else {
+#pragma unroll 2
+                for (int pa = 0; pa < npa; ++pa, c += nij, e += Est, e1 += Est) eri_axpy42<true>(c, *e, *e1, s0, s1);
+              }
+              double* x = X + ef + nef * (pc + PCD * 4 * q);
+              eri_add4(x, nef * PCD, nij - 4 * q, s0);
+              if (two) eri_add4(x + half, nef * PCD, nij - 4 * q, s1);
+            }
           }
         }
       }
