@@ -166,8 +166,9 @@ __global__ void k_oz_lexp(const int* __restrict__ inv, int n, int64_t nrs, const
 // column a: 16 consecutive K bytes of row b of every slice, cut with row b's
 // cached exponent and packed in registers; the two threads of a row write its
 // 32 bytes of a slice, so a warp's store is 512 contiguous bytes (the blocked
-// layout of oz_blk_off).  The grid covers all ld columns a, so the K padding
-// a >= n is written as zeros (as are the rows b >= n).
+// layout of oz_blk_off).  The grid covers the K steps that the half-transform
+// reads: the padding a >= n of the last one is written as zeros, as are the rows
+// b >= n.
 // Cut: z = x 2^(8S-1-e), rounded to the nearest integer (at most half a unit of
 // the last slice; 2^(8S-1) itself, from a value just below it, becomes the
 // integer before).  For S <= 6 adding 1.5 2^52 leaves the two's-complement
@@ -552,7 +553,7 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
     oz_plan(ak, sk, 128);
     if (ax.stages < 2 || ak.stages < 2) { h->err = "mixed J/K: slice tiles do not fit in shared memory"; return MG_ERR_ARG; }
     ax.err = ak.err = d_err;
-    ax.nrt = ld / 128; ax.nnt = q.nnt; ax.ld = ld; ax.n = n; ax.r = q.r; ax.eA = eA; ax.fB = q.fC; ax.X = Xf;
+    ax.nrt = ld / 128; ax.nnt = q.nnt; ax.ld = ld; ax.kx = rup(n, kOzCutCols); ax.n = n; ax.r = q.r; ax.eA = eA; ax.fB = q.fC; ax.X = Xf;
     ax.xld = ld; ax.xmax = xmax;
     ak.ld = ld; ak.n = n; ak.ntile = ntile; ak.nsub = q.nsub; ak.kblk = q.kblk; ak.ksub = q.ksub; ak.eX = q.eX;
     ak.P = P; ak.K = q.K;
@@ -588,7 +589,7 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
       if (!Lb) { h->err = "vector block straddles storage blocks"; return MG_ERR_ARG; }
       oz_with_slices(s, [&](auto S) {
         k_oz_slice_l<decltype(S)::value>
-            <<<dim3(ld / kOzCutRows, ld / kOzCutCols, (nv + kOzVecs - 1) / kOzVecs), 2 * kOzCutRows, 0, st>>>(
+            <<<dim3(ld / kOzCutRows, (n + kOzCutCols - 1) / kOzCutCols, (nv + kOzVecs - 1) / kOzVecs), 2 * kOzCutRows, 0, st>>>(
                 inv, n, nrs, Lb, nv, ld, (int64_t)nb * ld * ld, eL + (size_t)J0 * ld, LS, eA);
       });
       if (!launched("k_oz_slice_l")) return MG_ERR_CUDA;
@@ -698,7 +699,7 @@ int oz_selftest(Handle* h, int ld, int r, int s, const double* d_A, const double
   });
   if (!attr) return MG_ERR_CUDA;
   ax.err = ak.err = d_err;
-  ax.nrt = ld / 128; ax.nnt = nnt; ax.ld = ld; ax.n = ld; ax.r = r; ax.eA = eA; ax.fB = fC; ax.X = d_X; ax.xld = ld;
+  ax.nrt = ld / 128; ax.nnt = nnt; ax.ld = ax.kx = ld; ax.n = ld; ax.r = r; ax.eA = eA; ax.fB = fC; ax.X = d_X; ax.xld = ld;
   ax.xmax = xmax; ax.nJ = 1; ax.nitems = ax.nrt * nnt;
   ak.ld = ld; ak.n = ld; ak.ntile = (ld / 128) * (ld / 128 + 1) / 2; ak.nsub = nsub; ak.kblk = kblk; ak.ksub = ksub;
   ak.eX = eX; ak.P = P; ak.K = d_K; ak.nblk = 1; ak.nitems = ak.ntile * nsub;

@@ -90,7 +90,8 @@ struct OzArgs {
   int* err;
   // half-transform X_J = L_J C (SYRK == false): items (row tile, vector, column tile)
   int nrt, nJ, nnt;
-  int ld;          // rows (and K extent) of one vector's square
+  int ld;          // rows of one vector's square
+  int kx;          // K extent that is read (multiple of 32; the slices are zero beyond n)
   int n;           // valid rows / columns (nbf)
   int r;           // columns of C
   const int* eA;   // row exponents of the L slices, [J * ld + a]
@@ -131,7 +132,7 @@ template <bool SYRK, typename F>
 __device__ __forceinline__ void oz_for_units(const OzArgs& a, F&& f) {
   const int npass = (a.s + a.nd - 1) / a.nd;
   if (!SYRK) {
-    const int nsubk = (a.ld + kOzKChunk - 1) / kOzKChunk;
+    const int nsubk = (a.kx + kOzKChunk - 1) / kOzKChunk;
     for (int item = blockIdx.x; item < a.nitems; item += gridDim.x) {
       const int nt = item % a.nnt, r1 = item / a.nnt, J = r1 % a.nJ, rt = r1 / a.nJ;
       for (int sk = 0; sk < nsubk; ++sk)
@@ -140,7 +141,7 @@ __device__ __forceinline__ void oz_for_units(const OzArgs& a, F&& f) {
           u.rowA = J * a.ld + rt * 128;
           u.rowB = nt * a.Nt;
           u.k0 = sk * kOzKChunk;
-          u.nk = (min(a.ld, u.k0 + kOzKChunk) - u.k0) / 32;
+          u.nk = (min(a.kx, u.k0 + kOzKChunk) - u.k0) / 32;
           u.d0 = g * a.nd;
           u.d1 = min(a.s, u.d0 + a.nd);
           u.same = false;
