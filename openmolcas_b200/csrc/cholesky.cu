@@ -272,34 +272,46 @@ __global__ void __launch_bounds__(kUpdThreads) k_cho_subtr(const ChoUpd u) {
       lqv[v] = (o < kUpdJ * NK && j0 + jj < je && i < u.ni) ? __ldg(u.lq + (size_t)(j0 + jj) * u.nq + ssel[i]) : 0.0;
     }
   };
-  stage(jb);
-  int s = 0;
-  for (int j0 = jb; j0 < je; j0 += kUpdJ, s ^= 1) {
-    double* sf = &sl[s][0][0];
+  // eight vectors of both rows are in flight while the eight before them are used
+  double x0[8], x1[8];
+  auto load = [&](int j) {
+    const double* Lp = u.Lt[j / kVecBlock] + u.nrs * (j % kVecBlock);
 #pragma unroll
-    for (int v = 0; v < KV; ++v)
-      if (tid + v * kUpdThreads < kUpdJ * NK) sf[tid + v * kUpdThreads] = lqv[v];
-    __syncthreads();
-    if (j0 + kUpdJ < je) stage(j0 + kUpdJ);
-    const int nj = min(kUpdJ, je - j0);
-    const double* Lp = u.Lt[j0 / kVecBlock] + u.nrs * (j0 % kVecBlock);
-    for (int q = 0; q < nj; q += 8) {
-      double x0[8], x1[8];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const double* p = Lp + u.nrs * (q + e);
-        x0[e] = a0 && q + e < nj ? __ldg(p + t0) : 0.0;
-        x1[e] = a1 && q + e < nj ? __ldg(p + t1) : 0.0;
-      }
-#pragma unroll
-      for (int e = 0; e < 8; ++e)
-#pragma unroll
-        for (int i = 0; i < NK; ++i) {
-          const double l = sl[s][q + e][i];
-          acc[0][i] = fma(x0[e], l, acc[0][i]);
-          acc[1][i] = fma(x1[e], l, acc[1][i]);
-        }
+    for (int e = 0; e < 8; ++e) {
+      const double* p = Lp + u.nrs * e;
+      x0[e] = a0 && j + e < je ? __ldg(p + t0) : 0.0;
+      x1[e] = a1 && j + e < je ? __ldg(p + t1) : 0.0;
     }
+  };
+  stage(jb);
+  if (jb < je) load(jb);
+  int s = 1;
+  for (int j = jb; j < je; j += 8) {
+    const int q = (j - jb) % kUpdJ;
+    if (q == 0) {
+      s ^= 1;
+      double* sf = &sl[s][0][0];
+#pragma unroll
+      for (int v = 0; v < KV; ++v)
+        if (tid + v * kUpdThreads < kUpdJ * NK) sf[tid + v * kUpdThreads] = lqv[v];
+      __syncthreads();
+      if (j + kUpdJ < je) stage(j + kUpdJ);
+    }
+    double y0[8], y1[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      y0[e] = x0[e];
+      y1[e] = x1[e];
+    }
+    if (j + 8 < je) load(j + 8);
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+#pragma unroll
+      for (int i = 0; i < NK; ++i) {
+        const double l = sl[s][q + e][i];
+        acc[0][i] = fma(y0[e], l, acc[0][i]);
+        acc[1][i] = fma(y1[e], l, acc[1][i]);
+      }
   }
   double* p = u.part + (size_t)blockIdx.y * u.ni * u.nrs;
 #pragma unroll
@@ -932,10 +944,11 @@ void cho_rs_list(const ChoState* c, int32_t* a, int32_t* b, int32_t* sp) {
 }
 int cho_copy_vectors(const ChoState* c, int first, int count, double* d_out, cudaStream_t st) {
   if (first < 0 || count < 0 || first + count > c->M) return MG_ERR_ARG;
-  for (int k = 0; k < count; ++k) {
-    const int J = first + k;
+  for (int k = 0; k < count;) {  // one copy per storage block
+    const int J = first + k, n = std::min(count - k, kVecBlock - J % kVecBlock);
     cudaMemcpyAsync(d_out + c->nrs * k, c->Lblk[J / kVecBlock] + (size_t)c->nrs * (J % kVecBlock),
-                    sizeof(double) * c->nrs, cudaMemcpyDeviceToDevice, st);
+                    sizeof(double) * c->nrs * n, cudaMemcpyDeviceToDevice, st);
+    k += n;
   }
   return 0;
 }
