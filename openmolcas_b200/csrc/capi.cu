@@ -102,6 +102,10 @@ int build_eri_items(Handle* h, const int32_t* q4, int64_t nq, const int64_t* off
   }
   items.clear();
   classes.clear();
+  size_t total = 0;
+  for (const auto& v : byc) total += v.size();
+  items.reserve(total);
+  std::vector<std::pair<long long, int64_t>> order;
   for (int key = 0; key < 64; ++key) {
     auto& v = byc[key];
     if (v.empty()) continue;
@@ -116,13 +120,15 @@ int build_eri_items(Handle* h, const int32_t* q4, int64_t nq, const int64_t* off
       h->err = "mg_eri_quartets: class does not fit in shared memory";
       return MG_ERR_ARG;
     }
-    // heaviest quartets first so the groups of one CTA carry similar work
-    std::stable_sort(v.begin(), v.end(), [&](const EriItem& a, const EriItem& b) {
-      const long long wa = (long long)h->pairs[a.p].np * h->pairs[a.q].np * (a.c1 - a.c0);
-      const long long wb = (long long)h->pairs[b.p].np * h->pairs[b.q].np * (b.c1 - b.c0);
-      return wa > wb;
-    });
-    items.insert(items.end(), v.begin(), v.end());
+    // heaviest quartets first so the groups of one CTA carry similar work, in the
+    // caller's order where equal: the complement of the work above the index
+    order.resize(v.size());
+    for (size_t k = 0; k < v.size(); ++k) {
+      const long long w = (long long)h->pairs[v[k].p].np * h->pairs[v[k].q].np * (v[k].c1 - v[k].c0);
+      order[k] = {-w, (int64_t)k};
+    }
+    std::sort(order.begin(), order.end());
+    for (const auto& o : order) items.push_back(v[o.second]);
     classes.push_back(c);
   }
   return 0;

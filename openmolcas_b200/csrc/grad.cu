@@ -19,7 +19,11 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
+#include <functional>
+#include <map>
+#include <unordered_map>
 #include <vector>
 
 #include "grad_kernel.cuh"
@@ -96,9 +100,47 @@ static inline int c_ncd1(int key) { return key % 8; }
 static const size_t kCtaLimit = 227 * 1024;
 static const size_t kGradMaxBudget = kCtaLimit / 8 - kGTabD;  // one group, doubles
 
+// Planning works on kinds of quartets, not on quartets: pairs of the same kind (l,
+// contracted functions, primitive pairs) have the same chunks, tiles and sort key,
+// so a plan of 1.7 million quartets looks at some ten thousand kinds (per-quartet
+// planning took 0.35 s of the first 460-function gradient, 0.12 s this way).
+struct QuartetKind {
+  int cij = 0, ckl = 0;  // contracted chunk; 0: not met yet
+  int key = 0;           // class
+  int rank = 0;          // place of its primitive-quartet count among its class's, largest first
+  long long count = 0;   // work items
+  int p = 0, q = 0;      // a quartet of the kind
+};
+
 int grad_build(Handle* h, double cutint, GradPlan& plan) {
   const int ns = h->sh.size();
+  // kinds of pairs
+  std::vector<int> pkind(h->pairs.size());
+  std::map<std::array<int, 5>, int> kinds;
+  for (size_t k = 0; k < h->pairs.size(); ++k) {
+    const DPair& P = h->pairs[k];
+    pkind[k] = kinds.emplace(std::array<int, 5>{P.la, P.lb, P.nci, P.ncj, P.np}, (int)kinds.size()).first->second;
+  }
+  const size_t T = kinds.size();
+  std::vector<QuartetKind> qk;
+  // number of a quartet's kind, from a table where that is small
+  std::vector<int> dense(T * T <= ((size_t)1 << 22) ? T * T : 0, -1);
+  std::unordered_map<size_t, int> sparse;
+  auto kind_of = [&](int p, int q) {
+    const size_t k = pkind[p] * T + pkind[q];
+    if (dense.empty()) {
+      const auto e = sparse.emplace(k, (int)qk.size());
+      if (e.second) qk.emplace_back();
+      return e.first->second;
+    }
+    if (dense[k] < 0) {
+      dense[k] = (int)qk.size();
+      qk.emplace_back();
+    }
+    return dense[k];
+  };
   std::vector<std::vector<GradItem>> byc(64);
+  std::vector<std::vector<int>> met(64);  // the kinds of each class
   struct Mx { int npab = 0, npcd = 0; };
   std::vector<Mx> mx(64);
   for (int i = 0; i < ns; ++i)
@@ -114,25 +156,34 @@ int grad_build(Handle* h, double cutint, GradPlan& plan) {
           if (P.atom_a == P.atom_b && P.atom_a == Q.atom_a && P.atom_a == Q.atom_b) continue;
           const int deg = (i == j ? 1 : 2) * (k == l ? 1 : 2) * (p == q ? 1 : 2);
           const int nkl = Q.nci * Q.ncj, nij = P.nci * P.ncj;
-          // chunk the contracted block (kl first, then ij) only when one quartet tile
-          // cannot fit at all: every chunk repeats the primitive-quartet work
-          int ckl = nkl, cij = nij;
-          while ((ckl > 1 || cij > 1) && grad_group_smem(P, Q, cij, ckl, 1, 1, 1) > kGradMaxBudget) {
-            if (ckl > 1) ckl = (ckl + 1) / 2;
-            else cij = (cij + 1) / 2;
+          const int kind = kind_of(p, q);
+          QuartetKind& K = qk[kind];
+          if (!K.cij) {
+            // chunk the contracted block (kl first, then ij) only when one quartet tile
+            // cannot fit at all: every chunk repeats the primitive-quartet work
+            int ckl = nkl, cij = nij;
+            while ((ckl > 1 || cij > 1) && grad_group_smem(P, Q, cij, ckl, 1, 1, 1) > kGradMaxBudget) {
+              if (ckl > 1) ckl = (ckl + 1) / 2;
+              else cij = (cij + 1) / 2;
+            }
+            if (grad_group_smem(P, Q, cij, ckl, 1, 1, 1) > kGradMaxBudget) {
+              h->err = "gradient quartet does not fit in shared memory";
+              return MG_ERR_ARG;
+            }
+            K.cij = cij;
+            K.ckl = ckl;
+            K.key = (P.la + P.lb + 1) * 8 + (Q.la + Q.lb + 1);
+            K.p = p;
+            K.q = q;
+            met[K.key].push_back(kind);
+            Mx& m = mx[K.key];
+            m.npab = std::max(m.npab, P.np);
+            m.npcd = std::max(m.npcd, Q.np);
           }
-          if (grad_group_smem(P, Q, cij, ckl, 1, 1, 1) > kGradMaxBudget) {
-            h->err = "gradient quartet does not fit in shared memory";
-            return MG_ERR_ARG;
-          }
-          const int key = (P.la + P.lb + 1) * 8 + (Q.la + Q.lb + 1);
-          Mx& m = mx[key];
-          for (int i0 = 0; i0 < nij; i0 += cij)
-            for (int c0 = 0; c0 < nkl; c0 += ckl) {
-              GradItem it{p, q, c0, std::min(nkl, c0 + ckl), i0, std::min(nij, i0 + cij), 0.5 * deg};
-              byc[key].push_back(it);
-              m.npab = std::max(m.npab, P.np);
-              m.npcd = std::max(m.npcd, Q.np);
+          for (int i0 = 0; i0 < nij; i0 += K.cij)
+            for (int c0 = 0; c0 < nkl; c0 += K.ckl) {
+              byc[K.key].push_back({p, q, c0, std::min(nkl, c0 + K.ckl), i0, std::min(nij, i0 + K.cij), 0.5 * deg});
+              ++K.count;
             }
         }
     }
@@ -142,22 +193,34 @@ int grad_build(Handle* h, double cutint, GradPlan& plan) {
   for (int key = 0; key < 64; ++key) {
     if (byc[key].empty()) continue;
     auto& v = byc[key];
-    std::stable_sort(v.begin(), v.end(), [&](const GradItem& a, const GradItem& b) {
-      return (long long)h->pairs[a.p].np * h->pairs[a.q].np > (long long)h->pairs[b.p].np * h->pairs[b.q].np;
-    });
+    // most primitive quartets first, in their order of generation where equal
+    std::map<long long, std::vector<int>, std::greater<long long>> by_work;
+    for (int k : met[key]) by_work[(long long)h->pairs[qk[k].p].np * h->pairs[qk[k].q].np].push_back(k);
+    std::vector<size_t> at;
+    size_t next = 0;
+    for (const auto& w : by_work) {
+      for (int k : w.second) qk[k].rank = (int)at.size();
+      at.push_back(next);
+      for (int k : w.second) next += qk[k].count;
+    }
+    const size_t base = plan.items.size();
+    plan.items.resize(base + v.size());
+    for (const GradItem& it : v) plan.items[base + at[qk[kind_of(it.p, it.q)].rank]++] = it;
+    const int nitems = (int)v.size();
     // tile: largest PAB x PCD (<= 8 x 4 primitive quartets) whose worst item fits the CTA budget
+    // (the first chunk of a kind is its largest)
     auto worst = [&](int a, int c, int rw) {
       size_t w = 0;
-      for (const GradItem& it : v)
-        w = std::max(w, grad_group_smem(h->pairs[it.p], h->pairs[it.q], it.i1 - it.i0, it.c1 - it.c0, a, c, rw));
+      for (int k : met[key])
+        w = std::max(w, grad_group_smem(h->pairs[qk[k].p], h->pairs[qk[k].q], qk[k].cij, qk[k].ckl, a, c, rw));
       return w;
     };
     const int NRc = (c_nab1(key) + c_ncd1(key) + 1) / 2;
     const Mx& m = mx[key];
     // widest per-quartet stage of the class (threads that can work at once)
     size_t wmax = 0;
-    for (const GradItem& it : v) {
-      const DPair &P = h->pairs[it.p], &Q = h->pairs[it.q];
+    for (int k : met[key]) {
+      const DPair &P = h->pairs[qk[k].p], &Q = h->pairs[qk[k].q];
       const size_t n4 = (size_t)ncart(P.la) * ncart(P.lb) * ncart(Q.la) * ncart(Q.lb);
       const size_t nU = (size_t)(P.la + 2) * (P.lb + 2) * (Q.la + 2) * (Q.lb + 1);
       wmax = std::max({wmax, n4, (size_t)3 * NRc * nU});
@@ -176,15 +239,15 @@ int grad_build(Handle* h, double cutint, GradPlan& plan) {
       // whole CTA takes one item, in the largest tile that fits (from 64 x 64 primitive
       // pairs, the larger dimension shrinks).  Above that the table's throughput tiles
       // are faster.  24 functions (406 quartets): 660 -> 292 us a gradient.
-      const bool small = (int)v.size() <= h->nsm && !h->grad_fixed[key];
+      const bool small = nitems <= h->nsm && !h->grad_fixed[key];
       const int order = small ? 3 : h->grad_order[key];
       const int cab = small ? 64 : h->grad_cap[key] ? 32 : 16, ccd = small ? 64 : h->grad_cap[key] ? 16 : 8;
       const int tpq0 = small ? nthr : h->grad_tpq[key] ? h->grad_tpq[key] : (wmax <= 512 ? 128 : 256);
       // a tile fits when its shared memory is within the group's share and every
       // run-time loop extent x divisor of the kernel stays below 2^32
       auto div_ok = [&](int a, int c, int rw) {
-        for (const GradItem& it : v)
-          if (grad_div_bound(h->pairs[it.p], h->pairs[it.q], it.i1 - it.i0, a, c, rw) >= 4294967296.0) return false;
+        for (int k : met[key])
+          if (grad_div_bound(h->pairs[qk[k].p], h->pairs[qk[k].q], qk[k].cij, a, c, rw) >= 4294967296.0) return false;
         return true;
       };
       for (int tpq = tpq0; tpq <= nthr && !c.tpq; tpq *= 2) {
@@ -213,23 +276,23 @@ int grad_build(Handle* h, double cutint, GradPlan& plan) {
       }
     }
     if (!c.tpq) { h->err = "gradient class does not fit in shared memory"; return MG_ERR_ARG; }
-    for (const GradItem& it : v)
-      if (grad_div_bound(h->pairs[it.p], h->pairs[it.q], it.i1 - it.i0, c.pab, c.pcd, c.rw) >= 4294967296.0) {
+    for (int k : met[key])
+      if (grad_div_bound(h->pairs[qk[k].p], h->pairs[qk[k].q], qk[k].cij, c.pab, c.pcd, c.rw) >= 4294967296.0) {
         h->err = "gradient work item exceeds the kernel's index range";
         return MG_ERR_ARG;
       }
     c.nab1 = key / 8;
     c.ncd1 = key % 8;
-    c.begin = plan.items.size();
-    c.count = v.size();
+    c.begin = (int)base;
+    c.count = nitems;
     c.work = 0;
-    for (const GradItem& it : v) {  // primitive quartets x Cartesian components x roots
-      const DPair &P = h->pairs[it.p], &Q = h->pairs[it.q];
-      c.work += (double)P.np * Q.np * ncart(P.la) * ncart(P.lb) * ncart(Q.la) * ncart(Q.lb) * NRc;
+    for (int k : met[key]) {  // primitive quartets x Cartesian components x roots
+      const DPair &P = h->pairs[qk[k].p], &Q = h->pairs[qk[k].q];
+      c.work += (double)qk[k].count * P.np * Q.np * ncart(P.la) * ncart(P.lb) * ncart(Q.la) * ncart(Q.lb) * NRc;
     }
     c.scr = 0;
-    for (const GradItem& it : v)
-      c.scr = std::max<long long>(c.scr, grad_item_scratch(h->pairs[it.p], h->pairs[it.q], it.i1 - it.i0, it.c1 - it.c0));
+    for (int k : met[key])
+      c.scr = std::max<long long>(c.scr, grad_item_scratch(h->pairs[qk[k].p], h->pairs[qk[k].q], qk[k].cij, qk[k].ckl));
     c.scr = (c.scr + 31) & ~31LL;  // 256-byte aligned slots
     {  // persistent grid: the CTAs that are resident at once
       GradFn k = grad_kernel_m1(c.nab1, c.ncd1);
@@ -242,7 +305,7 @@ int grad_build(Handle* h, double cutint, GradPlan& plan) {
       c.grid = std::min<long long>((c.count + c.groups - 1) / c.groups, (long long)per_sm * nsm);
     }
     scratch_need = std::max<size_t>(scratch_need, (size_t)c.grid * c.groups * c.scr);
-    plan.items.insert(plan.items.end(), v.begin(), v.end());
+    std::vector<GradItem>().swap(v);
     plan.classes.push_back(c);
   }
   cudaFree(plan.d_items);
