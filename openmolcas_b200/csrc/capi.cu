@@ -57,7 +57,14 @@ ClassPlan eri_plan_for(const Handle* h, int nab, int ncd, const ClassStats& cs, 
     const ClassPlan pl = eri_plan(nab, ncd, cs, kEriThreads, 4);
     if (pl.PAB >= 1) return pl;
   }
-  return eri_plan(nab, ncd, cs, h->eri_tpq[key], h->eri_order[key]);
+  const ClassPlan pl = eri_plan(nab, ncd, cs, h->eri_tpq[key], h->eri_order[key]);
+  // fewer items than groups: no more groups a CTA than there are items for (a
+  // decomposition's classes have some 500 items, and class (0, 0) in groups of 64
+  // threads takes 226 us there: 147 -> 142 ms at 300 functions)
+  const int least = group_threads(count, h->nsm, kEriThreads);
+  if (h->eri_fixed[key] || pl.tpq >= least) return pl;
+  const ClassPlan wide = eri_plan(nab, ncd, cs, least, h->eri_order[key]);
+  return wide.PAB >= 1 ? wide : pl;
 }
 
 // Split quartets into work items grouped by (la+lb, lc+ld) class; a work

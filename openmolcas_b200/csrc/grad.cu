@@ -242,7 +242,9 @@ int grad_build(Handle* h, double cutint, GradPlan& plan) {
       const bool small = nitems <= h->nsm && !h->grad_fixed[key];
       const int order = small ? 3 : h->grad_order[key];
       const int cab = small ? 64 : h->grad_cap[key] ? 32 : 16, ccd = small ? 64 : h->grad_cap[key] ? 16 : 8;
-      const int tpq0 = small ? nthr : h->grad_tpq[key] ? h->grad_tpq[key] : (wmax <= 512 ? 128 : 256);
+      int tpq0 = small ? nthr : h->grad_tpq[key] ? h->grad_tpq[key] : (wmax <= 512 ? 128 : 256);
+      // (nor more groups a CTA than there are items for)
+      if (!h->grad_fixed[key]) tpq0 = std::max(tpq0, group_threads(nitems, h->nsm, nthr));
       // a tile fits when its shared memory is within the group's share and every
       // run-time loop extent x divisor of the kernel stays below 2^32
       auto div_ok = [&](int a, int c, int rw) {

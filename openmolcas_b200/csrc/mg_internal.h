@@ -226,6 +226,14 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs, dou
 int jk_fp64_batch(Handle* h, int k, const double* const* Cs, const int* rs, double* const* Js, double* const* Ks,
                   cudaStream_t st);
 
+// threads of a CTA of nthr that each of `count` items can have when they spread
+// over nsm SMs: nthr over the items per SM, rounded up to a power of two
+inline int group_threads(int count, int nsm, int nthr) {
+  int g = 1;
+  while (g * nsm < count && g < nthr / 64) g *= 2;
+  return nthr / g;
+}
+
 // the next smaller tile extent of n items: one tile more, of equal extents
 inline int tile_shrink(int x, int n) {
   const int k = (n + x - 1) / x + 1;
