@@ -180,6 +180,8 @@ __global__ void k_oz_lexp(const int* __restrict__ inv, int n, int64_t nrs, const
 constexpr int kOzCutRows = 128;  // AOs b per CTA
 constexpr int kOzCutCols = 32;   // AOs a per CTA: one MMA K step
 constexpr int kOzVecs = 4;       // vectors per CTA
+// sliced squares of one launch at most
+constexpr size_t kOzGroupBytes = (size_t)512 << 20;
 
 template <int S>
 __global__ void __launch_bounds__(2 * kOzCutRows) k_oz_slice_l(const int* __restrict__ inv, int n, int64_t nrs,
@@ -287,6 +289,11 @@ __global__ void k_oz_slice_x(const double* __restrict__ X, int64_t xld, int n, i
   const int nch = kblk / 32;
   const int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (o >= (int64_t)ld * nch) return;
+  // block blockIdx.y of a launch
+  X += (size_t)blockIdx.y * kx * xld;
+  xmax += (size_t)blockIdx.y * ld;
+  eX += (size_t)blockIdx.y * ld;
+  col0 += (int64_t)blockIdx.y * kblk;
   const int ri = (int)(o & 127);
   const int64_t r2 = o >> 7;
   const int ch = (int)(r2 % nch), tile = (int)(r2 / nch);
@@ -486,11 +493,23 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
   const int* inv = cho_inv_dev(c, n, st);
   if (!inv) { h->err = "mixed J/K: inverse AO-pair table could not be stored"; return MG_ERR_MEMORY; }
   const size_t nn = (size_t)n * n;
-  const int jsplit = jacc_splits(nrs, nb, nsm);
+  // blocks per launch of the slicing, the half-transform and the Coulomb part: a
+  // power of two (storage blocks of 1024 vectors are not straddled), as many as
+  // keep the sliced squares within 512 MB and X within 256 MB.  One block of 64
+  // vectors is less than two waves of half-transform tiles below 500 functions and
+  // a few microseconds below 150.  Keeping the squares in L2 (128 MB) instead is
+  // slower: 403 functions, two densities 6.66 ms with single blocks, 6.70 with 128
+  // MB, 5.30 with 512; 96 functions 562, 257, 255 us; 168 functions 977, 588, 458 us.
+  int Lg = 1;
+  while (2 * Lg <= 16 && Lg < nblocks && (size_t)2 * Lg * s * nb * ld * ld <= kOzGroupBytes &&
+         (size_t)2 * Lg * 8 * ld * kxmax <= ((size_t)256 << 20))
+    Lg *= 2;
+  const int nbg = nb * Lg;
+  const int jsplit = jacc_splits(nrs, nbg, nsm);
   // one term per take() below (each rounded up to 256 bytes)
-  size_t need = 8 * (size_t)nb * k + (size_t)s * nb * ld * ld + 4 * (size_t)nb * ld + 8 * (size_t)ld * kxmax +
-                8 * (size_t)ld + 8 * (size_t)nsm * 128 * 128 + sizeof(int) +
-                8 * (size_t)(jsplit * (size_t)nrs + vmulti_ranges(nrs) * (size_t)nb) * k + 10 * 256;
+  size_t need = 8 * (size_t)nbg * k + (size_t)s * nbg * ld * ld + 4 * (size_t)nbg * ld + 8 * (size_t)ld * kxmax * Lg +
+                8 * (size_t)ld * Lg + 8 * (size_t)nsm * 128 * 128 + sizeof(int) +
+                8 * (size_t)(jsplit * (size_t)nrs + vmulti_ranges(nrs) * (size_t)nbg) * k + 10 * 256;
   for (const OzDens& q : dd)
     need += 8 * (size_t)nrs + (size_t)s * q.npad * ld + 8 * (size_t)q.npad + (size_t)sk * ld * q.xs_row +
             4 * (size_t)G * ld + 6 * 256;
@@ -498,15 +517,15 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
   if (!ws) { h->err = "jk workspace allocation failed"; return MG_ERR_MEMORY; }
   char* const ws_end = ws + need;
   auto take = [&](size_t bytes) { char* p = ws; ws += (bytes + 255) & ~(size_t)255; return (void*)p; };
-  double* V = (double*)take(8 * (size_t)nb * k);  // V[d nb + J]
-  uint8_t* LS = (uint8_t*)take((size_t)s * nb * ld * ld);
-  int* eA = (int*)take(4 * (size_t)nb * ld);
-  double* Xf = (double*)take(8 * (size_t)ld * kxmax);  // column-major, ld rows
-  unsigned long long* xmax = (unsigned long long*)take(8 * (size_t)ld);
+  double* V = (double*)take(8 * (size_t)nbg * k);  // V[d nbg + J]
+  uint8_t* LS = (uint8_t*)take((size_t)s * nbg * ld * ld);
+  int* eA = (int*)take(4 * (size_t)nbg * ld);
+  double* Xf = (double*)take(8 * (size_t)ld * kxmax * Lg);  // column-major, ld rows
+  unsigned long long* xmax = (unsigned long long*)take(8 * (size_t)ld * Lg);
   double* P = (double*)take(8 * (size_t)nsm * 128 * 128);
   int* d_err = (int*)take(sizeof(int));
   double* jrs_all = (double*)take(8 * (size_t)nrs * k * jsplit);  // jrs of density d at d nrs, per split
-  double* Vp = (double*)take(8 * (size_t)vmulti_ranges(nrs) * nb * k);
+  double* Vp = (double*)take(8 * (size_t)vmulti_ranges(nrs) * nbg * k);
   double* dws = (double*)take(8 * (size_t)nrs * k);      // packed weighted densities
   for (int d = 0; d < k; ++d) {
     OzDens& q = dd[d];
@@ -526,7 +545,7 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
     return false;
   };
   CUtensorMap map_l;
-  if (!make_slice_map(&map_l, LS, ld, (int64_t)nb * ld, s, 128, s)) {
+  if (!make_slice_map(&map_l, LS, ld, (int64_t)nbg * ld, s, 128, s)) {
     h->err = "tensor maps for the exchange GEMMs could not be encoded";
     return MG_ERR_CUDA;
   }
@@ -554,7 +573,7 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
     if (ax.stages < 2 || ak.stages < 2) { h->err = "mixed J/K: slice tiles do not fit in shared memory"; return MG_ERR_ARG; }
     ax.err = ak.err = d_err;
     ax.nrt = ld / 128; ax.nnt = q.nnt; ax.ld = ld; ax.kx = rup(n, kOzCutCols); ax.n = n; ax.r = q.r; ax.eA = eA; ax.fB = q.fC; ax.X = Xf;
-    ax.xld = ld; ax.xmax = xmax;
+    ax.xld = ld; ax.xmax = xmax; ax.jx = nb;
     ak.ld = ld; ak.n = n; ak.ntile = ntile; ak.nsub = q.nsub; ak.kblk = q.kblk; ak.ksub = q.ksub; ak.eX = q.eX;
     ak.P = P; ak.K = q.K;
   }
@@ -582,26 +601,28 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
   }
   for (int g0 = 0; g0 < nblocks; g0 += G) {
     const int gn = std::min(G, nblocks - g0);
-    for (int bi = 0; bi < gn; ++bi) {
+    for (int bi = 0; bi < gn; bi += Lg) {
+      const int bn = std::min(Lg, gn - bi);
       const int J0 = (g0 + bi) * nb;
-      const int nv = std::min(nb, M - J0);
+      const int nv = std::min(bn * nb, M - J0);
       const double* Lb = cho_vec_ptr(c, J0, nv, st, h);
       if (!Lb) { h->err = "vector block straddles storage blocks"; return MG_ERR_ARG; }
       oz_with_slices(s, [&](auto S) {
         k_oz_slice_l<decltype(S)::value>
             <<<dim3(ld / kOzCutRows, (n + kOzCutCols - 1) / kOzCutCols, (nv + kOzVecs - 1) / kOzVecs), 2 * kOzCutRows, 0, st>>>(
-                inv, n, nrs, Lb, nv, ld, (int64_t)nb * ld * ld, eL + (size_t)J0 * ld, LS, eA);
+                inv, n, nrs, Lb, nv, ld, (int64_t)nbg * ld * ld, eL + (size_t)J0 * ld, LS, eA);
       });
       if (!launched("k_oz_slice_l")) return MG_ERR_CUDA;
-      launch_vmulti(Lb, nrs, nv, nb, k, dws, Vp, V, st);
+      launch_vmulti(Lb, nrs, nv, nbg, k, dws, Vp, V, st);
       if (!launched("k_vmulti")) return MG_ERR_CUDA;
-      launch_jacc(Lb, nrs, nv, nb, k, jsplit, V, jrs_all, st);
+      launch_jacc(Lb, nrs, nv, nbg, k, jsplit, V, jrs_all, st);
       if (!launched("k_jacc_multi")) return MG_ERR_CUDA;
       for (OzDens& q : dd) {
         // a short last block: clear the columns of the missing vectors
-        if (nv < nb) cudaMemsetAsync(Xf, 0, 8 * (size_t)ld * q.kx, st);
-        cudaMemsetAsync(xmax, 0, 8 * (size_t)ld, st);
-        // X_J = L_J C for the block (the slice map covers nb vectors; nv <= nb of them are used)
+        if (nv < bn * nb)
+          cudaMemsetAsync(Xf + (size_t)nv * q.r * ld, 0, 8 * (size_t)(bn * nb - nv) * q.r * ld, st);
+        cudaMemsetAsync(xmax, 0, 8 * (size_t)ld * bn, st);
+        // X_J = L_J C for the blocks (the slice map covers nbg vectors; nv <= nbg of them are used)
         OzArgs& ax = q.ax;
         ax.nJ = nv;
         ax.nitems = ax.nrt * nv * q.nnt;
@@ -612,7 +633,7 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
         });
         if (!launched("oz_gemm_kernel<false>")) return MG_ERR_CUDA;
         oz_with_slices(sk, [&](auto S) {
-          k_oz_slice_x<decltype(S)::value><<<nb256((int64_t)ld * (q.kblk / 32)), 256, 0, st>>>(
+          k_oz_slice_x<decltype(S)::value><<<dim3(nb256((int64_t)ld * (q.kblk / 32)), bn), 256, 0, st>>>(
               Xf, ld, n, q.kx, ld, q.kblk, q.xs_row, (int64_t)bi * q.kblk, xmax, q.XS, q.eX + (size_t)bi * ld);
         });
         if (!launched("k_oz_slice_x")) return MG_ERR_CUDA;
@@ -700,7 +721,7 @@ int oz_selftest(Handle* h, int ld, int r, int s, const double* d_A, const double
   if (!attr) return MG_ERR_CUDA;
   ax.err = ak.err = d_err;
   ax.nrt = ld / 128; ax.nnt = nnt; ax.ld = ax.kx = ld; ax.n = ld; ax.r = r; ax.eA = eA; ax.fB = fC; ax.X = d_X; ax.xld = ld;
-  ax.xmax = xmax; ax.nJ = 1; ax.nitems = ax.nrt * nnt;
+  ax.xmax = xmax; ax.jx = 1; ax.nJ = 1; ax.nitems = ax.nrt * nnt;
   ak.ld = ld; ak.n = ld; ak.ntile = (ld / 128) * (ld / 128 + 1) / 2; ak.nsub = nsub; ak.kblk = kblk; ak.ksub = ksub;
   ak.eX = eX; ak.P = P; ak.K = d_K; ak.nblk = 1; ak.nitems = ak.ntile * nsub;
   cudaMemsetAsync(d_err, 0, sizeof(int), st);

@@ -98,7 +98,8 @@ struct OzArgs {
   const double* fB;  // column scale factors of C, 2^f_k
   double* X;       // X[(J * r + k) * xld + a] (FP64, column-major)
   int xld;
-  unsigned long long* xmax;  // per row a: bits of the largest |X| written (atomicMax)
+  unsigned long long* xmax;  // per group of jx vectors and row a: bits of the largest |X| written (atomicMax)
+  int jx;
   // exchange product K += X X^T (SYRK == true): items (lower tile, block, sub-chunk)
   int ntile, nblk, nsub;
   int kblk;        // K extent of one block (multiple of 32)
@@ -382,7 +383,8 @@ __global__ void __launch_bounds__(kOzThreads, 1)
           }
         }
         if (!SYRK && u.last && rmax > 0.0)  // (a single pass: the values written are final)
-          atomicMax(a.xmax + u.t0 * 128 + row, (unsigned long long)__double_as_longlong(rmax));
+          atomicMax(a.xmax + (size_t)(u.J / a.jx) * a.ld + u.t0 * 128 + row,
+                    (unsigned long long)__double_as_longlong(rmax));
         if (SYRK && u.last) {
           // this CTA's share of the tile is complete: add it into K
           const double* pc = a.P + (size_t)blockIdx.x * 128 * 128 + row;
