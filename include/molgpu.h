@@ -153,7 +153,7 @@ int mg_cho_diag(mg_handle* h, double* d_diag, void* stream);
  * with (ab|cd) ~ sum_J L_ab,J L_cd,J.  J, K: nbf x nbf device, overwritten
  * (the reference accumulates into FLT/KLT; mg_cho_lk_scf below does).
  * precision:
- *   MG_PREC_FP64     FP64 vectors, FP64 products (DGEMM/DSYRK);
+ *   MG_PREC_FP64     FP64 vectors, FP64 products;
  *   MG_PREC_MIXED    FP64 vectors cut into 8-bit slices per row (power-of-two
  *                    row scaling): MG_JK_SLICES for the half-transform
  *                    X_J = L_J C, MG_JK_SLICES_K for the exchange product
@@ -291,10 +291,10 @@ int mg_sliced_selftest(mg_handle* h, int ld, int r, int slices, const double* d_
                        double* d_K, void* d_slices, int* d_exps, void* stream);
 
 /* Number of kernels of this library launched so far in this process (library
- * calls such as cuBLAS are not counted).  No reference counterpart. */
+ * calls are not counted).  No reference counterpart. */
 long long mg_kernel_launches(void);
 /* Number of device allocations (cudaMalloc) this library has made so far in
- * this process, all handles together (allocations inside cuBLAS are not
+ * this process, all handles together (allocations inside other libraries are not
  * counted).  No reference counterpart. */
 long long mg_device_allocations(void);
 

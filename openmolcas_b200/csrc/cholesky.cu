@@ -545,6 +545,11 @@ static bool upload_rs(ChoState* c) {
   return true;
 }
 
+static void free_spare(Handle* h) {
+  for (double* p : h->cho_spare) cudaFree(p);
+  h->cho_spare.clear();
+}
+
 // ERI blocks (q4 quartets) into a scratch buffer; offsets per quartet
 static double* eri_blocks(Handle* h, const std::vector<int32_t>& q4, std::vector<int64_t>& off, cudaStream_t st,
                           int& rc) {
@@ -555,7 +560,13 @@ static double* eri_blocks(Handle* h, const std::vector<int32_t>& q4, std::vector
     for (int x = 0; x < 4; ++x) n *= (int64_t)h->sh[q4[4 * t + x]].nc * h->sh[q4[4 * t + x]].ncomp;
     off[t + 1] = off[t] + n;
   }
-  double* buf = (double*)keep_get(h->cho_buf, sizeof(double) * std::max<int64_t>(off[nq], 1), st);
+  const size_t need = sizeof(double) * std::max<int64_t>(off[nq], 1);
+  double* buf = (double*)keep_get(h->cho_buf, need, st);
+  if (!buf && !h->cho_spare.empty()) {  // the replaced vectors give way
+    cudaGetLastError();
+    free_spare(h);
+    buf = (double*)keep_get(h->cho_buf, need, st);
+  }
   if (!buf) { rc = MG_ERR_MEMORY; return nullptr; }
   std::vector<EriItem> items;
   std::vector<EriClass> classes;
@@ -708,8 +719,7 @@ int cho_decompose(Handle* h, const ChoCfgH& cfg, ChoState*& out, cudaStream_t st
           cudaFree(w->ptr);
           *w = Workspace{};
         }
-      for (double* p : h->cho_spare) cudaFree(p);
-      h->cho_spare.clear();
+      free_spare(h);
     }
   } give_back{h};
   int rc = 0;
@@ -759,10 +769,7 @@ int cho_decompose(Handle* h, const ChoCfgH& cfg, ChoState*& out, cudaStream_t st
   }
   const int64_t nrs = c->nrs;
   const size_t blk_bytes = sizeof(double) * (size_t)nrs * kVecBlock;
-  if (h->cho_spare_bytes != blk_bytes) {  // storage of the previous vectors, usable for the same list only
-    for (double* p : h->cho_spare) cudaFree(p);
-    h->cho_spare.clear();
-  }
+  if (h->cho_spare_bytes != blk_bytes) free_spare(h);  // the previous vectors' storage fits the same list only
   ChoItemPlan plan;
   make_item_plan(h, c, plan);
   int maxcnt = 1;
