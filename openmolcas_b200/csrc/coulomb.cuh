@@ -58,7 +58,8 @@ __device__ __forceinline__ double warp_sum(double v) {
 // the four vectors and the grid covers the chip also for a block of 64 vectors.
 // (One CTA per vector, its predecessor, left half of the SMs idle and each of
 // the others with a single stream of loads: 193 us per block of 64 vectors at
-// 403 functions with one further density; 8 us this way.)  The partial sums of
+// 403 functions with one further density; 8 us this way.  Eight vectors per CTA:
+// 5.3 instead of 3.9 ms a call at 1250 functions, one density.)  The partial sums of
 // the row ranges go to Vp[range][KD nb] and are added in order by k_vsum, so the
 // result does not depend on the order in which the CTAs run.
 template <int KD>
