@@ -367,8 +367,9 @@ __global__ void __launch_bounds__(kOzThreads, 1)
                 if (k < a.r) {
                   const double val = sum[i] * fa * a.fB[k];
                   double* xp = xc + (size_t)k * a.xld;
-                  *xp = u.first ? val : *xp + val;
-                  rmax = fmax(rmax, fabs(val));
+                  const double x = u.first ? val : *xp + val;
+                  *xp = x;
+                  rmax = fmax(rmax, fabs(x));
                 }
               }
             }
@@ -382,7 +383,7 @@ __global__ void __launch_bounds__(kOzThreads, 1)
             }
           }
         }
-        if (!SYRK && u.last && rmax > 0.0)  // (a single pass: the values written are final)
+        if (!SYRK && u.last && rmax > 0.0)  // (the last K chunk's unit writes the final values)
           atomicMax(a.xmax + (size_t)(u.J / a.jx) * a.ld + u.t0 * 128 + row,
                     (unsigned long long)__double_as_longlong(rmax));
         if (SYRK && u.last) {
