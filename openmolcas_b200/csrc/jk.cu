@@ -50,6 +50,18 @@ __global__ void k_fock_acc(double* __restrict__ F, const double* __restrict__ J,
   if (t < n) F[t] += J[t] - factxi * K[t];
 }
 
+// J = K = 0 of a decomposition without vectors (the threshold above the largest
+// diagonal: possibly without rows, too)
+int jk_no_vectors(Handle* h, int k, double* const* Js, double* const* Ks, cudaStream_t st) {
+  const size_t bytes = sizeof(double) * (size_t)h->nbf * h->nbf;
+  for (int d = 0; d < k; ++d)
+    if (cudaMemsetAsync(Js[d], 0, bytes, st) != cudaSuccess || cudaMemsetAsync(Ks[d], 0, bytes, st) != cudaSuccess) {
+      h->err = std::string("J/K: clearing the outputs: ") + cudaGetErrorString(cudaGetLastError());
+      return MG_ERR_CUDA;
+    }
+  return 0;
+}
+
 int fock_accumulate(double* F, const double* J, const double* K, double factxi, int64_t n, cudaStream_t st) {
   k_fock_acc<<<nb256(n), 256, 0, st>>>(F, J, K, factxi, n);
   g_launches.fetch_add(1, std::memory_order_relaxed);
@@ -459,6 +471,12 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
     h->err = std::string("mixed J/K: error pending from earlier work: ") + cudaGetErrorString(e);
     return MG_ERR_CUDA;
   }
+  for (int d = 0; d < k; ++d)
+    if (!Cs[d] || !Js[d] || !Ks[d] || rs_[d] < 1) {
+      h->err = "mixed J/K: a density of the batch has no factor or outputs";
+      return MG_ERR_ARG;
+    }
+  if (M == 0) return jk_no_vectors(h, k, Js, Ks, st);
   const int ld = rup(n, 128);
   // vectors per block: one block's K extent of the exchange product, nb r
   const int nb = std::min(block, M);
@@ -473,10 +491,6 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
     q.r = rs_[d];
     q.J = Js[d];
     q.K = Ks[d];
-    if (!q.C || !q.J || !q.K || q.r < 1) {
-      h->err = "mixed J/K: a density of the batch has no factor or outputs";
-      return MG_ERR_ARG;
-    }
     oz_col_tiles(q.r, s, q.nnt, q.Nt);
     q.npad = q.nnt * q.Nt;
     q.kx = nb * q.r;

@@ -247,6 +247,7 @@ int jk_fp64_batch(Handle* h, int k, const double* const* Cs, const int* rs_, dou
     if (!Cs[d] || !Js[d] || !Ks[d] || rs_[d] < 1) { h->err = "FP64 J/K: a density of the batch has no factor or outputs"; return MG_ERR_ARG; }
     rmax = std::max(rmax, rs_[d]);
   }
+  if (M == 0) return jk_no_vectors(h, k, Js, Ks, st);
   const int* inv = cho_inv_dev(c, n, st);
   if (!inv) { h->err = "FP64 J/K: inverse AO-pair table could not be stored"; return MG_ERR_MEMORY; }
   int nsm = 148;
@@ -260,7 +261,7 @@ int jk_fp64_batch(Handle* h, int k, const double* const* Cs, const int* rs_, dou
   int nb = 1024;
   while (nb > 16 && (size_t)nb * rmax * xld * 8 > ((size_t)256 << 20)) nb /= 2;
   nb = std::min(nb, cho_vec_block());
-  const int nbm = std::min(nb, std::max(M, 1));  // vectors X holds
+  const int nbm = std::min(nb, M);  // vectors X holds
   const int nt = xld / bt, ntile = nt * (nt + 1) / 2;
   // K splits of a full block of rank r: a few CTAs per SM in all, at least 8 chunks each
   auto splits = [&](int r, int& cps) {

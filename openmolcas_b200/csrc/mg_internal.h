@@ -218,6 +218,7 @@ int oz_selftest(Handle* h, int ld, int r, int s, const double* d_A, const double
 // (0, 101, 102, -1) or MG_ERR_*; X (n x n, column-major) is overwritten.
 int cd_incore(Handle* h, double* d_X, int n, double thr, double* d_vec, int maxvec, int* numcho, cudaStream_t st);
 int fock_accumulate(double* F, const double* J, const double* K, double factxi, int64_t n, cudaStream_t st);
+int jk_no_vectors(Handle* h, int k, double* const* Js, double* const* Ks, cudaStream_t st);
 int jk_fp64(Handle* h, const double* d_C, int r, double* d_J, double* d_K, cudaStream_t st);
 int jk_mixed(Handle* h, const double* d_C, int r, double* d_J, double* d_K, cudaStream_t st, int block, int s, int sk);
 // J/K of k (1..8) densities over one pass of the vectors (jk.cu)
