@@ -524,6 +524,10 @@ int mg_cho_drv(mg_handle* H, const mg_cho_cfg* cfg, void* stream) {
   c.maxvec = cfg->maxvec > 0 ? cfg->maxvec : h->nbf * (h->nbf + 1) / 2;
   ChoState* st = nullptr;
   int rc = cho_decompose(h, c, st, (cudaStream_t)stream, h->err);
+  if (rc && cho_nvec(st) == 0) {  // failed before its first vector: nothing that a later call could use
+    cho_free(st);
+    st = nullptr;
+  }
   h->cho = st;
   return rc;
 }

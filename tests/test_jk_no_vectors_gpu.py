@@ -1,12 +1,13 @@
 """J/K over a decomposition without vectors: a threshold above the largest
 diagonal (the reduced set is empty after the first look) and one so large that
 the initial screening leaves no AO pair at all.  Both precisions give zeros and
-add nothing to a Fock matrix."""
+add nothing to a Fock matrix; a decomposition that fails before its first vector
+leaves none behind."""
 import pytest
 import torch
 
 from openmolcas_b200 import basis as B
-from openmolcas_b200.molgpu import MolGpu
+from openmolcas_b200.molgpu import MolGpu, MolGpuError
 
 pytestmark = pytest.mark.gpu
 
@@ -30,3 +31,14 @@ def test_zero_vectors_give_zero_matrices(g, factor, precision):
     F0 = F.clone()
     g.choscf_lk(Cs[1] @ Cs[1].t(), 0.5, F, precision=precision)
     assert torch.equal(F, F0)
+
+
+def test_failed_decomposition_without_vectors_is_dropped(g):
+    g.cho_drv(thrcom=1e-6)
+    with pytest.raises(MolGpuError, match="rc=2"):
+        g.cho_drv(thrcom=1e-6, maxvec=1, maxqual=100)
+    C = torch.from_numpy(B.density_factor(g.nbf, 3, 3)).cuda()
+    with pytest.raises(MolGpuError, match="no Cholesky vectors"):
+        g.cho_jk(C)
+    g.cho_drv(thrcom=1e-6)
+    assert g.cho_jk(C)[1].any()
