@@ -297,6 +297,12 @@ long long mg_kernel_launches(void);
  * this process, all handles together (allocations inside other libraries are not
  * counted).  No reference counterpart. */
 long long mg_device_allocations(void);
+/* For tests of what happens when device memory is short: of the calling
+ * thread's next device allocations in this library, the first `skip` proceed
+ * and the `count` after them fail (cudaMalloc is asked for more than there is).
+ * Returns how many of the previous call's failures were still to come; (0, 0)
+ * ends it. */
+int mg_test_fail_allocations(int skip, int count);
 
 #ifdef __cplusplus
 }

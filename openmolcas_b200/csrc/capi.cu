@@ -18,6 +18,7 @@ struct mg_handle {
 namespace mg {
 std::atomic<long long> g_launches{0};
 std::atomic<long long> g_allocs{0};
+thread_local int t_alloc_skip = 0, t_alloc_fail = 0;
 
 // Accumulator budget (doubles) of one work item: nc * nef <= this.
 static const int kAccBudget = 12288;
@@ -696,6 +697,12 @@ int mg_sliced_selftest(mg_handle* H, int ld, int r, int slices, const double* d_
 
 long long mg_kernel_launches(void) { return g_launches.load(); }
 long long mg_device_allocations(void) { return g_allocs.load(); }
+int mg_test_fail_allocations(int skip, int count) {
+  const int left = t_alloc_fail;
+  t_alloc_skip = skip;
+  t_alloc_fail = count;
+  return left;
+}
 
 int mg_rys_roots(mg_handle* H, int nrys, int64_t n, const double* T, double* x, double* w) {
   if (!H || nrys < 1 || nrys > MG_MAX_RYS || n < 0 || (n && (!T || !x || !w))) return MG_ERR_ARG;

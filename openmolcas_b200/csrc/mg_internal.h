@@ -20,11 +20,25 @@ extern std::atomic<long long> g_launches;
 // number of device allocations this library has requested so far (all handles)
 extern std::atomic<long long> g_allocs;
 
-// Every device allocation of the library goes through here (counted).
+// allocations of this thread to let through, and then to make fail (mg_test_fail_allocations)
+extern thread_local int t_alloc_skip, t_alloc_fail;
+
+// Every device allocation of the library goes through here (counted).  The
+// caller gets a failure as the return value; it does not stay behind as the
+// runtime's last error, where the check of a later launch would find it.
 template <typename T>
 inline cudaError_t dev_malloc(T** p, size_t bytes) {
   g_allocs.fetch_add(1, std::memory_order_relaxed);
-  return cudaMalloc((void**)p, bytes);
+  if (t_alloc_fail > 0 && t_alloc_skip-- <= 0) {
+    --t_alloc_fail;
+    bytes = ~(size_t)0 >> 2;  // more than any device holds
+  }
+  const cudaError_t e = cudaMalloc((void**)p, bytes);
+  if (e != cudaSuccess) {
+    *p = nullptr;
+    cudaGetLastError();
+  }
+  return e;
 }
 
 // Per-order metadata of the Rys root/weight table (constant memory).
