@@ -284,10 +284,10 @@ int setup_pairs(Handle* h) {
   for (size_t i = 0; i < zeta.size(); ++i) izeta[i] = 1.0 / zeta[i];
   std::vector<double> prim;
   for (auto* v : {&zeta, &kappa, &px, &py, &pz, &al, &be, &izeta}) prim.insert(prim.end(), v->begin(), v->end());
-  if (dev_malloc(&h->d_prim, sizeof(double) * prim.size()) != cudaSuccess ||
-      dev_malloc(&h->d_coef, sizeof(double) * std::max<size_t>(coef.size(), 1)) != cudaSuccess ||
-      dev_malloc(&h->d_hrr, sizeof(double) * std::max<size_t>(hrr.size(), 1)) != cudaSuccess ||
-      dev_malloc(&h->d_pairs, sizeof(DPair) * h->pairs.size()) != cudaSuccess) {
+  if (dev_malloc(h, &h->d_prim, sizeof(double) * prim.size()) != cudaSuccess ||
+      dev_malloc(h, &h->d_coef, sizeof(double) * std::max<size_t>(coef.size(), 1)) != cudaSuccess ||
+      dev_malloc(h, &h->d_hrr, sizeof(double) * std::max<size_t>(hrr.size(), 1)) != cudaSuccess ||
+      dev_malloc(h, &h->d_pairs, sizeof(DPair) * h->pairs.size()) != cudaSuccess) {
     h->err = "cudaMalloc pair data";
     return 1;
   }
@@ -298,7 +298,17 @@ int setup_pairs(Handle* h) {
   return 0;
 }
 
-void* keep_get(Workspace& w, size_t bytes, cudaStream_t st) {
+void give_back(Handle* h) {
+  for (double* p : h->cho_spare) cudaFree(p);
+  h->cho_spare.clear();
+  if (h->cho_running) return;
+  for (Workspace* w : {&h->cho_scr, &h->cho_buf, &h->cho_lq, &h->cho_upd}) {
+    cudaFree(w->ptr);
+    *w = Workspace{};
+  }
+}
+
+void* keep_get(Handle* h, Workspace& w, size_t bytes, cudaStream_t st) {
   if (bytes <= w.size) return w.ptr;
   if (w.ptr) {
     cudaStreamSynchronize(st);
@@ -306,12 +316,12 @@ void* keep_get(Workspace& w, size_t bytes, cudaStream_t st) {
   }
   w = Workspace{};
   const size_t sz = std::max(bytes, (size_t)1 << 20);
-  if (dev_malloc(&w.ptr, sz) != cudaSuccess) return nullptr;
+  if (dev_malloc(h, &w.ptr, sz) != cudaSuccess) return nullptr;
   w.size = sz;
   return w.ptr;
 }
 
-void* ws_get(Handle* h, size_t bytes, cudaStream_t st) { return keep_get(h->ws, bytes, st); }
+void* ws_get(Handle* h, size_t bytes, cudaStream_t st) { return keep_get(h, h->ws, bytes, st); }
 
 void* pin_get(Handle* h, size_t bytes) {
   if (bytes <= h->pin.size) return h->pin.ptr;

@@ -421,7 +421,7 @@ int mg_twoel_nosym(mg_handle* H, const double* coor, int* noints, double* wrk, i
   rc = build_eri_items(h, q, 1, off, items, classes);
   if (rc) return rc;
   double* blk = nullptr;
-  if (dev_malloc(&blk, sizeof(double) * nout) != cudaSuccess) { h->err = "mg_twoel_nosym: allocation failed"; return MG_ERR_MEMORY; }
+  if (dev_malloc(h, &blk, sizeof(double) * nout) != cudaSuccess) { h->err = "mg_twoel_nosym: allocation failed"; return MG_ERR_MEMORY; }
   rc = run_eri_items(h, items, classes, blk, nullptr);
   std::vector<double> hb(nout);
   if (!rc && cudaMemcpy(hb.data(), blk, sizeof(double) * nout, cudaMemcpyDeviceToHost) != cudaSuccess) rc = MG_ERR_CUDA;
@@ -468,7 +468,7 @@ int mg_schwarz(mg_handle* H, double* tmax) {
     std::vector<int64_t> off(nq + 1);
     mg_eri_quartets_size(H, q.data(), nq, off.data());
     double* d_out = nullptr;
-    if (dev_malloc(&d_out, sizeof(double) * std::max<int64_t>(off[nq], 1)) != cudaSuccess) {
+    if (dev_malloc(h, &d_out, sizeof(double) * std::max<int64_t>(off[nq], 1)) != cudaSuccess) {
       h->err = "cudaMalloc Schwarz";
       return MG_ERR_MEMORY;
     }
@@ -630,7 +630,7 @@ int mg_cho_lk_scf(mg_handle* H, const double* d_C, int r, double factxi, double*
     cudaFree(h->d_lk);
     h->d_lk = nullptr;
     h->lk_cap = 0;
-    if (dev_malloc(&h->d_lk, 2 * nn * sizeof(double)) != cudaSuccess) {
+    if (dev_malloc(h, &h->d_lk, 2 * nn * sizeof(double)) != cudaSuccess) {
       h->err = "mg_cho_lk_scf: allocation failed";
       return MG_ERR_MEMORY;
     }
@@ -661,7 +661,7 @@ int mg_choscf_lk(mg_handle* H, const double* d_D, double factxi, double* d_FLT, 
     cudaFree(h->d_dcd);
     h->d_dcd = nullptr;
     h->dcd_cap = 0;
-    if (dev_malloc(&h->d_dcd, 2 * nn * sizeof(double)) != cudaSuccess) {
+    if (dev_malloc(h, &h->d_dcd, 2 * nn * sizeof(double)) != cudaSuccess) {
       h->err = "mg_choscf_lk: allocation failed";
       return MG_ERR_MEMORY;
     }
@@ -716,7 +716,7 @@ int mg_rys_roots(mg_handle* H, int nrys, int64_t n, const double* T, double* x, 
   if (cudaSetDevice(h->device) != cudaSuccess) return MG_ERR_CUDA;
   double* d = nullptr;
   const size_t bytes = sizeof(double) * (size_t)n * (1 + 2 * nrys);
-  if (dev_malloc(&d, bytes) != cudaSuccess) {
+  if (dev_malloc(h, &d, bytes) != cudaSuccess) {
     h->err = "mg_rys_roots: device allocation failed";
     return MG_ERR_MEMORY;
   }

@@ -520,14 +520,14 @@ static void make_rs(Handle* h, ChoState* c, const std::vector<char>* keep = null
 }
 
 // The state's device tables, in one allocation; the rs list goes up.
-static bool upload_rs(ChoState* c) {
+static bool upload_rs(Handle* h, ChoState* c) {
   const size_t n = std::max<int64_t>(c->nrs, 1), nsp = c->sp_first.size();
   size_t need = 0;
   auto place = [&](size_t bytes) { const size_t o = need; need += (bytes + 255) & ~(size_t)255; return o; };
   const size_t o_rs = place(sizeof(RsDev) * n), o_a = place(sizeof(int) * n), o_b = place(sizeof(int) * n),
                o_f = place(sizeof(int64_t) * nsp), o_c = place(sizeof(int) * nsp), o_d = place(sizeof(double) * n),
                o_d0 = place(sizeof(double) * n), o_in = place(n);
-  if (dev_malloc(&c->d_tab, need) != cudaSuccess) return false;
+  if (dev_malloc(h, &c->d_tab, need) != cudaSuccess) return false;
   c->d_rs = (RsDev*)(c->d_tab + o_rs);
   c->d_rs_a = (int*)(c->d_tab + o_a);
   c->d_rs_b = (int*)(c->d_tab + o_b);
@@ -545,11 +545,6 @@ static bool upload_rs(ChoState* c) {
   return true;
 }
 
-static void free_spare(Handle* h) {
-  for (double* p : h->cho_spare) cudaFree(p);
-  h->cho_spare.clear();
-}
-
 // ERI blocks (q4 quartets) into a scratch buffer; offsets per quartet
 static double* eri_blocks(Handle* h, const std::vector<int32_t>& q4, std::vector<int64_t>& off, cudaStream_t st,
                           int& rc) {
@@ -561,12 +556,7 @@ static double* eri_blocks(Handle* h, const std::vector<int32_t>& q4, std::vector
     off[t + 1] = off[t] + n;
   }
   const size_t need = sizeof(double) * std::max<int64_t>(off[nq], 1);
-  double* buf = (double*)keep_get(h->cho_buf, need, st);
-  if (!buf && !h->cho_spare.empty()) {  // the replaced vectors give way
-    cudaGetLastError();
-    free_spare(h);
-    buf = (double*)keep_get(h->cho_buf, need, st);
-  }
+  double* buf = (double*)keep_get(h, h->cho_buf, need, st);
   if (!buf) { rc = MG_ERR_MEMORY; return nullptr; }
   std::vector<EriItem> items;
   std::vector<EriClass> classes;
@@ -711,17 +701,19 @@ int cho_decompose(Handle* h, const ChoCfgH& cfg, ChoState*& out, cudaStream_t st
   const int nsp = c->sp_count.size();
   const double damp = cho_default_damp(cfg.thrcom);
   // the handle's buffers, kept for the next decomposition unless they are large
-  struct GiveBack {
+  struct Running {
     Handle* h;
-    ~GiveBack() {
+    explicit Running(Handle* hh) : h(hh) { h->cho_running = true; }
+    ~Running() {
       for (Workspace* w : {&h->cho_scr, &h->cho_buf, &h->cho_lq, &h->cho_upd})
         if (w->size > kKeepBytes) {
           cudaFree(w->ptr);
           *w = Workspace{};
         }
-      free_spare(h);
+      give_back(h);  // the replaced vectors' storage that was not used
+      h->cho_running = false;
     }
-  } give_back{h};
+  } running(h);
   int rc = 0;
   // ---- diagonal (CHO_GETDIAG): (AB|AB) for every shell pair, then the initial
   // screening (cho_calcdiag.F90:255-300): elements below
@@ -740,7 +732,7 @@ int cho_decompose(Handle* h, const ChoCfgH& cfg, ChoState*& out, cudaStream_t st
     if (rc) { err = "diagonal integrals failed: " + err; return rc; }
     // full diagonal, every shell pair
     const size_t rs_bytes = (sizeof(RsDev) * c->nrs + 255) & ~(size_t)255;
-    char* d = (char*)keep_get(h->cho_scr, rs_bytes + sizeof(int64_t) * nsp + sizeof(double) * c->nrs, st);
+    char* d = (char*)keep_get(h, h->cho_scr, rs_bytes + sizeof(int64_t) * nsp + sizeof(double) * c->nrs, st);
     if (!d) { err = "diagonal: out of device memory"; return MG_ERR_MEMORY; }
     RsDev* d_rs = (RsDev*)d;
     int64_t* d_off = (int64_t*)(d + rs_bytes);
@@ -760,7 +752,7 @@ int cho_decompose(Handle* h, const ChoCfgH& cfg, ChoState*& out, cudaStream_t st
       if (!(hd[t] < scrmax)) keep[c->rs_sp[t]] = 1;
     make_rs(h, c, &keep);
     // the diagonal over the kept shell pairs, from the same integral blocks
-    if (!upload_rs(c)) { err = "diagonal: out of device memory"; return MG_ERR_MEMORY; }
+    if (!upload_rs(h, c)) { err = "diagonal: out of device memory"; return MG_ERR_MEMORY; }
     k_extract_diag<<<nblk(std::max<int64_t>(c->nrs, 1)), 256, 0, st>>>(c->d_rs, c->nrs, h->d_pairs, d_off, buf,
                                                                         c->d_diag0);
     g_launches.fetch_add(1, std::memory_order_relaxed);
@@ -769,7 +761,7 @@ int cho_decompose(Handle* h, const ChoCfgH& cfg, ChoState*& out, cudaStream_t st
   }
   const int64_t nrs = c->nrs;
   const size_t blk_bytes = sizeof(double) * (size_t)nrs * kVecBlock;
-  if (h->cho_spare_bytes != blk_bytes) free_spare(h);  // the previous vectors' storage fits the same list only
+  if (h->cho_spare_bytes != blk_bytes) give_back(h);  // the previous vectors' storage fits the same list only
   ChoItemPlan plan;
   make_item_plan(h, c, plan);
   int maxcnt = 1;
@@ -788,11 +780,11 @@ int cho_decompose(Handle* h, const ChoCfgH& cfg, ChoState*& out, cudaStream_t st
                o_base = place(sizeof(int64_t) * nsp), o_lt = place(sizeof(double*) * maxblk), o_xm = place(16),
                o_cols = place(sizeof(int) * MQ), o_q = place(sizeof(double) * MQ * MQ),
                o_part = place(sizeof(double) * MQ * MQ * kParts);
-  char* scr = (char*)keep_get(h->cho_scr, need, st);
+  char* scr = (char*)keep_get(h, h->cho_scr, need, st);
   // partial sums of the update kernels
   const int nrow = (int)((nrs + kUpdRows - 1) / kUpdRows);
   const size_t upd = sizeof(double) * std::max<size_t>(1, 6 * h->nsm / std::max(nrow, 1)) * std::min(32, MQ) * std::max<int64_t>(nrs, 1);
-  double* d_upd = (double*)keep_get(h->cho_upd, upd, st);
+  double* d_upd = (double*)keep_get(h, h->cho_upd, upd, st);
   if (!scr || !d_upd) { err = "out of device memory for the passes' scratch"; return MG_ERR_MEMORY; }
   ChoSel* d_sel = (ChoSel*)(scr + o_sel);
   double* d_dpair = (double*)(d_sel + 1);
@@ -851,7 +843,7 @@ int cho_decompose(Handle* h, const ChoCfgH& cfg, ChoState*& out, cudaStream_t st
     // ---- integral columns (CD|AB) for every CD pair touching the reduced set
     const DPair& A = h->pairs[spab];
     const int64_t ksz = (int64_t)A.nci * A.ncj * A.nsa * A.nsb;
-    double* buf = (double*)keep_get(h->cho_buf, sizeof(double) * std::max<int64_t>(plan.total * ksz, 1), st);
+    double* buf = (double*)keep_get(h, h->cho_buf, sizeof(double) * std::max<int64_t>(plan.total * ksz, 1), st);
     if (!buf) { rc = MG_ERR_MEMORY; err = "column integrals failed: out of device memory"; break; }
     rc = pass_items(h, plan, halive, spab, items, classes);
     if (!rc) rc = run_eri_items(h, items, classes, buf, st);
@@ -860,7 +852,7 @@ int cho_decompose(Handle* h, const ChoCfgH& cfg, ChoState*& out, cudaStream_t st
     const int M = c->M;
     double* d_lq = (double*)h->cho_lq.ptr;
     if (h->cho_lq.size < sizeof(double) * (size_t)nq * (M + nq)) {  // grows with the vectors
-      d_lq = (double*)keep_get(h->cho_lq, sizeof(double) * (size_t)MQ * (M + kVecBlock + MQ), st);
+      d_lq = (double*)keep_get(h, h->cho_lq, sizeof(double) * (size_t)MQ * (M + kVecBlock + MQ), st);
       if (!d_lq) { rc = MG_ERR_MEMORY; err = "out of device memory for the LQ rows"; break; }
     }
     cudaMemcpyAsync(d_cols, qual.data(), sizeof(int) * nq, cudaMemcpyHostToDevice, st);
@@ -904,7 +896,7 @@ int cho_decompose(Handle* h, const ChoCfgH& cfg, ChoState*& out, cudaStream_t st
       if (!h->cho_spare.empty()) {
         p = h->cho_spare.back();
         h->cho_spare.pop_back();
-      } else if (dev_malloc(&p, blk_bytes) != cudaSuccess) {
+      } else if (dev_malloc(h, &p, blk_bytes) != cudaSuccess) {
         rc = MG_ERR_MEMORY;
         break;
       }
@@ -986,11 +978,11 @@ __global__ void k_rs_inverse(const int* __restrict__ rs_a, const int* __restrict
   inv[(size_t)b * n + a] = (int)t;
 }
 
-const int* cho_inv_dev(ChoState* c, int n, cudaStream_t st) {
+const int* cho_inv_dev(Handle* h, ChoState* c, int n, cudaStream_t st) {
   if (c->d_inv) return c->d_inv;
   int* p = nullptr;
   const size_t bytes = sizeof(int) * (size_t)n * n;
-  if (dev_malloc(&p, bytes) != cudaSuccess) return nullptr;
+  if (dev_malloc(h, &p, bytes) != cudaSuccess) return nullptr;
   cudaMemsetAsync(p, 0xFF, bytes, st);
   k_rs_inverse<<<nblk(std::max<int64_t>(c->nrs, 1)), 256, 0, st>>>(c->d_rs_a, c->d_rs_b, c->nrs, n, p);
   g_launches.fetch_add(1, std::memory_order_relaxed);

@@ -31,7 +31,7 @@
 namespace mg {
 
 // Device copy of the per-CTA tables (layout in grad_kernel.cuh).
-static int make_grad_tables(const Handle* h, double** d_tab) {
+static int make_grad_tables(Handle* h, double** d_tab) {
   std::vector<double> t(kGTabD, 0.0);
   int o = kGTabSph;
   for (int l = 0; l <= 3; ++l)
@@ -42,7 +42,7 @@ static int make_grad_tables(const Handle* h, double** d_tab) {
   for (int l = 0; l <= 7; ++l)
     for (int lx = l; lx >= 0; --lx)
       for (int ly = l - lx; ly >= 0; --ly) cart[k++] = lx | (ly << 8) | ((l - lx - ly) << 16);
-  if (dev_malloc(d_tab, sizeof(double) * kGTabD) != cudaSuccess) return MG_ERR_MEMORY;
+  if (dev_malloc(h, d_tab, sizeof(double) * kGTabD) != cudaSuccess) return MG_ERR_MEMORY;
   cudaMemcpy(*d_tab, t.data(), sizeof(double) * kGTabD, cudaMemcpyHostToDevice);
   return 0;
 }
@@ -313,7 +313,7 @@ int grad_build(Handle* h, double cutint, GradPlan& plan) {
   cudaFree(plan.d_items);
   plan.d_items = nullptr;
   if (!plan.items.empty()) {
-    if (dev_malloc(&plan.d_items, sizeof(GradItem) * plan.items.size()) != cudaSuccess) return MG_ERR_MEMORY;
+    if (dev_malloc(h, &plan.d_items, sizeof(GradItem) * plan.items.size()) != cudaSuccess) return MG_ERR_MEMORY;
     cudaMemcpy(plan.d_items, plan.items.data(), sizeof(GradItem) * plan.items.size(), cudaMemcpyHostToDevice);
   }
   cudaFree(plan.d_scratch);
@@ -323,8 +323,8 @@ int grad_build(Handle* h, double cutint, GradPlan& plan) {
   // one scratch region per side stream: class kernels on different streams run concurrently
   plan.scratch_stride = (std::max<size_t>(scratch_need, 32) + 31) & ~(size_t)31;
   plan.nstreams = std::max<int>(1, std::min<int>(MG_ERI_STREAMS, (int)plan.classes.size()));
-  if (dev_malloc(&plan.d_scratch, sizeof(double) * plan.scratch_stride * plan.nstreams) != cudaSuccess ||
-      dev_malloc(&plan.d_counters, sizeof(int) * std::max<size_t>(plan.classes.size(), 1)) != cudaSuccess) {
+  if (dev_malloc(h, &plan.d_scratch, sizeof(double) * plan.scratch_stride * plan.nstreams) != cudaSuccess ||
+      dev_malloc(h, &plan.d_counters, sizeof(int) * std::max<size_t>(plan.classes.size(), 1)) != cudaSuccess) {
     h->err = "gradient scratch allocation failed";
     return MG_ERR_MEMORY;
   }

@@ -410,7 +410,7 @@ static const short* oz_row_exponents(Handle* h, const int* inv, int ld, cudaStre
   const int M = cho_nvec(c), n = h->nbf, vb = cho_vec_block();
   const int64_t nrs = cho_nrs(c);
   short* e = nullptr;
-  if (dev_malloc(&e, sizeof(short) * (size_t)M * ld) != cudaSuccess) return nullptr;
+  if (dev_malloc(h, &e, sizeof(short) * (size_t)M * ld) != cudaSuccess) return nullptr;
   for (int J0 = 0; J0 < M; J0 += vb) {
     const int nv = std::min(vb, M - J0);
     const double* L = cho_vec_ptr(c, J0, nv, st, h);
@@ -504,7 +504,7 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
   const int* d_ra = cho_rs_a_dev(c);
   const int* d_rb = cho_rs_b_dev(c);
-  const int* inv = cho_inv_dev(c, n, st);
+  const int* inv = cho_inv_dev(h, c, n, st);
   if (!inv) { h->err = "mixed J/K: inverse AO-pair table could not be stored"; return MG_ERR_MEMORY; }
   const size_t nn = (size_t)n * n;
   // blocks per launch of the slicing, the half-transform and the Coulomb part: a

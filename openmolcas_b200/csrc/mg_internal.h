@@ -132,6 +132,7 @@ struct Handle {
   Workspace cho_scr, cho_buf, cho_lq, cho_upd;
   std::vector<double*> cho_spare;
   size_t cho_spare_bytes = 0;
+  bool cho_running = false;   // a decomposition is using the buffers
   std::string err;
   struct ChoState* cho = nullptr;  // Cholesky vectors of the current basis
   struct GradPlan* grad = nullptr; // gradient work list (per Schwarz threshold)
@@ -222,7 +223,7 @@ const double* cho_vec_ptr(const ChoState* c, int J0, int nb, cudaStream_t st, Ha
 int cho_vec_block();
 // rs index of every AO pair (n x n device table, -1 where no row is stored),
 // built on first use and owned by the state; nullptr when it cannot be stored
-const int* cho_inv_dev(ChoState* c, int n, cudaStream_t st);
+const int* cho_inv_dev(Handle* h, ChoState* c, int n, cudaStream_t st);
 // cached row exponents of the square Cholesky vectors (M x ld), owned by the state
 short* cho_lexp(const ChoState* c, int ld);
 void cho_set_lexp(ChoState* c, short* p, int ld);
@@ -266,9 +267,20 @@ void build_sph(Handle* h, int lmax);
 std::vector<double> hrr_matrix(const Handle* h, int la, int lb, const double* A, const double* B, int& ne, int& emin);
 int setup_pairs(Handle* h);
 void* ws_get(Handle* h, size_t bytes, cudaStream_t st);
+// Frees what the handle only keeps for a later call: the storage of replaced
+// vectors and, outside a decomposition, the decomposition's buffers.
+void give_back(Handle* h);
+// dev_malloc for a call on this handle: what the handle keeps gives way when
+// memory is short
+template <typename T>
+inline cudaError_t dev_malloc(Handle* h, T** p, size_t bytes) {
+  if (dev_malloc(p, bytes) == cudaSuccess) return cudaSuccess;
+  give_back(h);
+  return dev_malloc(p, bytes);
+}
 // device memory of one of the handle's workspaces, grown when too small (after
 // waiting for the stream); nullptr when it cannot be had
-void* keep_get(Workspace& w, size_t bytes, cudaStream_t st);
+void* keep_get(Handle* h, Workspace& w, size_t bytes, cudaStream_t st);
 // pinned host memory of the handle, kept between calls; the caller has waited
 // for every copy of the previous use.  nullptr when it cannot be had.
 void* pin_get(Handle* h, size_t bytes);
