@@ -481,7 +481,7 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
   // vectors per block: one block's K extent of the exchange product, nb r
   const int nb = std::min(block, M);
   const int nblocks = (M + nb - 1) / nb;
-  const int G = std::min(16, nblocks);  // blocks per exchange-product group
+  int G = std::min(16, nblocks);  // blocks per exchange-product group
   const int ntile = (ld / 128) * (ld / 128 + 1) / 2;
   std::vector<OzDens> dd(k);
   int kxmax = 0;
@@ -497,7 +497,6 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
     q.kblk = rup(q.kx, 32);
     q.nsub = (q.kblk + kOzKChunk - 1) / kOzKChunk;
     q.ksub = rup((q.kblk + q.nsub - 1) / q.nsub, 32);
-    q.xs_row = (int64_t)G * q.kblk;
     kxmax = std::max(kxmax, q.kx);
   }
   int nsm = 148;
@@ -518,16 +517,28 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
   while (2 * Lg <= 16 && Lg < nblocks && (size_t)2 * Lg * s * nb * ld * ld <= kOzGroupBytes &&
          (size_t)2 * Lg * 8 * ld * kxmax <= ((size_t)256 << 20))
     Lg *= 2;
-  const int nbg = nb * Lg;
-  const int jsplit = jacc_splits(nrs, nbg, nsm);
-  // one term per take() below (each rounded up to 256 bytes)
-  size_t need = 8 * (size_t)nbg * k + (size_t)s * nbg * ld * ld + 4 * (size_t)nbg * ld + 8 * (size_t)ld * kxmax * Lg +
-                8 * (size_t)ld * Lg + 8 * (size_t)nsm * 128 * 128 + sizeof(int) +
-                8 * (size_t)(jsplit * (size_t)nrs + vmulti_ranges(nrs) * (size_t)nbg) * k + 10 * 256;
-  for (const OzDens& q : dd)
-    need += 8 * (size_t)nrs + (size_t)s * q.npad * ld + 8 * (size_t)q.npad + (size_t)sk * ld * q.xs_row +
-            4 * (size_t)G * ld + 6 * 256;
-  char* ws = (char*)ws_get(h, need, st);
+  // Memory short: half as many blocks per launch, then per group of the exchange
+  // product, until the workspace can be had (one block each is the least).
+  int nbg = 0, jsplit = 0;
+  size_t need = 0;
+  char* ws = nullptr;
+  for (;;) {
+    nbg = nb * Lg;
+    jsplit = jacc_splits(nrs, nbg, nsm);
+    // one term per take() below (each rounded up to 256 bytes)
+    need = 8 * (size_t)nbg * k + (size_t)s * nbg * ld * ld + 4 * (size_t)nbg * ld + 8 * (size_t)ld * kxmax * Lg +
+           8 * (size_t)ld * Lg + 8 * (size_t)nsm * 128 * 128 + sizeof(int) +
+           8 * (size_t)(jsplit * (size_t)nrs + vmulti_ranges(nrs) * (size_t)nbg) * k + 10 * 256;
+    for (OzDens& q : dd) {
+      q.xs_row = (int64_t)G * q.kblk;
+      need += 8 * (size_t)nrs + (size_t)s * q.npad * ld + 8 * (size_t)q.npad + (size_t)sk * ld * q.xs_row +
+              4 * (size_t)G * ld + 6 * 256;
+    }
+    ws = (char*)ws_get(h, need, st);
+    if (ws || (Lg == 1 && G == 1)) break;
+    if (Lg > 1) Lg /= 2;
+    else G = (G + 1) / 2;
+  }
   if (!ws) { h->err = "jk workspace allocation failed"; return MG_ERR_MEMORY; }
   char* const ws_end = ws + need;
   auto take = [&](size_t bytes) { char* p = ws; ws += (bytes + 255) & ~(size_t)255; return (void*)p; };

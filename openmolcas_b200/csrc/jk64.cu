@@ -10,7 +10,8 @@
 //   k_syrk64   K += X X^T over the lower tiles, the K extent split over the
 //              CTAs so that a small matrix still fills the chip; every split
 //              keeps its own partial tiles, summed in order by k_finish_k
-// All sums run in a fixed order: a call gives the same bits every time.
+// All sums run in a fixed order: a call gives the same bits every time (unless
+// memory is short: blocks and splits then shrink, which changes the order).
 // Measured, 300 functions, 1400 vectors, rank 41 (cuBLAS over blocks of 32
 // unpacked squares before): half-transform 0.52 ms, 20 TFLOP/s (1.12 ms and 0.38
 // ms of unpacking); exchange product 0.25 ms, 21 TFLOP/s (1.26 ms); whole Fock
@@ -261,22 +262,36 @@ int jk_fp64_batch(Handle* h, int k, const double* const* Cs, const int* rs_, dou
   int nb = 1024;
   while (nb > 16 && (size_t)nb * rmax * xld * 8 > ((size_t)256 << 20)) nb /= 2;
   nb = std::min(nb, cho_vec_block());
-  const int nbm = std::min(nb, M);  // vectors X holds
-  const int nt = xld / bt, ntile = nt * (nt + 1) / 2;
-  // K splits of a full block of rank r: a few CTAs per SM in all, at least 8 chunks each
+  const int nt = xld / bt, ntile = nt * (nt + 1) / 2, nr = vmulti_ranges(nrs);
+  int nbm = 0;                       // vectors X holds
+  int per_sm = bt == 128 ? 4 : 8;    // CTAs per SM that the K splits aim at
+  // K splits of a full block of rank r: at least 8 chunks each
   auto splits = [&](int r, int& cps) {
     const int64_t nch = ((int64_t)nbm * r + kKc - 1) / kKc;
-    const int64_t want = std::max<int64_t>(1, (int64_t)nsm * (bt == 128 ? 4 : 8) / ntile);
+    const int64_t want = std::max<int64_t>(1, (int64_t)nsm * per_sm / ntile);
     const int64_t ns = std::max<int64_t>(1, std::min<int64_t>(want, nch / 8));
     cps = (int)((nch + ns - 1) / ns);
     return (int)((nch + cps - 1) / cps);
   };
-  int cps = 0, smax = 1;
-  for (int d = 0; d < k; ++d) smax = std::max(smax, splits(rs_[d], cps));
-  const int jsplit = jacc_splits(nrs, nbm, nsm), nr = vmulti_ranges(nrs);
-  const size_t nx = (size_t)nbm * rmax * xld, np = (size_t)smax * ntile * bt * bt, nj = (size_t)jsplit * k * nrs,
-               nvp = (size_t)nr * k * nb;
-  double* ws = (double*)ws_get(h, sizeof(double) * (nx + np + nj + nvp + (size_t)nb * k + (size_t)nrs * k), st);
+  // Memory short: blocks of half as many vectors, down to 16, then half as many
+  // splits, until the workspace can be had.
+  int cps = 0, jsplit = 0;
+  size_t nx = 0, np = 0, nj = 0, nvp = 0;
+  double* ws = nullptr;
+  for (;;) {
+    nbm = std::min(nb, M);
+    int smax = 1;
+    for (int d = 0; d < k; ++d) smax = std::max(smax, splits(rs_[d], cps));
+    jsplit = jacc_splits(nrs, nbm, nsm);
+    nx = (size_t)nbm * rmax * xld;
+    np = (size_t)smax * ntile * bt * bt;
+    nj = (size_t)jsplit * k * nrs;
+    nvp = (size_t)nr * k * nb;
+    ws = (double*)ws_get(h, sizeof(double) * (nx + np + nj + nvp + (size_t)nb * k + (size_t)nrs * k), st);
+    if (ws || (nb <= 16 && per_sm == 0)) break;
+    if (nb > 16) nb /= 2;
+    else per_sm /= 2;
+  }
   if (!ws) { h->err = "jk workspace allocation failed"; return MG_ERR_MEMORY; }
   double* X = ws;  // first: 16-byte aligned columns for cp.async (xld even)
   double* P = X + nx;

@@ -64,3 +64,35 @@ def test_kept_memory_gives_way():
                 # (the gradient and the mixed exchange add with atomics: rounding only)
                 assert float((a - b).abs().max()) <= 1e-12 * float(b.abs().max())
         assert skip or r.failed == 1
+
+
+@pytest.mark.parametrize("natom,thrcom,r", [(6, 1e-7, 9), (46, 0.3, 17)])
+def test_jk_workspaces_shrink(natom, thrcom, r):
+    """J/K calls whose workspace is refused again and again run with fewer vectors
+    per launch: the FP64 path against the products of the unpacked vectors (bars
+    of its tests), the mixed one against it, until nothing smaller is left."""
+    from tests.test_jk64_gpu import _reference
+    mol = B.make_molecule("shrink", natom, [("3s2p1d", natom)], 6)
+    g = MolGpu(mol)
+    g.cho_drv(thrcom=thrcom)
+    C = _density(g, r)
+    Jr, Kr, tj, tk = _reference(g, C)
+    for prec, bars in ((MolGpu.PREC_FP64, (tj, tk)),
+                       (MolGpu.PREC_MIXED, (1e-13 * float(Jr.abs().max()) + tj, 1e-10 * float(Kr.abs().max()) + tk))):
+        done = 0
+        for tries in range(1, 40):
+            g2 = MolGpu(mol)
+            g2.cho_drv(thrcom=thrcom)
+            g2.cho_jk(_density(g, 1))  # the tables that belong to the vectors are there
+            try:
+                # (each request is made twice)
+                with refuse(0, 2 * tries) as rf:
+                    J, K = g2.cho_jk(C, precision=prec)
+            except MolGpuError:
+                break
+            if rf.failed == 2 * tries:
+                done += 1
+                assert float((J - Jr).abs().max()) <= bars[0]
+                assert float((K - Kr).abs().max()) <= bars[1]
+        assert done >= 2  # (how many steps there are depends on the number of vectors)
+        assert g2.cho_jk(C, precision=prec)[1].any()
