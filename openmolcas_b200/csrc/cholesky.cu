@@ -465,9 +465,13 @@ struct ChoState {
 };
 
 // The vectors' storage of a state about to be replaced, for the next
-// decomposition of the same list (which frees what it does not use).
+// decomposition of the same list (which frees what it does not use).  FP64 J/K
+// and mg_cho_copy_vectors return while their kernels and copies still read the
+// vectors on the caller's stream, and the next decomposition may come on
+// another one: the device finishes before the storage is written again.
 void cho_recycle(Handle* h, ChoState* c) {
   if (!c) return;
+  cudaDeviceSynchronize();
   h->cho_spare.swap(c->Lblk);
   h->cho_spare_bytes = sizeof(double) * (size_t)c->nrs * kVecBlock;
   cho_free(c);
