@@ -328,7 +328,11 @@ void* pin_get(Handle* h, size_t bytes) {
   if (h->pin.ptr) cudaFreeHost(h->pin.ptr);
   h->pin.ptr = nullptr;
   h->pin.size = 0;
-  if (cudaMallocHost(&h->pin.ptr, bytes) != cudaSuccess) return nullptr;
+  if (cudaMallocHost(&h->pin.ptr, bytes) != cudaSuccess) {
+    h->pin.ptr = nullptr;
+    cudaGetLastError();  // (as dev_malloc)
+    return nullptr;
+  }
   h->pin.size = bytes;
   return h->pin.ptr;
 }
