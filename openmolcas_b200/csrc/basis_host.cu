@@ -67,7 +67,7 @@ int load_rys_table(Handle* h, const char* path) {
   if (fread(coef.data(), 8, off, f) != (size_t)off) { fclose(f); h->err = "truncated Rys table"; return 5; }
   fclose(f);
   if (dev_malloc(&h->d_rys, sizeof(double) * off) != cudaSuccess) { h->err = "cudaMalloc rys"; return 6; }
-  cudaMemcpy(h->d_rys, coef.data(), sizeof(double) * off, cudaMemcpyHostToDevice);
+  upload(h->d_rys, coef.data(), sizeof(double) * off);
   return 0;
 }
 
@@ -291,10 +291,10 @@ int setup_pairs(Handle* h) {
     h->err = "cudaMalloc pair data";
     return 1;
   }
-  cudaMemcpy(h->d_prim, prim.data(), sizeof(double) * prim.size(), cudaMemcpyHostToDevice);
-  cudaMemcpy(h->d_coef, coef.data(), sizeof(double) * coef.size(), cudaMemcpyHostToDevice);
-  cudaMemcpy(h->d_hrr, hrr.data(), sizeof(double) * hrr.size(), cudaMemcpyHostToDevice);
-  cudaMemcpy(h->d_pairs, h->pairs.data(), sizeof(DPair) * h->pairs.size(), cudaMemcpyHostToDevice);
+  upload(h->d_prim, prim.data(), sizeof(double) * prim.size());
+  upload(h->d_coef, coef.data(), sizeof(double) * coef.size());
+  upload(h->d_hrr, hrr.data(), sizeof(double) * hrr.size());
+  upload(h->d_pairs, h->pairs.data(), sizeof(DPair) * h->pairs.size());
   return 0;
 }
 

@@ -723,7 +723,7 @@ int mg_rys_roots(mg_handle* H, int nrys, int64_t n, const double* T, double* x, 
   double* dT = d;
   double* dx = d + n;
   double* dw = dx + n * nrys;
-  cudaMemcpy(dT, T, sizeof(double) * n, cudaMemcpyHostToDevice);
+  upload(dT, T, sizeof(double) * n);
   int rc = rys_eval(h, nrys, n, dT, dx, dw);
   if (!rc && (cudaMemcpy(x, dx, sizeof(double) * n * nrys, cudaMemcpyDeviceToHost) != cudaSuccess ||
               cudaMemcpy(w, dw, sizeof(double) * n * nrys, cudaMemcpyDeviceToHost) != cudaSuccess))

@@ -523,8 +523,8 @@ static void make_rs(Handle* h, ChoState* c, const std::vector<char>* keep = null
   c->nrs = c->rs_a.size();
 }
 
-// The state's device tables, in one allocation; the rs list goes up.
-static bool upload_rs(Handle* h, ChoState* c) {
+// The state's device tables, in one allocation; the rs list goes up in stream order.
+static bool upload_rs(Handle* h, ChoState* c, cudaStream_t st) {
   const size_t n = std::max<int64_t>(c->nrs, 1), nsp = c->sp_first.size();
   size_t need = 0;
   auto place = [&](size_t bytes) { const size_t o = need; need += (bytes + 255) & ~(size_t)255; return o; };
@@ -540,11 +540,11 @@ static bool upload_rs(Handle* h, ChoState* c) {
   c->d_diag = (double*)(c->d_tab + o_d);
   c->d_diag0 = (double*)(c->d_tab + o_d0);
   c->d_inred = (unsigned char*)(c->d_tab + o_in);
-  cudaMemcpy(c->d_rs, c->rsd.data(), sizeof(RsDev) * c->nrs, cudaMemcpyHostToDevice);
-  cudaMemcpy(c->d_rs_a, c->rs_a.data(), sizeof(int) * c->nrs, cudaMemcpyHostToDevice);
-  cudaMemcpy(c->d_rs_b, c->rs_b.data(), sizeof(int) * c->nrs, cudaMemcpyHostToDevice);
-  cudaMemcpy(c->d_sp_first, c->sp_first.data(), sizeof(int64_t) * nsp, cudaMemcpyHostToDevice);
-  cudaMemcpy(c->d_sp_count, c->sp_count.data(), sizeof(int) * nsp, cudaMemcpyHostToDevice);
+  cudaMemcpyAsync(c->d_rs, c->rsd.data(), sizeof(RsDev) * c->nrs, cudaMemcpyHostToDevice, st);
+  cudaMemcpyAsync(c->d_rs_a, c->rs_a.data(), sizeof(int) * c->nrs, cudaMemcpyHostToDevice, st);
+  cudaMemcpyAsync(c->d_rs_b, c->rs_b.data(), sizeof(int) * c->nrs, cudaMemcpyHostToDevice, st);
+  cudaMemcpyAsync(c->d_sp_first, c->sp_first.data(), sizeof(int64_t) * nsp, cudaMemcpyHostToDevice, st);
+  cudaMemcpyAsync(c->d_sp_count, c->sp_count.data(), sizeof(int) * nsp, cudaMemcpyHostToDevice, st);
   std::vector<RsDev>().swap(c->rsd);
   return true;
 }
@@ -756,7 +756,7 @@ int cho_decompose(Handle* h, const ChoCfgH& cfg, ChoState*& out, cudaStream_t st
       if (!(hd[t] < scrmax)) keep[c->rs_sp[t]] = 1;
     make_rs(h, c, &keep);
     // the diagonal over the kept shell pairs, from the same integral blocks
-    if (!upload_rs(h, c)) { err = "diagonal: out of device memory"; return MG_ERR_MEMORY; }
+    if (!upload_rs(h, c, st)) { err = "diagonal: out of device memory"; return MG_ERR_MEMORY; }
     k_extract_diag<<<nblk(std::max<int64_t>(c->nrs, 1)), 256, 0, st>>>(c->d_rs, c->nrs, h->d_pairs, d_off, buf,
                                                                         c->d_diag0);
     g_launches.fetch_add(1, std::memory_order_relaxed);

@@ -43,7 +43,7 @@ static int make_grad_tables(Handle* h, double** d_tab) {
     for (int lx = l; lx >= 0; --lx)
       for (int ly = l - lx; ly >= 0; --ly) cart[k++] = lx | (ly << 8) | ((l - lx - ly) << 16);
   if (dev_malloc(h, d_tab, sizeof(double) * kGTabD) != cudaSuccess) return MG_ERR_MEMORY;
-  cudaMemcpy(*d_tab, t.data(), sizeof(double) * kGTabD, cudaMemcpyHostToDevice);
+  upload(*d_tab, t.data(), sizeof(double) * kGTabD);
   return 0;
 }
 
@@ -314,7 +314,7 @@ int grad_build(Handle* h, double cutint, GradPlan& plan) {
   plan.d_items = nullptr;
   if (!plan.items.empty()) {
     if (dev_malloc(h, &plan.d_items, sizeof(GradItem) * plan.items.size()) != cudaSuccess) return MG_ERR_MEMORY;
-    cudaMemcpy(plan.d_items, plan.items.data(), sizeof(GradItem) * plan.items.size(), cudaMemcpyHostToDevice);
+    upload(plan.d_items, plan.items.data(), sizeof(GradItem) * plan.items.size());
   }
   cudaFree(plan.d_scratch);
   cudaFree(plan.d_counters);

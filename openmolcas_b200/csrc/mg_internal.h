@@ -41,6 +41,14 @@ inline cudaError_t dev_malloc(T** p, size_t bytes) {
   return e;
 }
 
+// Host data to device memory, complete on return: cudaMemcpy may return while
+// the last part of pageable memory is on its way, in the legacy stream's order
+// only, and the kernels that follow may come on a stream that does not wait for it.
+inline cudaError_t upload(void* dst, const void* src, size_t bytes) {
+  const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+  return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+}
+
 // Per-order metadata of the Rys root/weight table (constant memory).
 struct RysMeta {
   double h, invh, tmax;
