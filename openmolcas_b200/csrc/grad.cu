@@ -113,6 +113,7 @@ struct QuartetKind {
 };
 
 int grad_build(Handle* h, double cutint, GradPlan& plan) {
+  plan.cutint = -1;  // no plan until this one is complete
   const int ns = h->sh.size();
   // kinds of pairs
   std::vector<int> pkind(h->pairs.size());

@@ -96,3 +96,18 @@ def test_jk_workspaces_shrink(natom, thrcom, r):
                 assert float((K - Kr).abs().max()) <= bars[1]
         assert done >= 2  # (how many steps there are depends on the number of vectors)
         assert g2.cho_jk(C, precision=prec)[1].any()
+
+
+def test_gradient_after_a_plan_that_could_not_be_made():
+    """A re-plan (another threshold) that is refused memory leaves no half-made plan
+    to a call with the old threshold."""
+    g = MolGpu(B.small_molecule(3, seed=5))
+    D = _density(g, 5)
+    D = D @ D.t()
+    want = g.drvg1(D, cutint=1e-12)
+    for skip in range(3):
+        with pytest.raises(MolGpuError, match="rc=2"), refuse(skip):
+            g.drvg1(D, cutint=1e-10)
+        got = g.drvg1(D, cutint=1e-12)
+        # (atomic sums: rounding only)
+        assert float((got - want).abs().max()) <= 1e-12 * float(want.abs().max())
