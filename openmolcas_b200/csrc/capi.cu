@@ -583,7 +583,7 @@ int mg_drvg1_x(mg_handle* H, const double* d_D, const double* d_DS, double coulf
     if (rc) return rc;
   }
   if (!h->grad) h->grad = new GradPlan;
-  if (h->grad->cutint != cutint) {
+  if (!h->grad->ready || h->grad->cutint != cutint) {
     int rc = grad_build(h, cutint, *h->grad);
     if (rc) return rc;
   }
@@ -746,7 +746,7 @@ int mg_grad_set_tile(mg_handle* H, int nab1, int ncd1, int tpq, int order) {
   h->grad_order[nab1 * 8 + ncd1] = order % 3;
   h->grad_cap[nab1 * 8 + ncd1] = order / 3;
   h->grad_fixed[nab1 * 8 + ncd1] = true;
-  if (h->grad) h->grad->cutint = -1;  // re-plan at the next gradient
+  if (h->grad) h->grad->ready = false;  // re-plan at the next gradient
   return 0;
 }
 
@@ -754,7 +754,7 @@ int mg_tile_defaults(mg_handle* H) {
   if (!H) return MG_ERR_ARG;
   Handle* h = &H->h;
   for (int k = 0; k < 64; ++k) h->grad_fixed[k] = h->eri_fixed[k] = false;
-  if (h->grad) h->grad->cutint = -1;  // re-plan at the next gradient
+  if (h->grad) h->grad->ready = false;  // re-plan at the next gradient
   return 0;
 }
 
@@ -826,7 +826,7 @@ int mg_eri_class_times(mg_handle* H, int* keys, double* ms, int* tpq, int* pab, 
 int mg_grad_plan_info(mg_handle* H, int* keys, int* tpq, int* pab, int* pcd, int* rw, int maxn) {
   if (!H || (maxn > 0 && (!keys || !tpq || !pab || !pcd || !rw))) return MG_ERR_ARG;
   Handle* h = &H->h;
-  if (!h->grad || h->grad->cutint < 0) return 0;
+  if (!h->grad || !h->grad->ready) return 0;
   const std::vector<GradClass>& cl = h->grad->classes;
   for (int k = 0; k < std::min<int>(maxn, (int)cl.size()); ++k) {
     keys[k] = cl[k].nab1 * 8 + cl[k].ncd1;
@@ -846,7 +846,7 @@ double mg_drvg1_flops(mg_handle* H, double cutint) {
     if (mg_schwarz(H, t.data())) return -1;
   }
   if (!h->grad) h->grad = new GradPlan;
-  if (h->grad->cutint != cutint && grad_build(h, cutint, *h->grad)) return -1;
+  if ((!h->grad->ready || h->grad->cutint != cutint) && grad_build(h, cutint, *h->grad)) return -1;
   return grad_plan_flops(h, *h->grad);
 }
 

@@ -113,7 +113,7 @@ struct QuartetKind {
 };
 
 int grad_build(Handle* h, double cutint, GradPlan& plan) {
-  plan.cutint = -1;  // no plan until this one is complete
+  plan.ready = false;
   const int ns = h->sh.size();
   // kinds of pairs
   std::vector<int> pkind(h->pairs.size());
@@ -334,6 +334,7 @@ int grad_build(Handle* h, double cutint, GradPlan& plan) {
     if (rc) { h->err = "gradient tables"; return rc; }
   }
   plan.cutint = cutint;
+  plan.ready = true;
   return 0;
 }
 

@@ -198,7 +198,8 @@ struct GradPlan {
   double* d_tab = nullptr;       // per-CTA tables of the gradient kernel
   double* d_scratch = nullptr;   // per-group 2-PDM slots
   int* d_counters = nullptr;     // one work counter per class
-  double cutint = -1;
+  double cutint = 0;             // Schwarz threshold the list was made for
+  bool ready = false;            // false: to be made (again) before use
 };
 int grad_build(Handle* h, double cutint, GradPlan& plan);
 // fork the first n of the handle's side streams from `st` (created on first use) / join them back into `st`
