@@ -162,6 +162,8 @@ int mg_cho_diag(mg_handle* h, double* d_diag, void* stream);
  *                    recombination; Coulomb part FP64.  Energy within 1e-8 Eh
  *                    of MG_PREC_FP64 at 1500 functions / 12865 vectors;
  *   MG_PREC_SLICED(s) the same with s slices for both GEMMs (2..8).
+ * MG_PREC_FP64 only queues on the stream (a call that needs a larger workspace
+ * than any before it waits for the stream first); the others are synchronous.
  */
 #define MG_PREC_FP64 0
 #define MG_PREC_MIXED 1

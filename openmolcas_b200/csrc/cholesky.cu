@@ -437,6 +437,17 @@ __global__ void k_init_red(double* __restrict__ diag, unsigned char* __restrict_
   }
 }
 
+// inv[a*n + b] = inv[b*n + a] = t for every rs pair t (filled with -1 first:
+// AO pairs of shell pairs without rows keep it)
+__global__ void k_rs_inverse(const int* __restrict__ rs_a, const int* __restrict__ rs_b, int64_t nrs, int n,
+                             int* __restrict__ inv) {
+  int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (t >= nrs) return;
+  const int a = rs_a[t], b = rs_b[t];
+  inv[(size_t)a * n + b] = (int)t;
+  inv[(size_t)b * n + a] = (int)t;
+}
+
 static inline unsigned nblk(int64_t n, int b = 256) { return (unsigned)((n + b - 1) / b); }
 
 // --------------------------------------------------------------- host side
@@ -455,13 +466,13 @@ struct ChoState {
   double* d_diag = nullptr;     // working diagonal
   double* d_diag0 = nullptr;    // exact (ab|ab)
   unsigned char* d_inred = nullptr;
+  int* d_inv = nullptr;         // rs index of every AO pair (n x n, -1: no row), J/K
   std::vector<double*> Lblk;    // FP64 vector blocks, nrs x kVecBlock each
   int M = 0;
   std::vector<int> piv, pass_of;
   int npass = 0;
   short* d_lexp = nullptr;      // row exponents of the square L_J (mixed J/K), M x lexp_ld
   int lexp_ld = 0;
-  int* d_inv = nullptr;         // rs index of every AO pair (n x n, -1: no row), J/K
 };
 
 // The vectors' storage of a state about to be replaced, for the next
@@ -479,7 +490,7 @@ void cho_recycle(Handle* h, ChoState* c) {
 
 void cho_free(ChoState* c) {
   if (!c) return;
-  cudaFree(c->d_tab); cudaFree(c->d_lexp); cudaFree(c->d_inv);
+  cudaFree(c->d_tab); cudaFree(c->d_lexp);
   for (auto p : c->Lblk) cudaFree(p);
   delete c;
 }
@@ -523,14 +534,16 @@ static void make_rs(Handle* h, ChoState* c, const std::vector<char>* keep = null
   c->nrs = c->rs_a.size();
 }
 
-// The state's device tables, in one allocation; the rs list goes up in stream order.
+// The state's device tables, in one allocation; the rs list goes up in stream
+// order.  The inverse table of the J/K calls is made here, too: the decomposition
+// waits for its stream anyway, and FP64 J/K calls, the first one included, only queue.
 static bool upload_rs(Handle* h, ChoState* c, cudaStream_t st) {
   const size_t n = std::max<int64_t>(c->nrs, 1), nsp = c->sp_first.size();
   size_t need = 0;
   auto place = [&](size_t bytes) { const size_t o = need; need += (bytes + 255) & ~(size_t)255; return o; };
   const size_t o_rs = place(sizeof(RsDev) * n), o_a = place(sizeof(int) * n), o_b = place(sizeof(int) * n),
                o_f = place(sizeof(int64_t) * nsp), o_c = place(sizeof(int) * nsp), o_d = place(sizeof(double) * n),
-               o_d0 = place(sizeof(double) * n), o_in = place(n);
+               o_d0 = place(sizeof(double) * n), o_in = place(n), o_inv = place(sizeof(int) * (size_t)h->nbf * h->nbf);
   if (dev_malloc(h, &c->d_tab, need) != cudaSuccess) return false;
   c->d_rs = (RsDev*)(c->d_tab + o_rs);
   c->d_rs_a = (int*)(c->d_tab + o_a);
@@ -540,11 +553,15 @@ static bool upload_rs(Handle* h, ChoState* c, cudaStream_t st) {
   c->d_diag = (double*)(c->d_tab + o_d);
   c->d_diag0 = (double*)(c->d_tab + o_d0);
   c->d_inred = (unsigned char*)(c->d_tab + o_in);
+  c->d_inv = (int*)(c->d_tab + o_inv);
   cudaMemcpyAsync(c->d_rs, c->rsd.data(), sizeof(RsDev) * c->nrs, cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(c->d_rs_a, c->rs_a.data(), sizeof(int) * c->nrs, cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(c->d_rs_b, c->rs_b.data(), sizeof(int) * c->nrs, cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(c->d_sp_first, c->sp_first.data(), sizeof(int64_t) * nsp, cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(c->d_sp_count, c->sp_count.data(), sizeof(int) * nsp, cudaMemcpyHostToDevice, st);
+  cudaMemsetAsync(c->d_inv, 0xFF, sizeof(int) * (size_t)h->nbf * h->nbf, st);
+  k_rs_inverse<<<nblk(n), 256, 0, st>>>(c->d_rs_a, c->d_rs_b, c->nrs, h->nbf, c->d_inv);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
   std::vector<RsDev>().swap(c->rsd);
   return true;
 }
@@ -971,32 +988,7 @@ void cho_set_lexp(ChoState* c, short* p, int ld) {
   c->lexp_ld = ld;
 }
 
-// inv[a*n + b] = inv[b*n + a] = t for every rs pair t (filled with -1 first:
-// AO pairs of shell pairs without rows keep it)
-__global__ void k_rs_inverse(const int* __restrict__ rs_a, const int* __restrict__ rs_b, int64_t nrs, int n,
-                             int* __restrict__ inv) {
-  int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= nrs) return;
-  const int a = rs_a[t], b = rs_b[t];
-  inv[(size_t)a * n + b] = (int)t;
-  inv[(size_t)b * n + a] = (int)t;
-}
-
-const int* cho_inv_dev(Handle* h, ChoState* c, int n, cudaStream_t st) {
-  if (c->d_inv) return c->d_inv;
-  int* p = nullptr;
-  const size_t bytes = sizeof(int) * (size_t)n * n;
-  if (dev_malloc(h, &p, bytes) != cudaSuccess) return nullptr;
-  cudaMemsetAsync(p, 0xFF, bytes, st);
-  k_rs_inverse<<<nblk(std::max<int64_t>(c->nrs, 1)), 256, 0, st>>>(c->d_rs_a, c->d_rs_b, c->nrs, n, p);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  // later calls may come on other streams: the table is complete before it is kept
-  if (cudaStreamSynchronize(st) != cudaSuccess) {
-    cudaFree(p);
-    return nullptr;
-  }
-  return c->d_inv = p;
-}
+const int* cho_inv_dev(const ChoState* c) { return c->d_inv; }
 
 // ------------------------------------------------- in-core decomposition
 // CD_InCore (cholesky_util/cd_incore.F90:14 -> cd_incore_1.F90): pivoted

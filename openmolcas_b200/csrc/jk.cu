@@ -503,8 +503,7 @@ int jk_mixed_batch(Handle* h, int k, const double* const* Cs, const int* rs_, do
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
   const int* d_ra = cho_rs_a_dev(c);
   const int* d_rb = cho_rs_b_dev(c);
-  const int* inv = cho_inv_dev(h, c, n, st);
-  if (!inv) { h->err = "mixed J/K: inverse AO-pair table could not be stored"; return MG_ERR_MEMORY; }
+  const int* inv = cho_inv_dev(c);
   const size_t nn = (size_t)n * n;
   // blocks per launch of the slicing, the half-transform and the Coulomb part: a
   // power of two (storage blocks of 1024 vectors are not straddled), as many as

@@ -249,8 +249,7 @@ int jk_fp64_batch(Handle* h, int k, const double* const* Cs, const int* rs_, dou
     rmax = std::max(rmax, rs_[d]);
   }
   if (M == 0) return jk_no_vectors(h, k, Js, Ks, st);
-  const int* inv = cho_inv_dev(h, c, n, st);
-  if (!inv) { h->err = "FP64 J/K: inverse AO-pair table could not be stored"; return MG_ERR_MEMORY; }
+  const int* inv = cho_inv_dev(c);
   int nsm = 148;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
   // tiles of 128 once they leave no more than half a tile of padding and still

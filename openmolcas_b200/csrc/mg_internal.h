@@ -230,9 +230,8 @@ const int* cho_rs_a_dev(const ChoState* c);
 const int* cho_rs_b_dev(const ChoState* c);
 const double* cho_vec_ptr(const ChoState* c, int J0, int nb, cudaStream_t st, Handle* h);
 int cho_vec_block();
-// rs index of every AO pair (n x n device table, -1 where no row is stored),
-// built on first use and owned by the state; nullptr when it cannot be stored
-const int* cho_inv_dev(Handle* h, ChoState* c, int n, cudaStream_t st);
+// rs index of every AO pair (n x n device table, -1 where no row is stored)
+const int* cho_inv_dev(const ChoState* c);
 // cached row exponents of the square Cholesky vectors (M x ld), owned by the state
 short* cho_lexp(const ChoState* c, int ld);
 void cho_set_lexp(ChoState* c, short* p, int ld);

@@ -29,3 +29,25 @@ def test_replaced_vectors_outlive_their_readers():
     torch.cuda.synchronize()
     assert not torch.equal(g.cho_vectors()[:L0.shape[0]], L0[:g.cho_info()["M"]])
     assert torch.equal(J1, J0) and torch.equal(K1, K0) and torch.equal(L1, L0)
+
+
+def test_first_fp64_jk_after_a_decomposition_only_queues():
+    """FP64 J/K calls queue their kernels and return, the first call over new vectors
+    included: behind a delay on the same stream the call comes back before the
+    delay has ended."""
+    g = MolGpu(B.make_molecule("queue", 6, [("3s2p1d", 6)], 4))
+    g.cho_drv(thrcom=1e-5)
+    C = torch.from_numpy(B.density_factor(g.nbf, 9, 9)).cuda()
+    J0, K0 = g.cho_jk(C)  # (the workspace is there)
+    g.cho_drv(thrcom=1e-5)
+    torch.cuda.synchronize()
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        done = torch.cuda.Event()
+        torch.cuda._sleep(DELAY)
+        done.record()
+        J1, K1 = g.cho_jk(C)
+        pending = not done.query()
+    torch.cuda.synchronize()
+    assert pending
+    assert torch.equal(J1, J0) and torch.equal(K1, K0)
