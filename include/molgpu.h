@@ -230,11 +230,15 @@ int mg_grad_plan_info(mg_handle* h, int* keys, int* tpq, int* pab, int* pcd, int
  * next batch.  mg_eri_class_times reports the last profiled batch's classes
  * with their plan (group size, pab x pcd tile). */
 int mg_eri_set_tile(mg_handle* h, int nab, int ncd, int tpq, int order);
-/* Marks the gradient and ERI tiles set so far as defaults for throughput: a
+/* Marks the gradient and ERI tiles set so far as defaults for throughput.  A
  * class with no more work items than the GPU has SMs then runs its items with
- * the whole CTA and the largest tile that fits, whatever its tile says.  A tile
- * set after this call holds for every size.  The Python layer calls it after
- * applying its tables. */
+ * the whole CTA (512 threads) and the largest tile that fits, whatever its tile
+ * says; with up to two (four) items per SM its groups have at least 256 (128)
+ * threads, so that none stays idle; and an ERI group whose tile would hold
+ * fewer than four primitive quartets gives way to the next larger one.  A tile
+ * set after this call holds for every size: the group size asked for is taken
+ * if any tile fits it, else the next larger one.  The Python layer calls it
+ * after applying its tables. */
 int mg_tile_defaults(mg_handle* h);
 int mg_eri_profile(mg_handle* h, int enable);
 int mg_eri_class_times(mg_handle* h, int* keys, double* ms, int* tpq, int* pab, int* pcd, int maxn);

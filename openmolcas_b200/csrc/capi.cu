@@ -55,16 +55,18 @@ void eri_class_stats(ClassStats& cs, int nij, int nklc, int ne, int nf, int nsab
 ClassPlan eri_plan_for(const Handle* h, int nab, int ncd, const ClassStats& cs, int count) {
   const int key = nab * 8 + ncd;
   if (count <= h->nsm && !h->eri_fixed[key]) {
-    const ClassPlan pl = eri_plan(nab, ncd, cs, kEriThreads, 4);
+    const ClassPlan pl = eri_plan(nab, ncd, cs, kEriThreads, 4, 1);
     if (pl.PAB >= 1) return pl;
   }
-  const ClassPlan pl = eri_plan(nab, ncd, cs, h->eri_tpq[key], h->eri_order[key]);
+  // (a group that the caller asked for is taken whatever tile is left to it)
+  const int least_tile = h->eri_fixed[key] && h->eri_tpq[key] ? 1 : 4;
+  const ClassPlan pl = eri_plan(nab, ncd, cs, h->eri_tpq[key], h->eri_order[key], least_tile);
   // fewer items than groups: no more groups a CTA than there are items for (a
   // decomposition's classes have some 500 items, and class (0, 0) in groups of 64
   // threads takes 226 us there: 147 -> 142 ms at 300 functions)
   const int least = group_threads(count, h->nsm, kEriThreads);
   if (h->eri_fixed[key] || pl.tpq >= least) return pl;
-  const ClassPlan wide = eri_plan(nab, ncd, cs, least, h->eri_order[key]);
+  const ClassPlan wide = eri_plan(nab, ncd, cs, least, h->eri_order[key], 4);
   return wide.PAB >= 1 ? wide : pl;
 }
 

@@ -69,8 +69,9 @@ static size_t eri_group_smem(int nab, int ncd, const ClassStats& cs, int pab, in
 // dimension shrunk first when it does not fit (0 ket primitives, 1 bra; + 2:
 // the tile starts from 64 x 16 primitive pairs instead of 32 x 8; 4: from 64 x
 // 64 and shrinks towards four times as many bra as ket primitives: the bra sum of
-// a tile is formed in registers)
-ClassPlan eri_plan(int nab, int ncd, const ClassStats& cs, int tpq0, int order) {
+// a tile is formed in registers); least_tile: the
+// fewest primitive quartets of a tile that a group smaller than the CTA is taken for
+ClassPlan eri_plan(int nab, int ncd, const ClassStats& cs, int tpq0, int order, int least_tile) {
   const int NR = (nab + ncd) / 2 + 1;
   ClassPlan pl{0, 0, 0, 0, 0};
   const size_t budget = (227 * 1024) / 8 - kETabD;  // one CTA per SM
@@ -98,7 +99,7 @@ ClassPlan eri_plan(int nab, int ncd, const ClassStats& cs, int tpq0, int order) 
     // a group whose accumulators leave no room for a tile of a few quartets gives
     // way to the next larger one (class (2, 6), f f ket pairs: 34.2 ms with 1 x 1 tiles
     // in 256-thread groups, 6.1 ms in one group of 512)
-    if (tpq < kEriThreads && a * c < std::min(4, cs.max_npab * cs.max_npcd)) continue;
+    if (tpq < kEriThreads && a * c < std::min(least_tile, cs.max_npab * cs.max_npcd)) continue;
     if (eri_group_smem(nab, ncd, cs, a, c) <= gbudget) {
       pl.tpq = tpq;
       pl.PAB = a;

@@ -294,7 +294,7 @@ void* keep_get(Handle* h, Workspace& w, size_t bytes, cudaStream_t st);
 void* pin_get(Handle* h, size_t bytes);
 
 // ERI work lists (capi.cu) and launchers (eri.cu)
-ClassPlan eri_plan(int nab, int ncd, const ClassStats& cs, int tpq0 = 0, int order = 0);
+ClassPlan eri_plan(int nab, int ncd, const ClassStats& cs, int tpq0, int order, int least_tile);
 int eri_launch_class(Handle* h, const EriItem* d_items, int nitems, int nab, int ncd, const ClassPlan& pl, double* out,
                      int* d_counter, cudaStream_t st);
 // contracted ket pairs of one work item (0: even one does not fit)

@@ -40,3 +40,22 @@ def test_few_and_many_items_give_the_same_integrals(mix):
     for t in rng.choice(len(q), min(40, len(q)), replace=False):
         r = np.asarray(o.eri_quartet(*[int(v) for v in q[t]])).ravel(order="F")
         assert np.abs(few[off[t]:off[t + 1]] - r).max() < tol
+
+
+def test_group_size_set_by_the_caller_holds():
+    """A group size set by the caller is taken also where it leaves room for one
+    primitive quartet a tile only (f f ket pairs: the planner's own groups give way
+    to larger ones there), with the same integrals."""
+    mol = B.make_molecule("held", 2, [("4s3p2d1f_r", 2)], 5)
+    l = np.array([s.l for s in mol.shells])
+    ff = [(i, j) for i in range(len(l)) for j in range(i + 1) if l[i] == l[j] == 3]
+    pp = [(i, j) for i in range(len(l)) for j in range(i + 1) if l[i] == l[j] == 1]
+    q = np.array([a + b for a in pp for b in ff], dtype=np.int32)
+    g = MolGpu(mol)
+    want = g.eri_quartets(q)[0]
+    g.set_eri_tile(2, 6, 256, 0)
+    g.eri_profile(True)
+    got = g.eri_quartets(q)[0]
+    tpq, pab, pcd = g.eri_class_times()[(2, 6)][1]
+    assert tpq == 256 and pab * pcd < 4
+    assert float((got - want).abs().max()) < O.ERI_ABS_TOL * max(1.0, float(want.abs().max()))
