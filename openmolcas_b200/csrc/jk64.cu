@@ -123,16 +123,18 @@ __device__ __forceinline__ void cp16(void* dst, const void* src, bool valid) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(sz) : "memory");
 }
 
-// P[split][tile] (+)= X X^T (lower tiles of BT x BT, column-major): X
-// column-major with leading dimension xld (a multiple of BT; rows n.. zero), kt
+// P[split][tile] (+)= X X^T (lower tiles of 64 x 64, column-major): X
+// column-major with leading dimension xld (a multiple of 64; rows n.. zero), kt
 // columns.  blockIdx.x: lower tile, blockIdx.y: split, a range of cps chunks of
-// 16 columns.  Three-stage cp.async ring; warps of 8 FM x 8 FN.  first: write
-// instead of add.
-template <int BT, int NWM, int NWN, int FM, int FN>
-__global__ void __launch_bounds__(32 * NWM * NWN) k_syrk64(const double* __restrict__ X, int xld, int64_t kt, int cps,
-                                                           int first, double* __restrict__ P) {
-  static_assert(BT == NWM * FM * 8 && BT == NWN * FN * 8, "warp tiles cover the block");
-  constexpr int T = 32 * NWM * NWN, ST = BT + 4, NSTG = 3;
+// 16 columns.  Three-stage cp.async ring; 2 x 2 warps of 32 x 32.  first: write
+// instead of add.  Tiles of 128 in eight warps halve the L2 reads but were slower
+// at every size tried (whole J/K call, ms): 644 functions 1.40 against 1.25, 896
+// 4.04 against 3.83, 1246 16.1 against 15.8, 2100 123 against 109.
+constexpr int kSyTile = 64;
+
+__global__ void __launch_bounds__(128) k_syrk64(const double* __restrict__ X, int xld, int64_t kt, int cps, int first,
+                                                double* __restrict__ P) {
+  constexpr int BT = kSyTile, NWM = 2, FM = 4, FN = 4, T = 128, ST = BT + 4, NSTG = 3;
   extern __shared__ __align__(16) double sy_smem[];
   int ti = (int)((sqrtf(8.0f * blockIdx.x + 1.0f) - 1.0f) * 0.5f);
   while ((ti + 1) * (ti + 2) / 2 <= (int)blockIdx.x) ++ti;
@@ -230,8 +232,7 @@ static int launch_half64(int nt, dim3 grid, const double* L, int64_t nrs, const 
   return 0;
 }
 
-constexpr int kSyrkSmem64 = 3 * 2 * kKc * (64 + 4) * 8;
-constexpr int kSyrkSmem128 = 3 * 2 * kKc * (128 + 4) * 8;
+constexpr int kSyrkSmem = 3 * 2 * kKc * (kSyTile + 4) * 8;
 
 int jk_fp64(Handle* h, const double* d_C, int r, double* d_J, double* d_K, cudaStream_t st) {
   return jk_fp64_batch(h, 1, &d_C, &r, &d_J, &d_K, st);
@@ -252,9 +253,7 @@ int jk_fp64_batch(Handle* h, int k, const double* const* Cs, const int* rs_, dou
   const int* inv = cho_inv_dev(c);
   int nsm = 148;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
-  // tiles of 128 once they leave no more than half a tile of padding and still
-  // give some tens of lower tiles (half the L2 reads of the 64 tiles)
-  const int bt = n >= 640 ? 128 : 64;
+  constexpr int bt = kSyTile;
   const int xld = (n + bt - 1) / bt * bt;
   // vectors per block: a power of two (storage blocks of 1024 are not
   // straddled) that keeps X at or below 256 MB, at least 16
@@ -263,7 +262,7 @@ int jk_fp64_batch(Handle* h, int k, const double* const* Cs, const int* rs_, dou
   nb = std::min(nb, cho_vec_block());
   const int nt = xld / bt, ntile = nt * (nt + 1) / 2, nr = vmulti_ranges(nrs);
   int nbm = 0;                       // vectors X holds
-  int per_sm = bt == 128 ? 4 : 8;    // CTAs per SM that the K splits aim at
+  int per_sm = 8;                    // CTAs per SM that the K splits aim at
   // K splits of a full block of rank r: at least 8 chunks each
   auto splits = [&](int r, int& cps) {
     const int64_t nch = ((int64_t)nbm * r + kKc - 1) / kKc;
@@ -299,8 +298,7 @@ int jk_fp64_batch(Handle* h, int k, const double* const* Cs, const int* rs_, dou
   double* V = Vp + nvp;
   double* dw = V + (size_t)nb * k;
   auto count = [](int m) { g_launches.fetch_add(m, std::memory_order_relaxed); };
-  if (bt == 128 ? !smem_attr_once((const void*)k_syrk64<128, 2, 4, 8, 4>, kSyrkSmem128)
-                : !smem_attr_once((const void*)k_syrk64<64, 2, 2, 4, 4>, kSyrkSmem64)) {
+  if (!smem_attr_once((const void*)k_syrk64, kSyrkSmem)) {
     h->err = "FP64 J/K: shared-memory limit could not be raised";
     return MG_ERR_CUDA;
   }
@@ -332,8 +330,7 @@ int jk_fp64_batch(Handle* h, int k, const double* const* Cs, const int* rs_, dou
       launch_half64(nt8, dim3(xld / 64, nct, nv), Lb, nrs, inv, n, Cs[d], r, X, xld, st);
       const int64_t kt = (int64_t)nv * r, nch = (kt + kKc - 1) / kKc;
       const dim3 grid(ntile, (unsigned)std::min<int64_t>(nsplit, (nch + cps - 1) / cps));
-      if (bt == 128) k_syrk64<128, 2, 4, 8, 4><<<grid, 256, kSyrkSmem128, st>>>(X, xld, kt, cps, J0 == 0, P);
-      else k_syrk64<64, 2, 2, 4, 4><<<grid, 128, kSyrkSmem64, st>>>(X, xld, kt, cps, J0 == 0, P);
+      k_syrk64<<<grid, 128, kSyrkSmem, st>>>(X, xld, kt, cps, J0 == 0, P);
       used = std::max(used, (int)grid.y);
       count(2);
     }

@@ -1,5 +1,5 @@
 """FP64 J/K kernels (jk64.cu, coulomb.cuh) at the edges of their tiles: 64-row
-and 128-row tiles of the exchange product with remainders, column counts around
+tiles of the exchange product with remainders, column counts around
 the 8- and 64-column steps of the half-transform, one vector block and several,
 against torch products of the unpacked vectors.
 
@@ -47,7 +47,7 @@ def _reference(g, C):
     (2, 1e-6, (1, 7)),            # 28 functions: less than one tile
     (5, 1e-4, (8, 9, 63)),        # 70: a tile and a remainder
     (9, 1e-3, (64, 65)),          # 126
-    (46, 0.3, (17, 129)),         # 644: the 128-row tiles
+    (46, 0.3, (17, 129)),         # 644: many lower tiles, a remainder
 ])
 def test_fp64_jk_at_tile_edges(natom, thrcom, ranks):
     g = MolGpu(B.make_molecule("edge", natom, [("3s2p1d", natom)], 3))
