@@ -141,11 +141,16 @@ __device__ __forceinline__ void axpy4(const double* __restrict__ c, double v, do
 
 // Largest NI * NJ whose recursion stage runs one thread per job with the whole
 // 2D table of the job (NI NJ doubles) and the transfer rows in registers.  Larger
-// classes (from (3, 4): the registers would spill, and their tiles have too few
-// jobs to hide one long thread) go through a table in shared memory.  460-function
-// gradient, all classes with unchanged tiles 1723 -> 1554 ms: (3, 3) 167 -> 139,
-// (2, 3) 78 -> 50, (2, 2) 28 -> 17; (3, 5) 103 -> 92, (4, 5) 120 -> 106, (5, 4) 110
-// -> 101.
+// classes (from (3, 4): the registers spill more and more, and their tiles have
+// too few jobs to hide one long thread) go through a table in shared memory.
+// 460-function gradient, all classes with unchanged tiles 1723 -> 1554 ms: (3, 3)
+// 167 -> 139, (2, 3) 78 -> 50, (2, 2) 28 -> 17; (3, 5) 103 -> 92, (4, 5) 120 -> 106,
+// (5, 4) 110 -> 101.  The largest classes below the limit spill, too (bytes stored:
+// (5, 2) 224, (4, 2) 176, (3, 3) 88, (2, 5) 68), and are the faster this way all
+// the same: against the shared-memory table, each with its best tile, 10 atoms of
+// 4s3p2d: (4, 2) 4.03 and 4.29 ms, (3, 3) 10.0 and 11.5, (2, 5) 2.63 and 2.71, the
+// smaller tables 1.3 to 1.5 times as fast.  (5, 2) alone is slower, 3.05 and 3.00 (5
+// atoms with f shells: 2.43 and 2.27), too little for a rule of its own.
 constexpr int kGradJobMax = 18;
 
 // The recursion stage with one thread per (quartet, root, direction) job.  The
