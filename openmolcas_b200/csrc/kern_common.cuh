@@ -43,29 +43,38 @@ __device__ __forceinline__ int d_ccum(int l) { return l * (l + 1) * (l + 2) / 6;
 __device__ __forceinline__ int d_sph_off(int l) { return l == 0 ? 0 : l == 1 ? 1 : l == 2 ? 10 : 40; }
 __device__ __forceinline__ int ev2(int x) { return (x + 1) & ~1; }
 
+// high half of the product (host side: for the tests of the divisions)
+__host__ __device__ __forceinline__ unsigned mul_hi(unsigned a, unsigned b) {
+#ifdef __CUDA_ARCH__
+  return __umulhi(a, b);
+#else
+  return (unsigned)((unsigned long long)a * b >> 32);
+#endif
+}
+
 // Division by a run-time divisor n through a multiply-high:
 // q = floor(o * ceil(2^32 / n) / 2^32), exact for o < 2^32 / n (the host
 // planner checks every loop extent against that bound); n = 1 uses the mask.
 struct FDiv {
   unsigned m, k, n;
 };
-__device__ __forceinline__ FDiv fdiv(unsigned n) {
+__host__ __device__ __forceinline__ FDiv fdiv(unsigned n) {
   FDiv f;
   f.n = n;
   f.m = n == 1 ? 0u : 0xFFFFFFFFu / n + 1u;
   f.k = n == 1 ? 0xFFFFFFFFu : 0u;
   return f;
 }
-__device__ __forceinline__ unsigned fq(unsigned o, const FDiv& f) { return __umulhi(o, f.m) + (o & f.k); }
+__host__ __device__ __forceinline__ unsigned fq(unsigned o, const FDiv& f) { return mul_hi(o, f.m) + (o & f.k); }
 
 // The same with a correction step: exact for every o < 2^32, whatever n
 // (floor(2^32 / n) o / 2^32 is at most one below the quotient).
 struct SDiv {
   unsigned m, n;
 };
-__device__ __forceinline__ SDiv sdiv(unsigned n) { return {n == 1 ? 0xFFFFFFFFu : 0xFFFFFFFFu / n + (0xFFFFFFFFu % n == n - 1), n}; }
-__device__ __forceinline__ int sq(int o, const SDiv& f, int& rem) {
-  unsigned q = __umulhi((unsigned)o, f.m), r = (unsigned)o - q * f.n;
+__host__ __device__ __forceinline__ SDiv sdiv(unsigned n) { return {n == 1 ? 0xFFFFFFFFu : 0xFFFFFFFFu / n + (0xFFFFFFFFu % n == n - 1), n}; }
+__host__ __device__ __forceinline__ int sq(int o, const SDiv& f, int& rem) {
+  unsigned q = mul_hi((unsigned)o, f.m), r = (unsigned)o - q * f.n;
   if (r >= f.n) {
     ++q;
     r -= f.n;
@@ -74,8 +83,9 @@ __device__ __forceinline__ int sq(int o, const SDiv& f, int& rem) {
   return (int)q;
 }
 
-// x^-1 and x^-1/2: one reciprocal root, its square with one Newton step (both
-// within a unit in the last place, as the division and the root they replace)
+// x^-1 and x^-1/2: one reciprocal root, its square with one Newton step.  Over
+// eleven decades of x the largest errors are 0.500 and 0.506 units in the last
+// place (a division, and the root of its rounded result: 0.5 and up to 0.75).
 __device__ __forceinline__ void recip_root(double x, double& xi, double& rxi) {
   rxi = rsqrt(x);
   const double y = rxi * rxi;
