@@ -306,9 +306,5 @@ int build_eri_items(Handle* h, const int32_t* q4, int64_t nq, const int64_t* off
                     std::vector<EriClass>& classes);
 int run_eri_items(Handle* h, const std::vector<EriItem>& items, const std::vector<EriClass>& classes, double* d_out,
                   cudaStream_t st);
-int eri_run(Handle* h, const EriItem* d_items, const std::vector<int>& class_begin, const std::vector<int>& class_nab,
-            const std::vector<int>& class_ncd, const std::vector<int>& class_np, const std::vector<size_t>& class_smem,
-            double* out, cudaStream_t st);
-void rys_upload_meta(Handle* h);
 
 }  // namespace mg

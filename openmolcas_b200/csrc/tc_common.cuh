@@ -50,14 +50,7 @@ __device__ __forceinline__ bool tc_mbar_wait(uint32_t bar, uint32_t parity, vola
   return false;
 }
 
-// 2D and 5D tiled TMA loads into shared memory, completion on an mbarrier.
-__device__ __forceinline__ void tc_tma_load(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
-          dst),
-      "l"((uint64_t)map), "r"(bar), "r"(x), "r"(y)
-      : "memory");
-}
+// 5D tiled TMA load into shared memory, completion on an mbarrier.
 __device__ __forceinline__ void tc_tma_load5(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2,
                                              int c3, int c4) {
   asm volatile(
@@ -67,44 +60,23 @@ __device__ __forceinline__ void tc_tma_load5(uint32_t dst, const CUtensorMap* ma
       : "memory");
 }
 
-// Shared-memory matrix descriptors (Blackwell version 1), K-major operands.
-// 128-byte swizzle: 8-row atoms of 1024 bytes stacked along M/N.
-__device__ __forceinline__ uint64_t tc_desc_sw128(uint32_t addr) {
-  uint64_t d = (uint64_t)((addr >> 4) & 0x3FFF);
-  d |= (uint64_t)1 << 16;            // leading byte offset (unused for swizzled K-major)
-  d |= (uint64_t)(1024 >> 4) << 32;  // stride byte offset
-  d |= (uint64_t)1 << 46;            // descriptor version
-  d |= (uint64_t)2 << 61;            // SWIZZLE_128B
-  return d;
-}
-// 32-byte swizzle: rows of 32 bytes (one K = 32 step of 8-bit operands),
-// 8-row atoms of 256 bytes stacked along M/N.
+// Shared-memory matrix descriptor (Blackwell version 1), K-major operand,
+// 32-byte swizzle: rows of 32 bytes (one K = 32 step of 8-bit operands), 8-row
+// atoms of 256 bytes stacked along M/N.
 __device__ __forceinline__ uint64_t tc_desc_sw32(uint32_t addr) {
   uint64_t d = (uint64_t)((addr >> 4) & 0x3FFF);
-  d |= (uint64_t)1 << 16;
-  d |= (uint64_t)(256 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)1 << 16;           // leading byte offset (unused for swizzled K-major)
+  d |= (uint64_t)(256 >> 4) << 32;  // stride byte offset
+  d |= (uint64_t)1 << 46;           // descriptor version
   d |= (uint64_t)6 << 61;  // SWIZZLE_32B
   return d;
 }
 
-// Instruction descriptor, M = 128, both operands K-major.
-//   BF16 x BF16 -> FP32 (kind::f16)
-__host__ __device__ constexpr uint32_t tc_idesc_bf16(int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((128u >> 4) << 24);
-}
-//   8-bit integers -> S32 (kind::i8); a_signed / b_signed select S8 (else U8)
+// Instruction descriptor, M = 128, both operands K-major: 8-bit integers -> S32
+// (kind::i8); a_signed / b_signed select S8 (else U8)
 __host__ __device__ constexpr uint32_t tc_idesc_i8(int n, bool a_signed, bool b_signed) {
   return (2u << 4) | ((a_signed ? 1u : 0u) << 7) | ((b_signed ? 1u : 0u) << 10) | ((uint32_t)(n >> 3) << 17) |
          ((128u >> 4) << 24);
-}
-
-__device__ __forceinline__ void tc_mma_f16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(tmem_d),
-      "l"(a), "l"(b), "r"(idesc), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
 }
 
 // One lane of a converged warp (1 there, 0 in the others).
@@ -130,11 +102,7 @@ __device__ __forceinline__ void tc_mma_i8(uint32_t tmem_d, uint64_t a, uint64_t 
 }
 
 // Arrive on an mbarrier once every tcgen05 operation issued so far by this
-// thread has completed.
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
+// thread has completed (the lanes with el != 0).
 __device__ __forceinline__ void tc_commit_if(uint32_t bar, uint32_t el) {
   asm volatile(
       "{\n\t.reg .pred q;\n\t"
@@ -144,21 +112,8 @@ __device__ __forceinline__ void tc_commit_if(uint32_t bar, uint32_t el) {
       : "memory");
 }
 
-// 32 consecutive 32-bit TMEM columns of this thread's lane (warp w reads
-// lanes 32 (w % 4) .. +31).
-__device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&v)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-      "%15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-        "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-        "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// 16 consecutive 32-bit TMEM columns of this thread's lane, without waiting:
+// 16 consecutive 32-bit TMEM columns of this thread's lane (warp w reads lanes
+// 32 (w % 4) .. +31), without waiting:
 // several loads may be in flight; tc_ld_wait() completes them and
 // tc_ld_bind() orders every later use of the registers after it.
 __device__ __forceinline__ void tc_ld16_async(uint32_t taddr, uint32_t (&v)[16]) {
@@ -173,17 +128,6 @@ __device__ __forceinline__ void tc_ld_wait() { asm volatile("tcgen05.wait::ld.sy
 __device__ __forceinline__ void tc_ld_bind(uint32_t (&v)[16]) {
 #pragma unroll
   for (int i = 0; i < 16; ++i) asm volatile("" : "+r"(v[i]));
-}
-
-// 16 consecutive 32-bit TMEM columns of this thread's lane.
-__device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-      "%15}, [%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
 }  // namespace mg
