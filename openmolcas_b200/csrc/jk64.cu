@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "coulomb.cuh"
 #include "kern_common.cuh"
@@ -35,23 +36,33 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
 
 constexpr int kKc = 16;  // K extent of a shared-memory chunk
 
-// X_J = L_J C: 4 warps of 16 rows x 8 NT columns.  The fragments of both
-// operands are read from [k][row] tiles whose row stride is 4 mod 16 doubles,
-// so the 16 lanes of a half-warp touch 16 different banks.  The rs indices are
-// fetched two chunks and the vector elements one chunk ahead (two dependent
-// loads per element).  Rows n..xld of X come out as zeros.
+// X_J = L_J C, a tile of 64 rows x 8 NT columns: 4 warps of 16 rows.  The rs
+// indices are fetched two chunks and the vector elements one chunk ahead (two
+// dependent loads per element).  Rows n..xld of X come out as zeros.
+// Bound: the FP64 tensor pipe (82 percent busy at 896 functions, rank 320) and,
+// close behind, the shared-memory and L1 pipe (per chunk of 16 k and 64 columns 1024
+// clocks of products; some 900 of fragment reads, stores and gathers).  Hence the
+// layout: A and B tiles have rows of 4 mod 16 doubles per k, so that the 16 lanes of
+// a half-warp (4 k x 4 rows or columns) read 16 banks, and B's rows are shifted by
+// one double after every fourth, so that a store (16 k of one column) has 16, too
+// (it had 4: 1820 functions, 699 vectors, rank 300, 54.2 -> 52.1 ms).  The last
+// column tile forms only the eights of columns there are (52.1 -> 48.1 ms; rank 193
+// 37.0 -> 32.8).  Two such groups of warps over 112 columns, which halve the gathers
+// per product, were no faster: 48.9 ms, rank 229 40.9 against 37.0.
 template <int NT>
 __global__ void __launch_bounds__(128) k_half64(const double* __restrict__ L, int64_t nrs,
-                                                const int* __restrict__ inv, int n, const double* __restrict__ C,
-                                                int r, double* __restrict__ X, int xld) {
-  constexpr int BN = 8 * NT, SA = 68, SB = BN % 16 ? BN + 12 : BN + 4;
+                                                   const int* __restrict__ inv, int n, const double* __restrict__ C,
+                                                   int r, double* __restrict__ X, int xld) {
+  constexpr int BN = 8 * NT, SA = 68, SB = BN % 16 ? BN + 12 : BN + 4, SB4 = 4 * SB + 1;
   __shared__ double As[2][kKc][SA];
-  __shared__ double Bs[2][kKc][SB];
+  __shared__ double Bs[2][kKc / 4 * SB4];
   const int a0 = blockIdx.x * 64, c0 = blockIdx.y * BN, J = blockIdx.z;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nj = min(NT, (r - c0 + 7) >> 3);  // eights of columns
   const double* LJ = L + nrs * J;
-  const int row = tid & 63, kr = tid >> 6;   // A: row, k = kr + 2 i
-  const int bk = tid & 15, bc = tid >> 4;    // B: k, column bc + 8 i
+  const int row = tid & 63, kr = tid >> 6;  // A: row, k = kr + 2 i
+  const int bk = tid & 15, bc = tid >> 4;   // B: k, column bc + 8 i
+  const int bo = (bk >> 2) * SB4 + (bk & 3) * SB + bc;
   const int nch = (n + kKc - 1) / kKc;
   int idx[8];
   double av[8], bv[NT];
@@ -77,6 +88,23 @@ __global__ void __launch_bounds__(128) k_half64(const double* __restrict__ L, in
   for (int i = 0; i < 2; ++i)
 #pragma unroll
     for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  auto product = [&](int s, auto cols) {
+    constexpr int N = decltype(cols)::value;
+    if constexpr (N <= NT) {
+#pragma unroll
+      for (int ks = 0; ks < kKc / 4; ++ks) {
+        const double* ap = &As[s][4 * ks + (lane & 3)][warp * 16 + (lane >> 2)];
+        const double* bp = &Bs[s][ks * SB4 + (lane & 3) * SB + (lane >> 2)];
+        const double f0 = ap[0], f1 = ap[8];
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+          const double b = bp[8 * j];
+          dmma(acc[0][j], f0, b);
+          dmma(acc[1][j], f1, b);
+        }
+      }
+    }
+  };
   load_idx(0);
   load_val(0);
   load_idx(1);
@@ -85,23 +113,21 @@ __global__ void __launch_bounds__(128) k_half64(const double* __restrict__ L, in
 #pragma unroll
     for (int i = 0; i < 8; ++i) As[s][kr + 2 * i][row] = av[i];
 #pragma unroll
-    for (int i = 0; i < NT; ++i) Bs[s][bk][bc + 8 * i] = bv[i];
+    for (int i = 0; i < NT; ++i) Bs[s][bo + 8 * i] = bv[i];
     __syncthreads();
     if (ch + 1 < nch) {
       load_val(ch + 1);
       load_idx(ch + 2);
     }
-#pragma unroll
-    for (int ks = 0; ks < kKc / 4; ++ks) {
-      const double* ap = &As[s][4 * ks + (lane & 3)][warp * 16 + (lane >> 2)];
-      const double* bp = &Bs[s][4 * ks + (lane & 3)][lane >> 2];
-      const double f0 = ap[0], f1 = ap[8];
-#pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        const double b = bp[8 * j];
-        dmma(acc[0][j], f0, b);
-        dmma(acc[1][j], f1, b);
-      }
+    switch (nj) {  // (unrolled for every width: a test per eight columns costs a tenth)
+      case 1: product(s, std::integral_constant<int, 1>{}); break;
+      case 2: product(s, std::integral_constant<int, 2>{}); break;
+      case 3: product(s, std::integral_constant<int, 3>{}); break;
+      case 4: product(s, std::integral_constant<int, 4>{}); break;
+      case 5: product(s, std::integral_constant<int, 5>{}); break;
+      case 6: product(s, std::integral_constant<int, 6>{}); break;
+      case 7: product(s, std::integral_constant<int, 7>{}); break;
+      case 8: product(s, std::integral_constant<int, 8>{}); break;
     }
   }
 #pragma unroll
@@ -109,7 +135,7 @@ __global__ void __launch_bounds__(128) k_half64(const double* __restrict__ L, in
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const int c = c0 + 8 * j + 2 * (lane & 3) + e;
-      if (c < r) {
+      if (j < nj && c < r) {
         double* x = X + ((size_t)J * r + c) * xld + a0 + warp * 16 + (lane >> 2);
         x[0] = acc[0][j][e];
         x[8] = acc[1][j][e];
@@ -263,11 +289,22 @@ int jk_fp64_batch(Handle* h, int k, const double* const* Cs, const int* rs_, dou
   const int nt = xld / bt, ntile = nt * (nt + 1) / 2, nr = vmulti_ranges(nrs);
   int nbm = 0;                       // vectors X holds
   int per_sm = 8;                    // CTAs per SM that the K splits aim at
-  // K splits of a full block of rank r: at least 8 chunks each
+  // K splits of a full block of rank r, at least 8 chunks each: of that number and
+  // up to twice as many, the first that fills the last wave of CTAs (four of 52 KB
+  // are resident per SM) within 3 percent of the best (exchange product at 1246
+  // functions, rank 300, 210 tiles: five splits 9.2 ms, eight 8.7)
   auto splits = [&](int r, int& cps) {
     const int64_t nch = ((int64_t)nbm * r + kKc - 1) / kKc;
     const int64_t want = std::max<int64_t>(1, (int64_t)nsm * per_sm / ntile);
-    const int64_t ns = std::max<int64_t>(1, std::min<int64_t>(want, nch / 8));
+    int64_t ns = std::max<int64_t>(1, std::min<int64_t>(want, nch / 8));
+    const int64_t most = per_sm ? std::max<int64_t>(ns, std::min<int64_t>(2 * ns, nch / 8)) : ns;
+    auto fill = [&](int64_t q) {
+      const int64_t slots = 4 * (int64_t)nsm, ctas = q * ntile;
+      return (double)ctas / (double)((ctas + slots - 1) / slots * slots);
+    };
+    double best = 0.0;
+    for (int64_t q = ns; q <= most; ++q) best = std::max(best, fill(q));
+    while (fill(ns) < best - 0.03) ++ns;
     cps = (int)((nch + ns - 1) / ns);
     return (int)((nch + cps - 1) / cps);
   };

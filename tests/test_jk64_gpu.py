@@ -59,3 +59,19 @@ def test_fp64_jk_at_tile_edges(natom, thrcom, ranks):
         assert float((J - Jr).abs().max()) <= tj
         assert float((K - Kr).abs().max()) <= tk
         assert torch.equal(K, K.t()) and torch.equal(J, J.t())
+
+
+def test_fp64_jk_column_tiles():
+    """Ranks around the half-transform's column tiles (up to 64 columns, spread
+    evenly, the last one cut to the eights of columns there are): every width of
+    the last tile, and more columns than functions."""
+    g = MolGpu(B.make_molecule("edge", 5, [("3s2p1d", 5)], 3))
+    g.cho_drv(thrcom=1e-3)
+    ranks = (56, 57, 64, 66, 80, 81, 111, 112, 113, 121, 168, 169, 177, 224, 225, 336)
+    Cs = [torch.from_numpy(np.random.default_rng(r).standard_normal((g.nbf, r)) / np.sqrt(r)).cuda() for r in ranks]
+    got = g.cho_jk_batch(Cs[:8], precision=MolGpu.PREC_FP64) + g.cho_jk_batch(Cs[8:], precision=MolGpu.PREC_FP64)
+    for C, (J, K) in zip(Cs, got):
+        Jr, Kr, tj, tk = _reference(g, C)
+        assert float((J - Jr).abs().max()) <= tj
+        assert float((K - Kr).abs().max()) <= tk
+        assert torch.equal(K, K.t())
