@@ -150,6 +150,7 @@ def _set_all_eri(g, tpq, order):
     for a in range(0, 8):
         for b in range(0, 8):
             g.set_eri_tile(a, b, tpq, order)
+    g.tile_defaults()  # timed as the table's entries will be used
 
 
 def _eri_ms(g, sel, out, reps):
@@ -192,6 +193,7 @@ def tune_eri(cfg="c2", sample=400_000, reps=2, margin=0.02, device=0, log=print)
     for key, t in classes.items():
         a, b = (int(x) for x in key.split(","))
         g.set_eri_tile(a, b, t["tpq"], t["order"])
+    g.tile_defaults()
     tuned, _ = _eri_batch(g, sel, out, reps)
     ms_tuned = _eri_ms(g, full, out, max(reps, 3))
     _set_all_eri(g, 0, 0)

@@ -128,7 +128,7 @@ class MolGpu:
                 for key, t in json.load(f)["classes"].items():
                     nab, ncd = (int(x) for x in key.split(","))
                     self.set_eri_tile(nab, ncd, t["tpq"], t["order"])
-        self._check(self.L.mg_tile_defaults(self.h), "mg_tile_defaults")
+        self.tile_defaults()
 
     def _check(self, rc, what):
         if rc != 0:
@@ -212,6 +212,12 @@ class MolGpu:
         the planner's) and the dimension shrunk first (0 ket, 1 bra primitives;
         + 2: starting from 64 x 16 primitive pairs instead of 32 x 8)."""
         self._check(self.L.mg_eri_set_tile(self.h, nab, ncd, tpq, order), "mg_eri_set_tile")
+
+    def tile_defaults(self):
+        """The tiles set so far are defaults: the planner may pass over them where a
+        class has few work items or a group's tile would be too small; tiles set
+        later hold."""
+        self._check(self.L.mg_tile_defaults(self.h), "mg_tile_defaults")
 
     def eri_profile(self, enable: bool = True):
         """Later ERI batches run their classes one after another on the
