@@ -13,10 +13,12 @@
 // All sums run in a fixed order: a call gives the same bits every time (unless
 // memory is short: blocks and splits then shrink, which changes the order).
 // Measured, 300 functions, 1400 vectors, rank 41 (cuBLAS over blocks of 32
-// unpacked squares before): half-transform 0.52 ms, 20 TFLOP/s (1.12 ms and 0.38
+// unpacked squares before): half-transform 0.50 ms, 21 TFLOP/s (1.12 ms and 0.38
 // ms of unpacking); exchange product 0.25 ms, 21 TFLOP/s (1.26 ms); whole Fock
-// update 4.55 -> 1.78 ms.  1250 functions, 3789 vectors, rank 167: 146.8 -> 117.1
-// ms (25 TFLOP/s; the FP64 pipe peaks at 37).
+// update 4.55 -> 1.18 ms with the parallel in-core decomposition.  1250 functions,
+// 3789 vectors, rank 167: 146.8 -> 108.8 ms (27 TFLOP/s; the FP64 pipe peaks at
+// 37).  Eight densities of rank 50 to 300 at 1820 functions, 699 vectors: 350 ms,
+// against 336 with cuBLAS, where one unpacking served all eight.
 #include <cuda_runtime.h>
 
 #include <algorithm>
